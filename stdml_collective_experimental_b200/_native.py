@@ -6,6 +6,7 @@ library is an ImportError with the build command, never a silent Python
 fallback.
 """
 import ctypes
+import importlib.util
 import os
 import subprocess
 import threading
@@ -14,8 +15,11 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(_HERE, "csrc")
 LIB_PATH = os.path.join(_HERE, "libstdml_collective_b200.so")
 
+FASTCALL_PATH = os.path.join(_HERE, "_fastcall.so")
+
 _lock = threading.Lock()
 _lib = None
+_fastcall = None
 
 
 def build(jobs=None, verbose=False, target="all"):
@@ -46,6 +50,26 @@ def lib():
             _lib = ctypes.CDLL(LIB_PATH, mode=ctypes.RTLD_GLOBAL)
             _declare(_lib)
         return _lib
+
+
+def fastcall():
+    """The module that takes DeviceSession's calls to the library (csrc/python/fastcall.cpp)."""
+    global _fastcall
+    lib()
+    with _lock:
+        if _fastcall is None:
+            if not os.path.exists(FASTCALL_PATH):
+                try:
+                    build(target="lib")
+                except Exception as e:
+                    raise ImportError(f"{FASTCALL_PATH} is missing and could not be built ({e}); "
+                                      f"build it with `make -C {CSRC}`") from e
+            spec = importlib.util.spec_from_file_location(
+                __package__ + "._fastcall", FASTCALL_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            _fastcall = module
+        return _fastcall
 
 
 class NativeError(RuntimeError):
@@ -94,12 +118,6 @@ def _declare(l):
     l.stdmlc_dw_set_tuning.argtypes = [vp, c.c_int, c.c_longlong, c.c_longlong, c.c_longlong]
     l.stdmlc_dw_set_knob.argtypes = [vp, c.c_char_p, c.c_longlong]
     l.stdmlc_dw_drop_registrations.argtypes = [vp]
-    l.stdmlc_dw_all_reduce.argtypes = [vp, vpp, vpp, u64, c.c_int, c.c_int, c.c_double, c.c_int, vp]
-    l.stdmlc_dw_reduce.argtypes = [vp, vpp, vpp, u64, c.c_int, c.c_int, c.c_int, c.c_double, vp]
-    l.stdmlc_dw_group_all_reduce.argtypes = [vp, u64, vpp, vpp, c.POINTER(u64), c.c_int, c.c_int,
-                                             c.c_int, c.c_double, c.c_int, vp]
-    l.stdmlc_dw_all_gather.argtypes = [vp, vpp, vpp, u64, c.c_int, vp]
-    l.stdmlc_dw_broadcast.argtypes = [vp, vpp, vpp, u64, c.c_int, c.c_int, vp]
     l.stdmlc_dw_barrier.argtypes = [vp, vp]
     l.stdmlc_dw_raw_all_reduce.argtypes = [vp, u64, vpp, vpp, u64, c.c_int, c.c_int, c.c_int,
                                            c.c_int, c.c_int, c.c_int, c.c_int, c.c_double, vp]

@@ -10,6 +10,7 @@ sum/min/max/prod/bit_xor, rank-major ``all_gather``, ``broadcast`` (root 0 by
 default, as the reference fixes it), plus ``reduce`` and a fused
 ``group_all_reduce`` with optional gradient scale and f32<->bf16/f16 cast.
 """
+import contextlib
 import ctypes
 import os
 
@@ -75,7 +76,11 @@ def _ptr_array(tensors):
 class DeviceSession:
     def __init__(self, handle, device):
         self._h = handle
+        self._hv = handle.value  # the same as a number, 0 once closed
+        self._prof = None
+        self._device_index = device
         self._lib = _native.lib()
+        self._fast = _native.fastcall()
         self.device = torch.device("cuda", device)
         self.rank = self._info(0)
         self.world = self._info(1)
@@ -133,7 +138,7 @@ class DeviceSession:
     def close(self):
         if self._h is not None:
             self._symm.clear()
-            h, self._h = self._h, None
+            h, self._h, self._hv = self._h, None, 0
             _native.check(self._lib.stdmlc_dw_destroy(h))
 
     def __enter__(self):
@@ -235,46 +240,42 @@ class DeviceSession:
             return list(x)
         return [x]
 
-    @staticmethod
-    def _checked(ts, what):
-        for t in ts:
-            if t is None:
-                continue
-            if not t.is_cuda:
-                raise ValueError(f"{what}: CUDA tensor expected")
-            if not t.is_contiguous():
-                raise ValueError(f"{what}: contiguous tensor expected")
-        return ts
-
     def _stream(self, stream):
         s = torch.cuda.current_stream(self.device) if stream is None else stream
         return ctypes.c_void_p(s.cuda_stream)
 
+    def _raw_stream(self, stream):
+        if stream is None:
+            return torch._C._cuda_getCurrentRawStream(self._device_index)
+        return stream.cuda_stream
+
     def all_reduce(self, tensor, out=None, op="sum", scale=None, algo=None, stream=None):
         """out = scale * reduce(tensor over ranks); in place when `out` is None."""
-        ins = self._checked(self._per_rank(tensor, "tensor"), "all_reduce")
-        outs = ins if out is None else self._checked(self._per_rank(out, "out"), "all_reduce")
-        t0 = ins[0]
-        self._profiled("all_reduce", t0.numel() * t0.element_size(), stream,
-                       lambda: _native.check(self._lib.stdmlc_dw_all_reduce(
-                           self._h, _ptr_array(ins), _ptr_array(outs), t0.numel(),
-                           dtype_code(t0.dtype), op_code(op),
-                           1.0 if scale is None else float(scale), _algo_code(algo),
-                           self._stream(stream))))
+        if self._prof is not None:
+            with self._recorded("all_reduce", self._nbytes(tensor), stream):
+                self._all_reduce(tensor, out, op, scale, algo, stream)
+        else:
+            self._all_reduce(tensor, out, op, scale, algo, stream)
         return out if out is not None else tensor
+
+    def _all_reduce(self, tensor, out, op, scale, algo, stream):
+        rc = self._fast.all_reduce(self._hv, self.vranks, tensor, out, op_code(op), scale,
+                                   _algo_code(algo), self._raw_stream(stream))
+        if rc:
+            _native.check(rc)
 
     def reduce(self, tensor, out=None, op="sum", root=0, scale=None, stream=None):
         """Reduce to `root`; other ranks' `out` is left untouched (may be None)."""
-        ins = self._checked(self._per_rank(tensor, "tensor"), "reduce")
-        if out is None:
-            outs = [t if (self.vranks > 1 and i == root) or (self.vranks == 1 and self.rank == root)
-                    else None for i, t in enumerate(ins)]
+        if out is not None:
+            outs = out
+        elif self.vranks > 1:
+            outs = [t if i == root else None for i, t in enumerate(tensor)]
         else:
-            outs = self._checked(self._per_rank(out, "out"), "reduce")
-        t0 = ins[0]
-        _native.check(self._lib.stdmlc_dw_reduce(
-            self._h, _ptr_array(ins), _ptr_array(outs), t0.numel(), dtype_code(t0.dtype),
-            op_code(op), root, 1.0 if scale is None else float(scale), self._stream(stream)))
+            outs = tensor if self.rank == root else None
+        rc = self._fast.reduce(self._hv, self.vranks, tensor, outs, op_code(op), root, scale,
+                               self._raw_stream(stream))
+        if rc:
+            _native.check(rc)
         return out if out is not None else tensor
 
     def group_all_reduce(self, tensors, outs=None, op="sum", scale=None, wire_dtype=None,
@@ -283,100 +284,73 @@ class DeviceSession:
 
         `wire_dtype` (bf16/f16) sends f32 tensors as 16-bit floats (cast fused into
         the pack/unpack phases).  Loopback: `tensors[rank][i]`."""
-        # The same tensors are usually passed every step (a model's gradients):
-        # the prepared pointer table is kept, keyed by every data pointer and
-        # element count of the call, so a step costs one pass over the list and
-        # one native call instead of the checks and conversions below.
-        cache = getattr(self, "_group_cache", None)
-        if cache is None:
-            cache = self._group_cache = {}
-        if outs is None and self.vranks == 1 and isinstance(tensors, list) and tensors:
-            key = (tuple([t.data_ptr() for t in tensors]), tuple([t.numel() for t in tensors]),
-                   tensors[0].dtype, wire_dtype)
-            hit = cache.get(key)
-            if hit is not None:
-                n, arr, counts, wire, user, nbytes = hit
-                self._profiled("group_all_reduce", nbytes, stream,
-                               lambda: _native.check(self._lib.stdmlc_dw_group_all_reduce(
-                                   self._h, n, arr, arr, counts, wire, op_code(op), user,
-                                   1.0 if scale is None else float(scale), _algo_code(algo),
-                                   self._stream(stream))))
-                return tensors
+        ins, dsts = self._lists(tensors), None if outs is None else self._lists(outs)
+        if self._prof is not None:
+            flat = ins[0] if self.vranks > 1 else ins
+            with self._recorded("group_all_reduce",
+                                sum(t.numel() * t.element_size() for t in flat), stream):
+                self._group_all_reduce(ins, dsts, op, scale, wire_dtype, algo, stream)
         else:
-            key = None
-        per_rank = self._per_rank(tensors, "tensors") if self.vranks > 1 else [list(tensors)]
-        per_rank_out = per_rank if outs is None else (
-            self._per_rank(outs, "outs") if self.vranks > 1 else [list(outs)])
-        n = len(per_rank[0])
-        if n == 0:
-            return outs if outs is not None else tensors
-        dtypes = []
-        for t in per_rank[0]:
-            if t.dtype not in dtypes:
-                dtypes.append(t.dtype)
-        if len(dtypes) > 1:
-            # one fused call per dtype, each keeping the callers' order
-            for dt_ in dtypes:
-                idx = [i for i, t in enumerate(per_rank[0]) if t.dtype == dt_]
-                sub_in = [[pr[i] for i in idx] for pr in per_rank]
-                sub_out = [[pr[i] for i in idx] for pr in per_rank_out]
-                self.group_all_reduce(sub_in if self.vranks > 1 else sub_in[0],
-                                      outs=None if outs is None else
-                                      (sub_out if self.vranks > 1 else sub_out[0]),
-                                      op=op, scale=scale,
-                                      wire_dtype=wire_dtype if dt_ == torch.float32 else None,
-                                      algo=algo, stream=stream)
-            return outs if outs is not None else tensors
-        dt = per_rank[0][0].dtype
-        flat_in, flat_out = [], []
-        for r in range(len(per_rank)):
-            if len(per_rank[r]) != n or len(per_rank_out[r]) != n:
-                raise ValueError("group_all_reduce: every rank needs the same number of tensors")
-            for t in per_rank[r]:
-                if t.dtype != dt:
-                    raise ValueError("group_all_reduce: one dtype per call")
-            flat_in += self._checked(list(per_rank[r]), "group_all_reduce")
-            flat_out += self._checked(list(per_rank_out[r]), "group_all_reduce")
-        counts = (ctypes.c_ulonglong * n)(*[t.numel() for t in per_rank[0]])
-        if wire_dtype is None or wire_dtype == dt:
-            wire, user = dtype_code(dt), -1
-        else:
-            wire, user = dtype_code(wire_dtype), dtype_code(dt)
-        nbytes = sum(t.numel() * t.element_size() for t in per_rank[0])
-        if key is not None:
-            if len(cache) > 64:
-                cache.clear()
-            arr = _ptr_array(flat_in)
-            cache[key] = (n, arr, counts, wire, user, nbytes)
-        self._profiled("group_all_reduce", nbytes, stream,
-                       lambda: _native.check(self._lib.stdmlc_dw_group_all_reduce(
-                           self._h, n, _ptr_array(flat_in), _ptr_array(flat_out), counts, wire,
-                           op_code(op), user, 1.0 if scale is None else float(scale),
-                           _algo_code(algo), self._stream(stream))))
+            self._group_all_reduce(ins, dsts, op, scale, wire_dtype, algo, stream)
         return outs if outs is not None else tensors
+
+    def _lists(self, x):
+        """Tensors of a group as lists or tuples (per rank in a loopback session)."""
+        if self.vranks > 1:
+            if isinstance(x, (list, tuple)) and not all(
+                    [isinstance(y, (list, tuple)) for y in x]):
+                return [list(y) for y in x]
+            return x
+        return x if isinstance(x, (list, tuple)) else list(x)
+
+    def _group_all_reduce(self, ins, outs, op, scale, wire_dtype, algo, stream):
+        rc = self._fast.group_all_reduce(
+            self._hv, self.vranks, ins, outs, -1 if wire_dtype is None else dtype_code(wire_dtype),
+            op_code(op), scale, _algo_code(algo), self._raw_stream(stream))
+        if rc == 0:
+            return
+        if rc != self._fast.MIXED_DTYPES:
+            _native.check(rc)
+        # one fused call per dtype, each keeping the callers' order
+        per_rank = ins if self.vranks > 1 else [ins]
+        per_rank_out = outs if self.vranks > 1 or outs is None else [outs]
+        for dt in dict.fromkeys(t.dtype for t in per_rank[0]):
+            idx = [i for i, t in enumerate(per_rank[0]) if t.dtype == dt]
+            sub = [[pr[i] for i in idx] for pr in per_rank]
+            sub_out = None if outs is None else [[pr[i] for i in idx] for pr in per_rank_out]
+            if self.vranks == 1:
+                sub, sub_out = sub[0], None if outs is None else sub_out[0]
+            self._group_all_reduce(sub, sub_out, op, scale,
+                                   wire_dtype if dt == torch.float32 else None, algo, stream)
 
     def all_gather(self, tensor, out, stream=None):
         """out[r * n:(r + 1) * n] = rank r's tensor (rank-major, as the reference)."""
-        ins = self._checked(self._per_rank(tensor, "tensor"), "all_gather")
-        outs = self._checked(self._per_rank(out, "out"), "all_gather")
-        t0 = ins[0]
-        if outs[0].numel() != t0.numel() * self.world:
-            raise ValueError("all_gather: out must hold world * tensor.numel() elements")
-        self._profiled("all_gather", t0.numel() * t0.element_size(), stream,
-                       lambda: _native.check(self._lib.stdmlc_dw_all_gather(
-                           self._h, _ptr_array(ins), _ptr_array(outs), t0.numel(),
-                           dtype_code(t0.dtype), self._stream(stream))))
+        if self._prof is not None:
+            with self._recorded("all_gather", self._nbytes(tensor), stream):
+                self._all_gather(tensor, out, stream)
+        else:
+            self._all_gather(tensor, out, stream)
         return out
 
+    def _all_gather(self, tensor, out, stream):
+        rc = self._fast.all_gather(self._hv, self.vranks, self.world, tensor, out,
+                                   self._raw_stream(stream))
+        if rc:
+            _native.check(rc)
+
     def broadcast(self, tensor, out=None, root=0, stream=None):
-        ins = self._checked(self._per_rank(tensor, "tensor"), "broadcast")
-        outs = ins if out is None else self._checked(self._per_rank(out, "out"), "broadcast")
-        t0 = ins[0]
-        self._profiled("broadcast", t0.numel() * t0.element_size(), stream,
-                       lambda: _native.check(self._lib.stdmlc_dw_broadcast(
-                           self._h, _ptr_array(ins), _ptr_array(outs), t0.numel(),
-                           dtype_code(t0.dtype), root, self._stream(stream))))
+        if self._prof is not None:
+            with self._recorded("broadcast", self._nbytes(tensor), stream):
+                self._broadcast(tensor, out, root, stream)
+        else:
+            self._broadcast(tensor, out, root, stream)
         return out if out is not None else tensor
+
+    def _broadcast(self, tensor, out, root, stream):
+        rc = self._fast.broadcast(self._hv, self.vranks, tensor, out, root,
+                                  self._raw_stream(stream))
+        if rc:
+            _native.check(rc)
 
     def barrier(self, stream=None):
         _native.check(self._lib.stdmlc_dw_barrier(self._h, self._stream(stream)))
@@ -447,21 +421,22 @@ class DeviceSession:
         (include/stdml/bits/collective/stat.hpp:196-202), which time the host."""
         self._prof = [] if on else None
 
-    def _profiled(self, name, nbytes, stream, call):
-        prof = getattr(self, "_prof", None)
-        if prof is None:
-            return call()
+    def _nbytes(self, tensor):
+        t = tensor[0] if self.vranks > 1 else tensor
+        return t.numel() * t.element_size()
+
+    @contextlib.contextmanager
+    def _recorded(self, name, nbytes, stream):
         s = torch.cuda.current_stream(self.device) if stream is None else stream
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         e0.record(s)
-        out = call()
+        yield
         e1.record(s)
-        prof.append((name, nbytes, e0, e1))
-        return out
+        self._prof.append((name, nbytes, e0, e1))
 
     def profile_summary(self, reset=True):
         """{op: {calls, bytes, ms, algbw_gb_s, busbw_gb_s}}; waits for the recorded work."""
-        prof = getattr(self, "_prof", None) or []
+        prof = self._prof or []
         out = {}
         n = self.world
         factor = {"all_reduce": 2 * (n - 1) / n, "group_all_reduce": 2 * (n - 1) / n,
@@ -476,7 +451,7 @@ class DeviceSession:
             sec = max(d["ms"], 1e-9) * 1e-3
             d["algbw_gb_s"] = d["bytes"] / sec / 1e9
             d["busbw_gb_s"] = d["algbw_gb_s"] * factor.get(name, 1.0)
-        if reset and getattr(self, "_prof", None) is not None:
+        if reset and self._prof is not None:
             self._prof = []
         return out
 
