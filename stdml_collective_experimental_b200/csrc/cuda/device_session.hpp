@@ -20,6 +20,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "device_world.hpp"
@@ -132,13 +133,15 @@ class DeviceSession
         int n = 0;
         size_t nvec = 0;
         unsigned long long stamp = 0;
+        // one pointer into each allocation that holds a tensor of the set, and its id
+        std::vector<std::pair<const void *, unsigned long long>> allocations;
     };
     std::map<std::string, PeerPlan> peer_plans_;
     unsigned long long peer_plan_builds_ = 0;
-    // Look up the allocation id behind every tensor on every call (one driver query
-    // per tensor), so that a tensor freed and allocated again at the same address
+    // Look up the allocation ids behind the tensors on every call (one driver query
+    // per allocation), so that a tensor freed and allocated again at the same address
     // is noticed.  Knob register_verify = 0 trusts the addresses instead (for sets of
-    // thousands of tensors in allocations that are never freed).
+    // thousands of allocations that are never freed).
     bool register_verify_ = true;
     void forget_peer_plans();
     // Returns false when the set has to be staged (decided alike on every rank).

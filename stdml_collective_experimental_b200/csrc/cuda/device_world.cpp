@@ -588,6 +588,18 @@ class World final : public DeviceWorld
         return id;
     }
 
+    const void *allocation_base(const void *p) const override
+    {
+        Driver &d = driver();
+        CUdeviceptr base = 0;
+        size_t size = 0;
+        if (p == nullptr || d.MemGetAddressRange == nullptr ||
+            d.MemGetAddressRange(&base, &size, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) {
+            return nullptr;
+        }
+        return reinterpret_cast<const void *>(base);
+    }
+
     void drop_registrations() override
     {
         if (opt_.loopback || opt_.world == 1) { return; }

@@ -140,6 +140,8 @@ class DeviceWorld
     // A number that identifies the allocation behind `p` and is never used twice
     // in a process (0: not a device allocation the driver knows).
     virtual unsigned long long buffer_id(const void *p) const = 0;
+    // Start of the allocation that holds `p` (null: the driver does not know one).
+    virtual const void *allocation_base(const void *p) const = 0;
     // Collective: unmaps every peer buffer imported so far.
     virtual void drop_registrations() = 0;
     virtual size_t registrations() const = 0;  // peer allocations mapped now
