@@ -128,6 +128,11 @@ struct GroupEntry {
     unsigned long long count;
 };
 
+// Vectors per block of the copies of a world of one GPU.
+constexpr int kLocalThreads = 1024;
+constexpr int kLocalUnroll = 2;
+constexpr unsigned long long kLocalTile = static_cast<unsigned long long>(kLocalThreads) * kLocalUnroll;
+
 struct AllReduceArgs {
     // Per virtual rank (index blockIdx.y); real multi-GPU launches use [0].
     const void *src[kMaxRanks];  // nullptr: input already at arena offset `off`
@@ -244,5 +249,12 @@ int launch_group_peer(const CommCtx &ctx, const GroupPeerArgs &a, int dt, int op
                       int vranks, void *stream);
 // world of one GPU: dst = scale * src (integers: copy), no arena involved
 int launch_local_scale(const void *src, void *dst, unsigned long long count, int dt, double scale,
-                       int has_scale, int sms, void *stream);
+                       int has_scale, void *stream);
+// the same for a fused group of tensors (user_dt: see AllReduceArgs::user_dtype).
+// first_of_tile[t]: entry that holds vector t * kLocalTile, one more element than
+// tiles (the last: the last entry).  chained: an independent piece of the same
+// call was launched just before on this stream and may still be running.
+int launch_local_group(const GroupEntry *table, const int *first_of_tile, unsigned long long nvec,
+                       int dt, int user_dt, double scale, int has_scale, bool chained,
+                       void *stream);
 }  // namespace stdml::collective::cuda

@@ -637,13 +637,30 @@ const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *
                 host[j].voff = p.voff;
                 host[j].count = p.count;
             }
+            std::vector<int> first_of_tile;
+            if (world_->world() == 1) {
+                size_t j = 0;
+                for (size_t at = 0; at < nvec; at += kLocalTile) {
+                    while (j + 1 < pieces.size() && pieces[j + 1].voff <= at) { ++j; }
+                    first_of_tile.push_back(static_cast<int>(j));
+                }
+                first_of_tile.push_back(static_cast<int>(pieces.size()) - 1);
+            }
+            const size_t tab_bytes = host.size() * sizeof(GroupEntry);
+            std::vector<char> image(tab_bytes + first_of_tile.size() * sizeof(int));
+            std::memcpy(image.data(), host.data(), tab_bytes);
+            std::memcpy(image.data() + tab_bytes, first_of_tile.data(),
+                        first_of_tile.size() * sizeof(int));
             void *dev = nullptr;
-            rt_check(cudaMalloc(&dev, host.size() * sizeof(GroupEntry)), "cudaMalloc(table)");
+            rt_check(cudaMalloc(&dev, image.size()), "cudaMalloc(table)");
             table_mem_.push_back(dev);
-            rt_check(cudaMemcpy(dev, host.data(), host.size() * sizeof(GroupEntry),
-                                cudaMemcpyHostToDevice),
+            rt_check(cudaMemcpy(dev, image.data(), image.size(), cudaMemcpyHostToDevice),
                      "cudaMemcpy(table)");
             per_rank[v].dev = static_cast<GroupEntry *>(dev);
+            if (!first_of_tile.empty()) {
+                per_rank[v].first_of_tile =
+                    reinterpret_cast<const int *>(static_cast<const char *>(dev) + tab_bytes);
+            }
             per_rank[v].n = static_cast<int>(host.size());
             per_rank[v].nvec = nvec;
         }
@@ -839,6 +856,7 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         return;
     }
     std::vector<const GroupEntry *> tabs(vr);
+    const bool in_capture = capturing(stream);
     for (const auto &chunk : plan.chunks) {
         for (int v = 0; v < vr; ++v) { tabs[v] = chunk[v].dev; }
         AllReduceCall c;
@@ -852,7 +870,9 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         c.has_scale = scale != 1.0;
         c.scale = scale;
         c.algo = algo;
-        c.end_barrier = capturing(stream);
+        c.end_barrier = in_capture;
+        c.first_of_tile = chunk[0].first_of_tile;
+        c.chained = &chunk != &plan.chunks.front() && !in_capture;
         launch_ar(c, stream);
     }
 }

@@ -99,6 +99,7 @@ class DeviceSession
         GroupEntry *dev = nullptr;
         int n = 0;
         size_t nvec = 0;
+        const int *first_of_tile = nullptr;  // world of one GPU: AllReduceCall::first_of_tile
     };
     struct GroupPlan {
         std::vector<std::vector<Table>> chunks;  // [chunk][vrank]

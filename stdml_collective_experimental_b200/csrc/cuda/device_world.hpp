@@ -63,6 +63,10 @@ struct AllReduceCall {
     void *const *dst = nullptr;
     const GroupEntry *const *table = nullptr;  // device pointers, one per vrank
     int ntable = 0;
+    // A world of one GPU: the table entry in which each tile starts (see launch_local_group),
+    // and whether the piece of the same call before this one may still be running.
+    const int *first_of_tile = nullptr;
+    bool chained = false;
     size_t count = 0;  // elements; for a group: flat length in wire elements
     int dt = 0;
     int op = 0;
