@@ -710,7 +710,6 @@ __device__ __forceinline__ bool tma_reduce_span(const CommCtx &ctx, const AllRed
     if (!ok) {
         if (threadIdx.x == 0) {
             report_timeout(ctx, rank, -1, 0u, 0u, 64 + sync->phase);
-            *reinterpret_cast<volatile int *>(&sync->failed) = 1;
             // copies already issued still write into this CTA's shared memory: give
             // them one more (bounded) chance to land before the CTA goes away
             for (unsigned long long t = in_flight_from;

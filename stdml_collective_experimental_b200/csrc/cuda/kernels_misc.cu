@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(kThreads)
                                            if (src != nullptr) { st_arena_v4(mine + v * 16ull, x); }
                                        });
                 }
-                signal_from(ctx, rank, &sync, k);
+                arrive_all(ctx, rank, &sync, k + 1);
             } else {
                 if (!wait_for(ctx, rank, a.root, &sync, k)) { return; }
                 for_each_block_vec(nullptr, mine, a.bytes, piece(my_slice, k),

@@ -2,9 +2,8 @@
 // 16-byte peer loads/stores, NVLS multimem wrappers, the bounded cross-rank
 // block barrier, and per-dtype vector arithmetic.
 //
-// Remote data is always fetched by the CTA itself with plain vector loads over
-// the peer mapping or with multimem instructions through the switch; there is
-// no bulk/TMA copy in this data plane.
+// These primitives fetch remote data with plain vector loads over the peer mapping
+// or with multimem instructions through the switch; the bulk copies are in ar_kernel.cuh.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -62,29 +61,32 @@ __device__ __forceinline__ unsigned long long global_ns()
 // ------------------------------------------------------------ block barrier
 struct BlockSync {
     uint32_t epoch;  // barriers this block index has passed (all launches)
-    int failed;
     int phase;
 };
+
+// The thread that looks after the epoch.  It reads it from global memory at the
+// start, which takes as long as the block's first data loads: a thread of the last
+// warp, which small messages leave idle, so that the two waits overlap.
+constexpr unsigned int kSyncThread = kThreads - 1;
 
 __device__ __forceinline__ SignalPad *pad_of(const CommCtx &ctx, int r)
 {
     return reinterpret_cast<SignalPad *>(ctx.base[r]);
 }
 
+// No __syncthreads here: everything that reads the epoch comes after one of its own.
 __device__ __forceinline__ void sync_begin(const CommCtx &ctx, int rank, BlockSync *s)
 {
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == kSyncThread) {
         s->epoch = pad_of(ctx, rank)->epoch[blockIdx.x];
-        s->failed = 0;
         s->phase = 0;
     }
-    __syncthreads();
 }
 
+// Only a block all of whose waits came through gets here.
 __device__ __forceinline__ void sync_end(const CommCtx &ctx, int rank, BlockSync *s)
 {
-    __syncthreads();
-    if (threadIdx.x == 0 && !s->failed) { pad_of(ctx, rank)->epoch[blockIdx.x] = s->epoch; }
+    if (threadIdx.x == kSyncThread) { pad_of(ctx, rank)->epoch[blockIdx.x] = s->epoch; }
 }
 
 static __device__ __noinline__ void report_timeout(const CommCtx &ctx, int rank, int peer,
@@ -106,97 +108,91 @@ static __device__ __noinline__ void report_timeout(const CommCtx &ctx, int rank,
     }
 }
 
-// Barrier between the blocks with the same blockIdx.x on every rank.  Thread p
-// (p < world) publishes this block's arrival to rank p with a release store and
-// waits, with a time and an iteration limit, for rank p's arrival with acquire
-// loads.  Writes made by any thread of the block before the call are visible
-// to the peers' threads after their call returns.  Returns false (for the whole
-// block) when a wait ran out; the caller must then skip its remaining work.
-__device__ __forceinline__ bool peer_barrier(const CommCtx &ctx, int rank, BlockSync *s)
+// One thread waits until rank src's flag for this block has reached `target`,
+// with a time and an iteration limit.  False: the limit was reached (reported).
+__device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src, uint32_t target,
+                                          int phase)
 {
-    __syncthreads();
-    const uint32_t target = s->epoch + 1u;
-    const int p = static_cast<int>(threadIdx.x);
-    if (p < ctx.world) {
-        st_release_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank], target);
-        const uint32_t *f = &pad_of(ctx, rank)->flag[blockIdx.x][p];
-        unsigned int spins = 0;
-        unsigned long long t0 = 0;
-        for (;;) {
-            const uint32_t seen = ld_acquire_sys_u32(f);
-            if (static_cast<int32_t>(seen - target) >= 0) { break; }
-            ++spins;
-            if ((spins & 127u) == 0u) {
-                const unsigned long long now = global_ns();
-                if (t0 == 0) { t0 = now; }
-                if (now - t0 > ctx.timeout_ns || spins >= ctx.max_spins) {
-                    report_timeout(ctx, rank, p, target, seen, s->phase);
-                    *reinterpret_cast<volatile int *>(&s->failed) = 1;
-                    break;
-                }
+    const uint32_t *f = &pad_of(ctx, rank)->flag[blockIdx.x][src];
+    unsigned int spins = 0;
+    unsigned long long t0 = 0;
+    for (;;) {
+        const uint32_t seen = ld_acquire_sys_u32(f);
+        if (static_cast<int32_t>(seen - target) >= 0) { return true; }
+        ++spins;
+        if ((spins & 127u) == 0u) {
+            const unsigned long long now = global_ns();
+            if (t0 == 0) { t0 = now; }
+            if (now - t0 > ctx.timeout_ns || spins >= ctx.max_spins) {
+                report_timeout(ctx, rank, src, target, seen, phase);
+                return false;
             }
         }
     }
-    __syncthreads();
-    const bool ok = (*reinterpret_cast<volatile int *>(&s->failed) == 0);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        s->epoch = target;
-        s->phase += 1;
-    }
-    return ok;
 }
 
-// One-way signals on the barrier's flags, for kernels in which one rank feeds
-// the others in rounds.  signal_from(): this block of `rank` tells block
-// blockIdx.x of every rank that everything its threads stored so far is in
-// place (value = epoch + round + 1).  wait_for(): the others wait for it, with
-// the barrier's limits.  After `rounds` rounds every rank calls rounds_done(),
-// so that the next full barrier of all ranks starts from the same epoch.
-__device__ __forceinline__ void signal_from(const CommCtx &ctx, int rank, BlockSync *s, int round)
+// The two halves of a barrier between the blocks with the same blockIdx.x on every
+// rank; `nth` counts from the kernel's current epoch, starting at 1.
+// arrive_all: thread p (p < world) tells rank p, with a release store, that this
+// block has arrived: writes made by any of its threads before are visible to whoever waits.
+// wait_all: thread p waits for rank p's arrival with acquire loads.  False (for
+// the whole block) when a wait ran out: the caller then skips its remaining work.
+// Work placed between the two hides the latency of the flags.
+__device__ __forceinline__ void arrive_all(const CommCtx &ctx, int rank, BlockSync *s, int nth)
 {
     __syncthreads();
     const int p = static_cast<int>(threadIdx.x);
     if (p < ctx.world) {
         st_release_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank],
-                           s->epoch + static_cast<uint32_t>(round) + 1u);
+                           s->epoch + static_cast<uint32_t>(nth));
     }
 }
 
+__device__ __forceinline__ bool wait_all(const CommCtx &ctx, int rank, BlockSync *s, int nth)
+{
+    bool ok = true;
+    const int p = static_cast<int>(threadIdx.x);
+    if (p < ctx.world) {
+        ok = poll_flag(ctx, rank, p, s->epoch + static_cast<uint32_t>(nth), s->phase);
+    }
+    return __syncthreads_and(ok ? 1 : 0) != 0;
+}
+
+// After waits up to `nth`: the next barrier of all ranks starts from there.
+__device__ __forceinline__ void advance_epoch(BlockSync *s, int nth)
+{
+    if (threadIdx.x == kSyncThread) {
+        s->epoch += static_cast<uint32_t>(nth);
+        s->phase += 1;
+    }
+}
+
+__device__ __forceinline__ bool peer_barrier(const CommCtx &ctx, int rank, BlockSync *s)
+{
+    arrive_all(ctx, rank, s, 1);
+    const bool ok = wait_all(ctx, rank, s, 1);
+    advance_epoch(s, 1);
+    return ok;
+}
+
+// One-way signals on the barrier's flags, for kernels in which one rank feeds
+// the others in rounds: the feeder calls arrive_all(round + 1), the others wait
+// for it here.  After `rounds` rounds every rank calls rounds_done(), so that the
+// next full barrier of all ranks starts from the same epoch.
 __device__ __forceinline__ bool wait_for(const CommCtx &ctx, int rank, int src, BlockSync *s,
                                          int round)
 {
-    if (threadIdx.x == 0) {
-        const uint32_t target = s->epoch + static_cast<uint32_t>(round) + 1u;
-        const uint32_t *f = &pad_of(ctx, rank)->flag[blockIdx.x][src];
-        unsigned int spins = 0;
-        unsigned long long t0 = 0;
-        for (;;) {
-            const uint32_t seen = ld_acquire_sys_u32(f);
-            if (static_cast<int32_t>(seen - target) >= 0) { break; }
-            ++spins;
-            if ((spins & 127u) == 0u) {
-                const unsigned long long now = global_ns();
-                if (t0 == 0) { t0 = now; }
-                if (now - t0 > ctx.timeout_ns || spins >= ctx.max_spins) {
-                    report_timeout(ctx, rank, src, target, seen, 32 + round);
-                    *reinterpret_cast<volatile int *>(&s->failed) = 1;
-                    break;
-                }
-            }
-        }
+    bool ok = true;
+    if (threadIdx.x == kSyncThread) {
+        ok = poll_flag(ctx, rank, src, s->epoch + static_cast<uint32_t>(round) + 1u, 32 + round);
     }
-    __syncthreads();
-    const bool ok = (*reinterpret_cast<volatile int *>(&s->failed) == 0);
-    __syncthreads();
-    return ok;
+    return __syncthreads_and(ok ? 1 : 0) != 0;
 }
 
 __device__ __forceinline__ void rounds_done(BlockSync *s, int rounds)
 {
     __syncthreads();
-    if (threadIdx.x == 0) { s->epoch += static_cast<uint32_t>(rounds); }
-    __syncthreads();
+    if (threadIdx.x == kSyncThread) { s->epoch += static_cast<uint32_t>(rounds); }
 }
 
 // ------------------------------------------------------------- dtype traits
