@@ -72,6 +72,7 @@ struct CommCtx {
     unsigned int max_spins;  // hard iteration limit of one wait
     int world;
     int rank;  // rank served by blockIdx.y == 0 (virtual ranks: rank + blockIdx.y)
+    int one_gpu;  // all ranks are on this GPU (loopback): flags need GPU scope only
 };
 
 enum : int {

@@ -671,6 +671,7 @@ class World final : public DeviceWorld
         ctx.max_spins = 1u << 30;
         ctx.world = opt_.world;
         ctx.rank = opt_.loopback ? 0 : opt_.rank;
+        ctx.one_gpu = opt_.loopback ? 1 : 0;
         return ctx;
     }
 

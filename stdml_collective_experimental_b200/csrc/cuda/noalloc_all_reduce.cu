@@ -162,6 +162,7 @@ extern "C" int stdmlc_all_reduce_noalloc(const void *const *in, void *const *out
     ctx.max_spins = 1u << 28;
     ctx.world = nranks;
     ctx.rank = 0;
+    ctx.one_gpu = 1;
 
     AllReduceArgs a;
     std::memset(&a, 0, sizeof(a));

@@ -20,16 +20,30 @@ enum : int { DT_I8, DT_I16, DT_I32, DT_I64, DT_U8, DT_U16, DT_U32, DT_U64, DT_BF
 enum : int { OP_SUM, OP_MIN, OP_MAX, OP_PROD, OP_XOR };
 
 // ---------------------------------------------------------------- memory ops
-__device__ __forceinline__ void st_release_sys_u32(uint32_t *p, uint32_t v)
+// Flags: relaxed accesses beside explicit fences.  (A polling ld.acquire would
+// invalidate the SM's L1 on every look, for all its blocks; the fence after the
+// last look does it once.)
+__device__ __forceinline__ void st_relaxed_sys_u32(uint32_t *p, uint32_t v)
 {
-    asm volatile("st.release.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+    asm volatile("st.relaxed.sys.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-__device__ __forceinline__ uint32_t ld_acquire_sys_u32(const uint32_t *p)
+__device__ __forceinline__ uint32_t ld_relaxed_sys_u32(const uint32_t *p)
 {
     uint32_t v;
-    asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    asm volatile("ld.relaxed.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
+}
+
+// Orders this thread's accesses before it against those after it as seen by the
+// other ranks: system scope, or GPU scope where all ranks are on this GPU.
+__device__ __forceinline__ void fence_ranks(const CommCtx &ctx)
+{
+    if (ctx.one_gpu) {
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+    } else {
+        asm volatile("fence.acq_rel.sys;" ::: "memory");
+    }
 }
 
 // Coherent 16-byte load (bypasses L1): used for every read of arena memory,
@@ -67,7 +81,7 @@ struct BlockSync {
 // The thread that looks after the epoch.  It reads it from global memory at the
 // start, which takes as long as the block's first data loads: a thread of the last
 // warp, which small messages leave idle, so that the two waits overlap.
-constexpr unsigned int kSyncThread = kThreads - 1;
+__device__ __forceinline__ bool is_sync_thread() { return threadIdx.x == blockDim.x - 1u; }
 
 __device__ __forceinline__ SignalPad *pad_of(const CommCtx &ctx, int r)
 {
@@ -77,7 +91,7 @@ __device__ __forceinline__ SignalPad *pad_of(const CommCtx &ctx, int r)
 // No __syncthreads here: everything that reads the epoch comes after one of its own.
 __device__ __forceinline__ void sync_begin(const CommCtx &ctx, int rank, BlockSync *s)
 {
-    if (threadIdx.x == kSyncThread) {
+    if (is_sync_thread()) {
         s->epoch = pad_of(ctx, rank)->epoch[blockIdx.x];
         s->phase = 0;
     }
@@ -86,7 +100,7 @@ __device__ __forceinline__ void sync_begin(const CommCtx &ctx, int rank, BlockSy
 // Only a block all of whose waits came through gets here.
 __device__ __forceinline__ void sync_end(const CommCtx &ctx, int rank, BlockSync *s)
 {
-    if (threadIdx.x == kSyncThread) { pad_of(ctx, rank)->epoch[blockIdx.x] = s->epoch; }
+    if (is_sync_thread()) { pad_of(ctx, rank)->epoch[blockIdx.x] = s->epoch; }
 }
 
 static __device__ __noinline__ void report_timeout(const CommCtx &ctx, int rank, int peer,
@@ -117,8 +131,11 @@ __device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src,
     unsigned int spins = 0;
     unsigned long long t0 = 0;
     for (;;) {
-        const uint32_t seen = ld_acquire_sys_u32(f);
-        if (static_cast<int32_t>(seen - target) >= 0) { return true; }
+        const uint32_t seen = ld_relaxed_sys_u32(f);
+        if (static_cast<int32_t>(seen - target) >= 0) {
+            fence_ranks(ctx);
+            return true;
+        }
         ++spins;
         if ((spins & 127u) == 0u) {
             const unsigned long long now = global_ns();
@@ -133,9 +150,9 @@ __device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src,
 
 // The two halves of a barrier between the blocks with the same blockIdx.x on every
 // rank; `nth` counts from the kernel's current epoch, starting at 1.
-// arrive_all: thread p (p < world) tells rank p, with a release store, that this
+// arrive_all: thread p (p < world) tells rank p, with a fence and a store, that this
 // block has arrived: writes made by any of its threads before are visible to whoever waits.
-// wait_all: thread p waits for rank p's arrival with acquire loads.  False (for
+// wait_all: thread p waits for rank p's arrival.  False (for
 // the whole block) when a wait ran out: the caller then skips its remaining work.
 // Work placed between the two hides the latency of the flags.
 __device__ __forceinline__ void arrive_all(const CommCtx &ctx, int rank, BlockSync *s, int nth)
@@ -143,7 +160,8 @@ __device__ __forceinline__ void arrive_all(const CommCtx &ctx, int rank, BlockSy
     __syncthreads();
     const int p = static_cast<int>(threadIdx.x);
     if (p < ctx.world) {
-        st_release_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank],
+        fence_ranks(ctx);
+        st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank],
                            s->epoch + static_cast<uint32_t>(nth));
     }
 }
@@ -161,7 +179,7 @@ __device__ __forceinline__ bool wait_all(const CommCtx &ctx, int rank, BlockSync
 // After waits up to `nth`: the next barrier of all ranks starts from there.
 __device__ __forceinline__ void advance_epoch(BlockSync *s, int nth)
 {
-    if (threadIdx.x == kSyncThread) {
+    if (is_sync_thread()) {
         s->epoch += static_cast<uint32_t>(nth);
         s->phase += 1;
     }
@@ -183,7 +201,7 @@ __device__ __forceinline__ bool wait_for(const CommCtx &ctx, int rank, int src, 
                                          int round)
 {
     bool ok = true;
-    if (threadIdx.x == kSyncThread) {
+    if (is_sync_thread()) {
         ok = poll_flag(ctx, rank, src, s->epoch + static_cast<uint32_t>(round) + 1u, 32 + round);
     }
     return __syncthreads_and(ok ? 1 : 0) != 0;
@@ -192,7 +210,7 @@ __device__ __forceinline__ bool wait_for(const CommCtx &ctx, int rank, int src, 
 __device__ __forceinline__ void rounds_done(BlockSync *s, int rounds)
 {
     __syncthreads();
-    if (threadIdx.x == kSyncThread) { s->epoch += static_cast<uint32_t>(rounds); }
+    if (is_sync_thread()) { s->epoch += static_cast<uint32_t>(rounds); }
 }
 
 // ------------------------------------------------------------- dtype traits
