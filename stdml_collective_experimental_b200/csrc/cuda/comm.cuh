@@ -120,6 +120,16 @@ inline void tma_geometry(int world, unsigned int want_tile_vec, int *stages,
     *smem_bytes = st * static_cast<unsigned int>(world) * tv * 16u;
 }
 
+// The staged all-reduce (staged_kernel.cuh): pieces of its ring per block, and
+// vectors that a block packs, reduces and unpacks per round over all shards.
+constexpr int kStagedRing = 3;
+constexpr int kStagedThreads = 256;
+constexpr int kStagedPerSm = 4;
+constexpr int kStagedStepShift = 8;  // smallest tile: one vector per thread
+static_assert(1 << kStagedStepShift == kStagedThreads, "a step is one vector per thread");
+constexpr int kStagedStarts = 1024;  // table entries searched in shared memory
+constexpr unsigned int kStagedRoundVec = 2048;
+
 // One tensor of a fused group: `count` elements that live at vector offset
 // `voff` (16-byte units) of the flat symmetric region.
 struct GroupEntry {
@@ -199,6 +209,24 @@ struct GroupPeerArgs {
     unsigned int tma_tile_vec;
 };
 
+struct StagedArgs {
+    // Per virtual rank (index blockIdx.y); real multi-GPU launches use [0].
+    const void *src[kMaxRanks];
+    void *dst[kMaxRanks];
+    const GroupEntry *table[kMaxRanks];  // non-null: fused group, src/dst unused
+    unsigned long long off;    // arena offset of the staging slot
+    unsigned long long count;  // elements (single buffer)
+    unsigned long long nvec;   // 16-byte vectors
+    int ntable;
+    int user_dtype;  // as in AllReduceArgs
+    int has_scale;
+    double scale;
+    int tile_shift;  // vectors per tile: 1 << tile_shift
+    int rounds;      // tiles per block and shard
+    unsigned long long slot_bytes;  // of the staging slot
+    int debug_checks;               // as in AllReduceArgs
+};
+
 enum : int { kPhasePack = 1, kPhaseReduce = 2, kPhaseUnpack = 4, kPhaseAll = 7 };
 
 struct GatherArgs {
@@ -245,6 +273,9 @@ int launch_unpack_blocks(const void *region, void *dst, unsigned long long bytes
 int launch_all_reduce(const CommCtx &ctx, const AllReduceArgs &a, int dt, int op,
                       int blocks, int vranks, void *stream);
 bool nvls_supported(int dt, int op);
+// kernels_st_*.cu: the same contract; blocks and rounds from staged_geometry()
+int launch_staged(const CommCtx &ctx, const StagedArgs &a, int dt, int op, int blocks, int vranks,
+                  void *stream);
 // kernels_group_peer.cu: two-shot over a table of registered tensors
 int launch_group_peer(const CommCtx &ctx, const GroupPeerArgs &a, int dt, int op, int blocks,
                       int vranks, void *stream);

@@ -52,6 +52,9 @@ void launch_check(int rc, const char *what)
 
 DeviceSession::DeviceSession(std::unique_ptr<DeviceWorld> world) : world_(std::move(world))
 {
+    // Three streams pay where pack and unpack can run beside transfers over links.  In a
+    // loopback world all phases share one GPU's memory, and the staged kernel overlaps them itself.
+    if (world_->vranks() > 1) { pipeline_min_bytes_ = SIZE_MAX; }
     if (const char *e = std::getenv("STDML_COLLECTIVE_PIPELINE_MIN_BYTES")) {
         pipeline_min_bytes_ = static_cast<size_t>(std::atoll(e));
     }
@@ -388,6 +391,7 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
         k.dst = dst.data();
         k.count = n;
         k.end_barrier = in_capture;
+        k.staged = true;
         launch_ar(k, stream);
     }
 }
@@ -871,6 +875,7 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         c.scale = scale;
         c.algo = algo;
         c.end_barrier = in_capture;
+        c.staged = true;
         c.first_of_tile = chunk[0].first_of_tile;
         c.chained = &chunk != &plan.chunks.front() && !in_capture;
         launch_ar(c, stream);

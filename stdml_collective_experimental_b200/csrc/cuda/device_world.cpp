@@ -16,6 +16,7 @@
 #include "algo_table.hpp"
 #include "local_rendezvous.hpp"
 #include "offset_heap.hpp"
+#include "staged_walk.hpp"
 
 namespace stdml::collective::cuda
 {
@@ -750,6 +751,11 @@ class World final : public DeviceWorld
             staged = staged || (c.table != nullptr && c.table[v] != nullptr) ||
                      (c.src != nullptr && c.src[v] != nullptr);
         }
+        if (c.staged && c.root < 0 && c.phases == kPhaseAll && opt_.world > 1 &&
+            (algo == kAlgoTwoShot || algo == kAlgoTwoShotTma)) {
+            const int rc = all_reduce_staged(c, nvec, user_dt, stream);
+            if (rc >= 0) { return rc; }  // else: the slot is too small for its ring
+        }
         int blocks = c.blocks > 0 ? c.blocks : pick_blocks(nvec, algo);
         if (c.blocks <= 0 && nvls && (staged || c.root >= 0)) {
             // the pack / unpack phases are plain HBM copies and a root-only pull
@@ -834,6 +840,40 @@ class World final : public DeviceWorld
         }
         const CommCtx ctx = make_ctx();
         const int rc = launch_all_reduce(ctx, a, c.dt, c.op, blocks, vranks_, stream);
+        if (rc < 0) { throw std::invalid_argument("all_reduce: (dtype, op) not built"); }
+        return rc;
+    }
+
+    // Peer-load two-shot of memory outside the arena: rounds over a small ring.
+    int all_reduce_staged(const AllReduceCall &c, size_t nvec, int user_dt, void *stream)
+    {
+        StagedArgs a;
+        std::memset(&a, 0, sizeof(a));
+        for (int v = 0; v < vranks_; ++v) {
+            a.src[v] = c.src != nullptr ? c.src[v] : nullptr;
+            a.dst[v] = c.dst != nullptr ? c.dst[v] : nullptr;
+            a.table[v] = c.table != nullptr ? c.table[v] : nullptr;
+            if (a.table[v] == nullptr && (a.src[v] == nullptr || a.dst[v] == nullptr)) {
+                throw std::invalid_argument("all_reduce: staged calls need a source and a destination");
+            }
+        }
+        a.off = c.off;
+        a.count = c.count;
+        a.nvec = nvec;
+        a.ntable = c.ntable;
+        a.user_dtype = user_dt;
+        a.has_scale = c.has_scale ? 1 : 0;
+        a.scale = c.scale;
+        a.slot_bytes = opt_.staging_bytes;
+        a.debug_checks = debug_checks_ ? 1 : 0;
+        // all resident (the kernel's launch bounds)
+        const int most = c.blocks > 0 ? c.blocks
+                                      : std::min(kMaxBlocks, std::max(1, kStagedPerSm * num_sms_ / vranks_));
+        const StagedGeometry g = staged_geometry(opt_.world, nvec, opt_.staging_bytes, most);
+        if (g.blocks == 0) { return -1; }
+        a.tile_shift = g.tile_shift;
+        a.rounds = g.rounds;
+        const int rc = launch_staged(make_ctx(), a, c.dt, c.op, g.blocks, vranks_, stream);
         if (rc < 0) { throw std::invalid_argument("all_reduce: (dtype, op) not built"); }
         return rc;
     }

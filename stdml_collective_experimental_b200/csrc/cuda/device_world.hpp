@@ -77,6 +77,9 @@ struct AllReduceCall {
     bool end_barrier = false;
     bool has_scale = false;
     double scale = 1.0;  // f64 buffers use all of it; other float types its f32 value
+    // `off` is a staging slot of which the call may make any use: nobody looks for
+    // the packed operands or the result there afterwards.
+    bool staged = false;
     int phases = 7;  // kPhasePack | kPhaseReduce | kPhaseUnpack
 };
 

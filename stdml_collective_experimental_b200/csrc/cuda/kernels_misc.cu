@@ -28,6 +28,19 @@ int launch_all_reduce(const CommCtx &ctx, const AllReduceArgs &a, int dt, int op
     return -1;
 }
 
+int launch_staged_f(const CommCtx &, const StagedArgs &, int, int, int, int, void *);
+int launch_staged_i(const CommCtx &, const StagedArgs &, int, int, int, int, void *);
+int launch_staged_u(const CommCtx &, const StagedArgs &, int, int, int, int, void *);
+
+int launch_staged(const CommCtx &ctx, const StagedArgs &a, int dt, int op, int blocks, int vranks,
+                  void *stream)
+{
+    if (dt >= DT_BF16 && dt <= DT_F64) { return launch_staged_f(ctx, a, dt, op, blocks, vranks, stream); }
+    if (dt >= DT_I8 && dt <= DT_I64) { return launch_staged_i(ctx, a, dt, op, blocks, vranks, stream); }
+    if (dt >= DT_U8 && dt <= DT_U64) { return launch_staged_u(ctx, a, dt, op, blocks, vranks, stream); }
+    return -1;
+}
+
 // A world of one GPU: all_reduce degenerates to out = scale * in.  No peers, no
 // barrier, no arena: an HBM copy.  One 32 KB tile per block and a grid as long as
 // the buffer: blocks start in address order as others finish, so the whole GPU

@@ -13,6 +13,7 @@
 #include "../cuda/device_session.hpp"
 #include "../cuda/algo_table.hpp"
 #include "../cuda/offset_heap.hpp"
+#include "../cuda/staged_walk.hpp"
 
 using namespace stdml::collective::cuda;
 
@@ -51,6 +52,40 @@ int main()
             EXPECT(len_max - len_min <= 2 * kSpanGranule);
         }
         EXPECT(expect == nvec);
+    }
+    // staged all-reduce: over shards, blocks and rounds the tiles cover the buffer exactly
+    // once; the ring pieces of all blocks are disjoint and stay inside the slot
+    for (int trial = 0; trial < 3000; ++trial) {
+        const unsigned long long nvec = 1 + rng() % (trial % 3 == 0 ? 70 : 3000000);
+        const int world = 2 + static_cast<int>(rng() % 15);
+        const size_t slot = (size_t{4096} << (rng() % 15)) + 4096;
+        const int most = 1 + static_cast<int>(rng() % 300);
+        const StagedGeometry g = staged_geometry(world, nvec, slot, most);
+        EXPECT(g.blocks <= most && g.tile_shift >= kStagedStepShift);
+        if (g.blocks == 0) {
+            EXPECT(slot < ((static_cast<size_t>(kStagedRing) * world) << kStagedStepShift) * 16);
+            continue;
+        }
+        const unsigned long long ring =
+            ((static_cast<unsigned long long>(kStagedRing) * world) << g.tile_shift) * 16;
+        EXPECT(ring * g.blocks <= slot);
+        std::vector<unsigned long long> bound(world + 1);
+        for (int s = 0; s <= world; ++s) { bound[s] = StagedWalk::shard_begin(nvec, world, s); }
+        EXPECT(bound[0] == 0 && bound[world] == nvec);
+        for (int s = 0; s < world; ++s) {
+            unsigned long long expect = bound[s];
+            for (int k = 0; k < g.rounds; ++k) {
+                for (int b = 0; b < g.blocks; ++b) {
+                    const StagedWalk w{bound.data(), world, g.blocks, b, g.tile_shift};
+                    const StagedTile t = w.tile_of(s, k);
+                    EXPECT(t.lo == expect && t.hi >= t.lo && t.hi <= bound[s + 1]);
+                    expect = t.hi;
+                    const unsigned long long piece = (1ull << g.tile_shift) * 16;
+                    EXPECT(w.piece(k, s) == ring * b + (k % kStagedRing * world + s) * piece);
+                }
+            }
+            EXPECT(expect == bound[s + 1]);
+        }
     }
     // registered groups: over all ranks and blocks, the tiles of the walk cover every whole
     // vector of every tensor exactly once, in order, never across a tensor boundary and
