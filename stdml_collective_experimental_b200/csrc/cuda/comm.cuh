@@ -130,6 +130,14 @@ static_assert(1 << kStagedStepShift == kStagedThreads, "a step is one vector per
 constexpr int kStagedStarts = 1024;  // table entries searched in shared memory
 constexpr unsigned int kStagedRoundVec = 2048;
 
+// all_gather / broadcast by pull (kernels_pull.cu)
+constexpr int kPullRing = 4;
+constexpr int kPullThreads = 256;
+constexpr int kPullPerSm = 4;
+constexpr int kPullStepShift = 8;  // smallest tile: one vector per thread
+constexpr int kPullVec = 16;            // vectors per thread and round over all sources
+static_assert(1 << kPullStepShift == kPullThreads, "a step is one vector per thread");
+
 // One tensor of a fused group: `count` elements that live at vector offset
 // `voff` (16-byte units) of the flat symmetric region.
 struct GroupEntry {
@@ -249,6 +257,17 @@ struct GatherArgs {
     int rounds;         // kBcastPipelined: pieces per block and slice
 };
 
+struct PullArgs {
+    const void *src[kMaxRanks];  // per virtual rank (broadcast: root's only)
+    void *dst[kMaxRanks];        // per virtual rank
+    unsigned long long off;      // arena offset of the staging slot
+    unsigned long long bytes;    // per rank block
+    unsigned long long stride;   // all_gather: distance between blocks in dst
+    int root;                    // < 0: all_gather; >= 0: broadcast
+    int end_barrier;             // as in GatherArgs
+    int tile_shift, rounds;      // from pull_geometry()
+};
+
 enum : int {
     kBcastPull = 0,     // root packs, everybody reads root's region (small messages);
                         // all_gather: everybody packs, then reads every peer's region
@@ -266,6 +285,8 @@ enum : int {
 void launch_barrier(const CommCtx &ctx, int vranks, void *stream);
 int launch_gather(const CommCtx &ctx, const GatherArgs &a, int blocks, int vranks,
                   void *stream);
+// kernels_pull.cu
+int launch_pull(const CommCtx &ctx, const PullArgs &a, int blocks, int vranks, void *stream);
 int launch_unpack_blocks(const void *region, void *dst, unsigned long long bytes,
                          unsigned long long sym_stride, unsigned long long stride, int blocks_n,
                          int grid, void *stream);

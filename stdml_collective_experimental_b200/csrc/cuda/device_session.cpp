@@ -1002,7 +1002,9 @@ void DeviceSession::all_gather(const void *const *in, void *const *out, size_t c
     // staged: a slot holds one block of every rank
     const bool in_capture = capturing(stream);
     const size_t slot = world_->staging_bytes();
-    const size_t chunk = std::max<size_t>(16, slot / static_cast<size_t>(world) / 16 * 16);
+    const size_t chunk = world_->pulls_staged(bytes, -1)
+                             ? bytes
+                             : std::max<size_t>(16, slot / static_cast<size_t>(world) / 16 * 16);
     std::vector<GatherCall> calls;
     std::vector<std::vector<const void *>> srcs;
     std::vector<std::vector<void *>> dsts;
@@ -1086,7 +1088,7 @@ void DeviceSession::broadcast(const void *const *in, void *const *out, size_t co
     }
 
     const bool in_capture = capturing(stream);
-    const size_t slot = world_->staging_bytes();
+    const size_t slot = world_->pulls_staged(bytes, root) ? bytes : world_->staging_bytes();
     std::vector<GatherCall> calls;
     std::vector<std::vector<const void *>> srcs;
     std::vector<std::vector<void *>> dsts;

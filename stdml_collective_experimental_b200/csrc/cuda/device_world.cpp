@@ -16,6 +16,7 @@
 #include "algo_table.hpp"
 #include "local_rendezvous.hpp"
 #include "offset_heap.hpp"
+#include "pull_walk.hpp"
 #include "staged_walk.hpp"
 
 namespace stdml::collective::cuda
@@ -182,6 +183,7 @@ class World final : public DeviceWorld
     int nvls_variant_ = kNvlsPipe4;        // STDML_COLLECTIVE_NVLS_VARIANT
     bool debug_checks_ = false;            // STDML_COLLECTIVE_DEBUG
     size_t bcast_pipelined_min_ = 8u << 20;  // STDML_COLLECTIVE_BCAST_PIPELINED_MIN_BYTES
+    size_t bcast_push_min_ = 256u << 10;     // below: pull (knob bcast_push_min_bytes)
     size_t group_bulk_min_ = 4u << 20;       // registered groups: bulk copies from here (knob group_bulk_min_bytes)
     size_t bcast_piece_vec_ = 1024;          // vectors per round, block and slice (knob bcast_piece_vec)
     size_t gather_push_min_ = 64u << 10;  // STDML_COLLECTIVE_GATHER_PUSH_MIN_BYTES
@@ -237,6 +239,13 @@ class World final : public DeviceWorld
         }
         if (const char *e = std::getenv("STDML_COLLECTIVE_NVLS_VARIANT")) {
             nvls_variant_ = std::max(0, std::min(kNvlsVariants - 1, std::atoi(e)));
+        }
+        if (o.loopback) {
+            // Pushing spares the round trip of loads over links and keeps root's links from
+            // carrying world - 1 copies.  Here there are no links, and the push's
+            // staging pass is HBM traffic: all sizes are pulled (8 ranks, 2.5 MB blocks:
+            // 518 us pushed and unpacked; 94 MB broadcast among 4: 345 us).
+            gather_push_min_ = bcast_push_min_ = bcast_pipelined_min_ = SIZE_MAX;
         }
         env_bytes("STDML_COLLECTIVE_GATHER_PUSH_MIN_BYTES", gather_push_min_);
         env_bytes("STDML_COLLECTIVE_BCAST_PIPELINED_MIN_BYTES", bcast_pipelined_min_);
@@ -407,6 +416,8 @@ class World final : public DeviceWorld
             bcast_piece_vec_ = static_cast<size_t>(std::max<long long>(32, value));
         } else if (name == "bcast_pipelined_min_bytes") {
             bcast_pipelined_min_ = value < 0 ? SIZE_MAX : static_cast<size_t>(value);
+        } else if (name == "bcast_push_min_bytes") {
+            bcast_push_min_ = value < 0 ? SIZE_MAX : static_cast<size_t>(value);
         } else if (name == "gather_push_min_bytes") {
             gather_push_min_ = value < 0 ? SIZE_MAX : static_cast<size_t>(value);
         } else if (name == "gather_mc") {
@@ -878,6 +889,59 @@ class World final : public DeviceWorld
         return rc;
     }
 
+    // How a block travels (see kGather* / kBcast*).
+    int pick_gather(size_t bytes, int root, bool mc_possible) const
+    {
+        if (root < 0) {
+            // measured: posted stores beat peer loads once the message is past the
+            // latency-bound sizes
+            return (opt_.world > 1 && bytes >= gather_push_min_) ? kGatherPush : kBcastPull;
+        }
+        if (opt_.world > 2 && bytes >= bcast_pipelined_min_) { return kBcastPipelined; }
+        if (opt_.world > 1 && bytes >= bcast_push_min_) {
+            // pulling from root costs (n-1) copies on root's links
+            return mc_possible ? kBcastNvls : (opt_.world > 2 ? kBcastScatter : kGatherPush);
+        }
+        return kBcastPull;
+    }
+
+    PullGeometry geometry_of_pull(size_t bytes, int root, int want_blocks) const
+    {
+        // all resident (the kernel's launch bounds)
+        const int most = want_blocks > 0
+                             ? want_blocks
+                             : std::min(kMaxBlocks, std::max(1, kPullPerSm * num_sms_ / vranks_));
+        return pull_geometry(root >= 0 ? 1 : opt_.world - 1, bytes, opt_.staging_bytes, most);
+    }
+
+    bool pulls_staged(size_t bytes, int root) const override
+    {
+        return opt_.world > 1 &&
+               pick_gather(bytes, root, has_nvls() && opt_.world > 2) == kBcastPull &&
+               geometry_of_pull(bytes, root, 0).blocks > 0;
+    }
+
+    int pull(const GatherArgs &g, int want_blocks, void *stream)
+    {
+        const PullGeometry geo = geometry_of_pull(g.bytes, g.root, want_blocks);
+        if (geo.blocks == 0) { return -1; }
+        if (g.off % 16 != 0 || g.off < kDataOffset || g.off + opt_.staging_bytes > arena_bytes_) {
+            throw std::invalid_argument("gather: staging slot outside the arena");
+        }
+        PullArgs a;
+        std::memset(&a, 0, sizeof(a));
+        std::memcpy(a.src, g.src, sizeof(a.src));
+        std::memcpy(a.dst, g.dst, sizeof(a.dst));
+        a.off = g.off;
+        a.bytes = g.bytes;
+        a.stride = g.stride;
+        a.root = g.root;
+        a.end_barrier = g.end_barrier;
+        a.tile_shift = geo.tile_shift;
+        a.rounds = geo.rounds;
+        return launch_pull(make_ctx(), a, geo.blocks, vranks_, stream);
+    }
+
     int gather(const GatherCall &c, void *stream) override
     {
         if (c.bytes == 0) { return 0; }
@@ -890,10 +954,6 @@ class World final : public DeviceWorld
         const size_t span = all_gather
                                 ? static_cast<size_t>(opt_.world - 1) * c.sym_stride + nvec * 16
                                 : nvec * 16;
-        if (!registered &&
-            (c.off % 16 != 0 || c.off < kDataOffset || c.off + span > arena_bytes_)) {
-            throw std::invalid_argument("gather: symmetric region outside the arena");
-        }
         GatherArgs a;
         std::memset(&a, 0, sizeof(a));
         for (int v = 0; v < vranks_; ++v) {
@@ -916,19 +976,19 @@ class World final : public DeviceWorld
         // with two GPUs the switch has nothing to add (measured: multimem.st 340 GB/s
         // against 640 GB/s for plain stores at 256 MB)
         const bool mc_possible = has_nvls() && !registered && opt_.world > 2;
-        if (c.algo >= 0) {
-            a.algo = c.algo;
-        } else if (all_gather) {
-            // measured: posted stores beat peer loads once the message is past the
-            // latency-bound sizes
-            a.algo = (opt_.world > 1 && c.bytes >= gather_push_min_) ? kGatherPush : kBcastPull;
-        } else if (opt_.world > 2 && c.bytes >= bcast_pipelined_min_) {
-            a.algo = kBcastPipelined;
-        } else if (opt_.world > 1 && c.bytes >= (256u << 10)) {
-            // pulling from root costs (n-1) copies on root's links
-            a.algo = mc_possible ? kBcastNvls : (opt_.world > 2 ? kBcastScatter : kGatherPush);
-        } else {
-            a.algo = kBcastPull;
+        a.algo = c.algo >= 0 ? c.algo : pick_gather(c.bytes, c.root, mc_possible);
+        bool staged = !registered && !c.start_barrier;  // and every destination is a tensor
+        for (int v = 0; v < vranks_; ++v) {
+            staged = staged && a.dst[v] != nullptr &&
+                     (a.src[v] != nullptr || (!all_gather && a.root != rank() + v));
+        }
+        if (a.algo == kBcastPull && staged && opt_.world > 1) {
+            const int rc = pull(a, c.blocks, stream);
+            if (rc >= 0) { return rc; }  // else: the slot is too small for a ring
+        }
+        if (!registered &&
+            (c.off % 16 != 0 || c.off < kDataOffset || c.off + span > arena_bytes_)) {
+            throw std::invalid_argument("gather: symmetric region outside the arena");
         }
         if (a.algo == kBcastNvls && !mc_possible) {
             throw std::invalid_argument("broadcast: NVLS needs the multicast mapping of the arena");
@@ -939,9 +999,6 @@ class World final : public DeviceWorld
             a.end_barrier = 1;
         }
         a.use_mc = c.use_mc >= 0 ? (c.use_mc != 0 && mc_possible) : (mc_possible && gather_mc_);
-        if (all_gather && a.algo == kBcastPull && c.src != nullptr && c.sym_stride == 0) {
-            // one block per region: block p is read at p * 0
-        }
         int blocks = c.blocks > 0 ? c.blocks : pick_blocks(nvec, kAlgoOneShot);
         if (vranks_ > 1) { blocks = std::min(blocks, std::max(1, num_sms_ / vranks_)); }
         if (a.algo == kBcastPipelined) {

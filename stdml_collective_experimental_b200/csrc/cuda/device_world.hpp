@@ -169,6 +169,9 @@ class DeviceWorld
     // arguments that the kernels could not run.
     virtual int all_reduce(const AllReduceCall &c, void *stream) = 0;
     virtual int gather(const GatherCall &c, void *stream) = 0;
+    // Whether a staged all_gather (root < 0) or broadcast of `bytes` per block goes by
+    // pull through a ring in the slot: then one call of any length will do.
+    virtual bool pulls_staged(size_t bytes, int root) const = 0;
     // Two-shot all-reduce over a table of registered tensors (see PeerEntry).
     virtual int group_peer(const PeerEntry *table, int ntable, size_t nvec, int dt, int op,
                            double scale, void *stream) = 0;

@@ -27,6 +27,7 @@
 // (src/stdml/collective/run_graph_pair_list_multi_thread.cpp:58-97 there).
 #pragma once
 #include "ar_kernel.cuh"
+#include "copy.cuh"
 #include "staged_walk.hpp"
 
 namespace stdml::collective::cuda
@@ -67,31 +68,6 @@ struct TileDesc {
     unsigned int n, fast;
     int first, last;
 };
-
-// Tensor memory goes past the L2 as far as it can (evict first): the L2 is for the rings.
-__device__ __forceinline__ unsigned long long evict_first_policy()
-{
-    unsigned long long p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-
-__device__ __forceinline__ uint4 ld_stream_v4(const void *p, unsigned long long policy)
-{
-    uint4 v;
-    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.v4.u32 {%0,%1,%2,%3}, [%4], %5;"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p), "l"(policy)
-                 : "memory");
-    return v;
-}
-
-__device__ __forceinline__ void st_stream_v4(void *p, const uint4 &v, unsigned long long policy)
-{
-    asm volatile("st.global.L2::cache_hint.v4.u32 [%0], {%1,%2,%3,%4}, %5;" ::"l"(p), "r"(v.x),
-                 "r"(v.y), "r"(v.z), "r"(v.w), "l"(policy)
-                 : "memory");
-}
 
 // Vector i of a fast tile.
 template <int DT>

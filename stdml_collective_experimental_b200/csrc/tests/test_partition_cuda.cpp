@@ -13,6 +13,7 @@
 #include "../cuda/device_session.hpp"
 #include "../cuda/algo_table.hpp"
 #include "../cuda/offset_heap.hpp"
+#include "../cuda/pull_walk.hpp"
 #include "../cuda/staged_walk.hpp"
 
 using namespace stdml::collective::cuda;
@@ -85,6 +86,38 @@ int main()
                 }
             }
             EXPECT(expect == bound[s + 1]);
+        }
+    }
+    // pull: over blocks and rounds the tiles cover the vectors of every rank's block exactly
+    // once, whatever its shift; ring pieces are disjoint and stay inside the slot
+    for (int trial = 0; trial < 2000; ++trial) {
+        const size_t bytes = 1 + rng() % (trial % 3 == 0 ? 100 : 40000000);
+        const size_t stride = bytes + rng() % 40;
+        const int world = 2 + static_cast<int>(rng() % 15);
+        const size_t slot = (size_t{4096} << (rng() % 15)) + 4096;
+        const int most = 1 + static_cast<int>(rng() % 300);
+        const PullGeometry g = pull_geometry(trial % 2 == 0 ? 1 : world - 1, bytes, slot, most);
+        EXPECT(g.blocks <= most && g.tile_shift >= kPullStepShift);
+        if (g.blocks == 0) {
+            EXPECT(slot < (static_cast<size_t>(kPullRing) << kPullStepShift) * 16);
+            continue;
+        }
+        const unsigned long long ring = (static_cast<unsigned long long>(kPullRing) << g.tile_shift) * 16;
+        EXPECT(ring * g.blocks <= slot);
+        unsigned long long expect = 0;
+        for (int k = 0; k < g.rounds; ++k) {
+            for (int b = 0; b < g.blocks; ++b) {
+                const PullWalk w{bytes, stride, g.blocks, b, g.tile_shift};
+                EXPECT(w.first_vector(k) == expect);
+                expect += 1ull << g.tile_shift;
+                EXPECT(w.piece(k) == ring * b + (k % kPullRing) * (ring / kPullRing));
+            }
+        }
+        for (int p = 0; p < world; ++p) {
+            const PullWalk w{bytes, stride, g.blocks, 0, g.tile_shift};
+            EXPECT(w.phase(p) == p * stride % 16);
+            EXPECT(expect >= w.vectors(w.phase(p)));
+            EXPECT((w.vectors(w.phase(p)) - 1) * 16 < bytes + w.phase(p));
         }
     }
     // registered groups: over all ranks and blocks, the tiles of the walk cover every whole

@@ -521,6 +521,44 @@ def test_all_gather_push_and_pull_agree(sess, algo_knob):
         sess.set_knob("gather_push_min_bytes", 64 << 10)
 
 
+@pytest.mark.parametrize("shift", [0, 4, 5])
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4097, 70_001, 3_000_001])
+def test_pull_ring_at_every_alignment(sess, n, shift):
+    """Staged all_gather and broadcast by pull: sizes around a vector, a tile and many
+    rounds, sources and destinations that start `shift` bytes off a vector boundary;
+    nothing beyond a destination's own bytes may change."""
+    if sess.world == 1:
+        pytest.skip("needs peers")
+    w = sess.world
+    sess.set_knob("gather_push_min_bytes", -1)
+    sess.set_knob("bcast_pipelined_min_bytes", -1)
+    sess.set_knob("bcast_push_min_bytes", -1)
+    try:
+        host = make_inputs(w, n, torch.uint8, seed=n)
+        ins = [torch.zeros(n + 16, dtype=torch.uint8, device="cuda")[shift:shift + n] for _ in range(w)]
+        for t, h in zip(ins, host):
+            t.copy_(h)
+        pads = [torch.full((n * w + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
+        outs = [p[16 + shift:16 + shift + n * w] for p in pads]
+        sess.all_gather(ins, outs)
+        bpads = [torch.full((n + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
+        bouts = [p[16 + shift:16 + shift + n] for p in bpads]
+        sess.broadcast(ins, out=bouts, root=w - 1)
+        sess.broadcast(ins, root=0)  # in place
+        torch.cuda.synchronize()
+        sess.check()
+        for r in range(w):
+            assert torch.equal(outs[r].cpu(), torch.cat(host)), r
+            assert bool((pads[r][:16 + shift] == 7).all() and (pads[r][16 + shift + n * w:] == 7).all())
+            assert torch.equal(bouts[r].cpu(), host[w - 1]), r
+            assert bool((bpads[r][:16 + shift] == 7).all() and (bpads[r][16 + shift + n:] == 7).all())
+            assert torch.equal(ins[r].cpu(), host[0]), r
+    finally:
+        sess.set_knob("gather_push_min_bytes", 64 << 10)
+        sess.set_knob("bcast_pipelined_min_bytes", 8 << 20)
+        sess.set_knob("bcast_push_min_bytes", 256 << 10)
+
+
 def test_kernels_against_plain_pytorch_arithmetic(sess):
     """An oracle that shares nothing with the library: the same reductions done by
     PyTorch in float32 / float64 on the host.  all_reduce (every algorithm), the
