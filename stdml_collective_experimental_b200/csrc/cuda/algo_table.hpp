@@ -59,6 +59,9 @@ inline int select_algo(const AlgoTuning &t, size_t bytes, bool nvls_defined_for_
         return kAlgoNvls;
     }
     if (!need_owner && bytes <= oneshot_limit(t)) { return kAlgoOneShot; }
+    // Two ranks on one GPU: the register path has enough loads in flight for local
+    // memory and no block sync per tile (256 MB in place: 191 us against 220-246).
+    if (t.vranks == 2) { return kAlgoTwoShot; }
     return bytes >= t.tma_min ? kAlgoTwoShotTma : kAlgoTwoShot;
 }
 

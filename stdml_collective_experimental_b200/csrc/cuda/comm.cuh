@@ -40,6 +40,10 @@ constexpr int kThreads = 512;     // block size of every collective kernel
 struct SignalPad {
     uint32_t flag[kMaxBlocks][kMaxRanks];
     uint32_t epoch[kMaxBlocks];
+    // Tickets of the kernels whose blocks take tiles as they get to them (own rank's
+    // blocks only; in a loopback world all blocks use rank 0's).  The last block to leave
+    // sets both back to zero.
+    uint32_t ticket, left;
 };
 
 constexpr size_t kDataOffset = 128u << 10;
@@ -102,14 +106,15 @@ STDML_HD inline bool is_owner_algo(int algo)
 constexpr int kTmaMaxStages = 16;
 constexpr unsigned int kTmaSmemBudget = 192u << 10;  // bytes of the 227 KB an SM offers
 
-// Ring geometry for a world: the wanted tile (default: 1024 vectors, 16 KB per
-// rank and copy; measured at 2 GPUs: 1024 > 512 > 256), halved until two slots
-// fit the budget, then as many slots as fit.
+// Ring geometry for a world: the wanted tile (default: 64 KB over all ranks, so that
+// a tile's block sync is spread over as many bytes in a small world as in a large
+// one; measured at 2 GPUs: 1024 vectors > 512 > 256), halved until two slots fit
+// the budget, then as many slots as fit.
 inline void tma_geometry(int world, unsigned int want_tile_vec, int *stages,
                          unsigned int *tile_vec, unsigned int *smem_bytes)
 {
-    unsigned int tv = want_tile_vec > 0 ? want_tile_vec : 1024u;
-    tv = (tv + 31u) / 32u * 32u;
+    unsigned int tv = want_tile_vec > 0 ? (want_tile_vec + 31u) / 32u * 32u
+                                        : 4096u / static_cast<unsigned int>(world) / 32u * 32u;
     while (tv > 32u && 2ull * world * tv * 16ull > kTmaSmemBudget) { tv /= 2; }
     unsigned int st = static_cast<unsigned int>(
         kTmaSmemBudget / (static_cast<unsigned long long>(world) * tv * 16ull));
@@ -178,6 +183,7 @@ struct AllReduceArgs {
     int has_scale;
     double scale;     // applied as f64 to f64 buffers, as its f32 value otherwise
     int phases;       // bit 0 pack, bit 1 reduce (with its barriers), bit 2 unpack
+    int dynamic;      // owner algorithms without pack and unpack: blocks take tiles by ticket
     int nvls_variant; // inner loop of the NVLS reduce: see kNvls* below
     int tma_stages;   // kAlgoTwoShotTma: slots of the shared-memory ring
     unsigned int tma_tile_vec;  // kAlgoTwoShotTma: vectors per rank per tile

@@ -179,7 +179,7 @@ class World final : public DeviceWorld
     size_t tma_over_nvls_min_ = SIZE_MAX;  // STDML_COLLECTIVE_TMA_OVER_NVLS_MIN_BYTES
     int nvls_blocks_ = 0;                  // STDML_COLLECTIVE_NVLS_BLOCKS
     int tma_blocks_ = 0;                   // STDML_COLLECTIVE_TMA_BLOCKS
-    unsigned int tma_tile_vec_ = 0;        // STDML_COLLECTIVE_TMA_TILE_VEC (0: 1024, two vectors per thread)
+    unsigned int tma_tile_vec_ = 0;        // STDML_COLLECTIVE_TMA_TILE_VEC (0: 64 KB over all ranks)
     int nvls_variant_ = kNvlsPipe4;        // STDML_COLLECTIVE_NVLS_VARIANT
     bool debug_checks_ = false;            // STDML_COLLECTIVE_DEBUG
     size_t bcast_pipelined_min_ = 8u << 20;  // STDML_COLLECTIVE_BCAST_PIPELINED_MIN_BYTES
@@ -757,8 +757,9 @@ class World final : public DeviceWorld
         if (nvls && (!has_nvls() || !nvls_supported(c.dt, c.op))) {
             throw std::invalid_argument("all_reduce: NVLS not available for this dtype/op/world");
         }
-        bool staged = false;
+        bool staged = false, any_dst = false;
         for (int v = 0; v < vranks_; ++v) {
+            any_dst = any_dst || (c.dst != nullptr && c.dst[v] != nullptr);
             staged = staged || (c.table != nullptr && c.table[v] != nullptr) ||
                      (c.src != nullptr && c.src[v] != nullptr);
         }
@@ -818,6 +819,10 @@ class World final : public DeviceWorld
         a.has_scale = c.has_scale ? 1 : 0;
         a.scale = c.scale;
         a.phases = c.phases;
+        a.dynamic = !staged && !any_dst && (algo == kAlgoTwoShot || algo == kAlgoTwoShotTma) &&
+                            c.phases == kPhaseAll && nvec < (1ull << 36)
+                        ? 1
+                        : 0;
         a.nvls_variant = nvls_variant_;
         a.debug_checks = debug_checks_ ? 1 : 0;
         if (debug_inject_ != 0) {

@@ -213,6 +213,34 @@ __device__ __forceinline__ void rounds_done(BlockSync *s, int rounds)
     if (is_sync_thread()) { s->epoch += static_cast<uint32_t>(rounds); }
 }
 
+// ------------------------------------------------------------------ tickets
+// Equal shares of a memory-bound job do not finish together: SMs differ in how far
+// they are from the memory they touch, and the slowest one sets the time (a copy in
+// equal shares runs at 5.7-6.2 TB/s, the same copy taken tile by tile at 6.7).  So the
+// blocks of a job take tiles as they get to them.  Every block draws tickets until
+// one is past the end, then leaves; the last to leave resets the counters.
+__device__ __forceinline__ SignalPad *ticket_pad(const CommCtx &ctx, int rank)
+{
+    return pad_of(ctx, ctx.one_gpu ? 0 : rank);
+}
+
+__device__ __forceinline__ unsigned int draw_ticket(SignalPad *pad)
+{
+    return atomicAdd(&pad->ticket, 1u);
+}
+
+// One thread per block, after its last ticket.  `blocks`: all that draw from this pad.
+// How often each of them drew does not matter, only that none draws after leaving.
+__device__ __forceinline__ void leave_tickets(SignalPad *pad, unsigned int blocks)
+{
+    __threadfence();
+    if (atomicAdd(&pad->left, 1u) + 1u == blocks) {
+        __threadfence();
+        atomicExch(&pad->ticket, 0u);
+        atomicExch(&pad->left, 0u);
+    }
+}
+
 // ------------------------------------------------------------- dtype traits
 template <int DT>
 struct Tr;
