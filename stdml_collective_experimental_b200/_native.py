@@ -119,6 +119,8 @@ def _declare(l):
     l.stdmlc_dw_set_knob.argtypes = [vp, c.c_char_p, c.c_longlong]
     l.stdmlc_dw_drop_registrations.argtypes = [vp]
     l.stdmlc_dw_barrier.argtypes = [vp, vp]
+    l.stdmlc_dw_host_all_reduce.argtypes = [vp, vp, vp, vp, u64, c.POINTER(u64), c.c_int, c.c_int,
+                                            c.c_double, vp, vp, vp, vp]
     l.stdmlc_dw_raw_all_reduce.argtypes = [vp, u64, vpp, vpp, u64, c.c_int, c.c_int, c.c_int,
                                            c.c_int, c.c_int, c.c_int, c.c_int, c.c_double, vp]
     l.stdmlc_dw_status.argtypes = [vp, c.POINTER(c.c_int)]

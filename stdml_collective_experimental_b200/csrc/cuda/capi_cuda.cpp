@@ -202,6 +202,16 @@ int stdmlc_dw_broadcast(void *h, const void *const *in, void *const *out,
     return guarded([&] { S(h)->broadcast(in, out, count, dt, root, stream); });
 }
 
+int stdmlc_dw_host_all_reduce(void *h, const void *host_in, void *host_out, void *dev,
+                              unsigned long long n, const unsigned long long *bounds, int dt,
+                              int op, double scale, void *after, void *h2d, void *comm, void *d2h)
+{
+    return guarded([&] {
+        S(h)->host_all_reduce(host_in, host_out, dev, n, reinterpret_cast<const size_t *>(bounds),
+                              dt, op, scale, after, h2d, comm, d2h);
+    });
+}
+
 int stdmlc_dw_barrier(void *h, void *stream)
 {
     return guarded([&] { S(h)->barrier(stream); });

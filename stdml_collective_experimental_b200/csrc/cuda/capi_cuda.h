@@ -66,6 +66,12 @@ int stdmlc_dw_all_gather(void *h, const void *const *in, void *const *out,
 int stdmlc_dw_broadcast(void *h, const void *const *in, void *const *out,
                         unsigned long long count, int dt, int root, void *stream);
 int stdmlc_dw_barrier(void *h, void *stream);
+/* All-reduce of pinned host memory through `dev` (symmetric heap), pieces
+ * [bounds[i], bounds[i + 1]) pipelined over three streams; starts after what
+ * `after` holds, returns when host_out is complete. */
+int stdmlc_dw_host_all_reduce(void *h, const void *host_in, void *host_out, void *dev,
+                              unsigned long long n, const unsigned long long *bounds, int dt,
+                              int op, double scale, void *after, void *h2d, void *comm, void *d2h);
 /* Loopback worlds: barrier among the first `rows` virtual ranks only (rows <
  * world makes the bounded wait run out; see stdmlc_dw_status). */
 int stdmlc_dw_barrier_rows(void *h, int rows, void *stream);

@@ -83,6 +83,7 @@ DeviceSession::~DeviceSession()
     for (void *p : table_mem_) { (void)cudaFree(p); }
     table_mem_.clear();
     forget_peer_plans();
+    for (void *e : host_ev_) { (void)cudaEventDestroy(static_cast<cudaEvent_t>(e)); }
     if (order_ev_ != nullptr) { (void)cudaEventDestroy(static_cast<cudaEvent_t>(order_ev_)); }
     (void)cudaGetLastError();
 }
@@ -1120,6 +1121,49 @@ void DeviceSession::broadcast(const void *const *in, void *const *out, size_t co
         launch_check(world_->gather(g, stream), "broadcast");
         ++launches_;
     }
+}
+
+void DeviceSession::host_all_reduce(const void *host_in, void *host_out, void *dev, size_t n,
+                                    const size_t *bounds, int dt, int op, double scale,
+                                    void *after, void *h2d, void *comm, void *d2h)
+{
+    if (world_->vranks() != 1) {
+        throw std::invalid_argument("host_all_reduce needs a real (one GPU per process) session");
+    }
+    const size_t es = elem_size(dt);
+    cudaStream_t in_s = static_cast<cudaStream_t>(h2d), red_s = static_cast<cudaStream_t>(comm),
+                 out_s = static_cast<cudaStream_t>(d2h);
+    std::unique_lock<std::recursive_mutex> lk(mu_);
+    while (host_ev_.size() < 2 * n + 1) {
+        cudaEvent_t e;
+        rt_check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        host_ev_.push_back(e);
+    }
+    auto ev = [&](size_t i) { return static_cast<cudaEvent_t>(host_ev_[i]); };
+    rt_check(cudaEventRecord(ev(2 * n), static_cast<cudaStream_t>(after)), "cudaEventRecord");
+    for (cudaStream_t s : {in_s, red_s, out_s}) {
+        rt_check(cudaStreamWaitEvent(s, ev(2 * n), 0), "cudaStreamWaitEvent");
+    }
+    for (size_t i = 0; i < n; ++i) {
+        const size_t at = bounds[i] * es, bytes = (bounds[i + 1] - bounds[i]) * es;
+        char *d = static_cast<char *>(dev) + at;
+        rt_check(cudaMemcpyAsync(d, static_cast<const char *>(host_in) + at, bytes,
+                                 cudaMemcpyHostToDevice, in_s),
+                 "cudaMemcpyAsync(H2D)");
+        rt_check(cudaEventRecord(ev(2 * i), in_s), "cudaEventRecord");
+        rt_check(cudaStreamWaitEvent(red_s, ev(2 * i), 0), "cudaStreamWaitEvent");
+        const void *in[1] = {d};
+        void *out[1] = {d};
+        all_reduce(in, out, bounds[i + 1] - bounds[i], dt, op, scale, -1, comm);
+        rt_check(cudaEventRecord(ev(2 * i + 1), red_s), "cudaEventRecord");
+        rt_check(cudaStreamWaitEvent(out_s, ev(2 * i + 1), 0), "cudaStreamWaitEvent");
+        rt_check(cudaMemcpyAsync(static_cast<char *>(host_out) + at, d, bytes,
+                                 cudaMemcpyDeviceToHost, out_s),
+                 "cudaMemcpyAsync(D2H)");
+    }
+    // other threads need not wait for the copies
+    lk.unlock();
+    rt_check(cudaStreamSynchronize(out_s), "cudaStreamSynchronize");
 }
 
 void DeviceSession::barrier(void *stream)

@@ -75,6 +75,14 @@ class DeviceSession
     void broadcast(const void *const *in, void *const *out, size_t count, int dt, int root,
                    void *stream);
     void barrier(void *stream);
+    // All-reduce of `bounds[n]` elements of pinned host memory through `dev` (device memory of
+    // the symmetric heap): piece i is [bounds[i], bounds[i + 1]) and flows host -> device
+    // on `h2d`, is reduced in place on `comm` and flows back on `d2h`, the three stages of
+    // different pieces side by side.  Starts after what `after` holds; returns when
+    // host_out is complete.  One rank per GPU only.
+    void host_all_reduce(const void *host_in, void *host_out, void *dev, size_t n,
+                         const size_t *bounds, int dt, int op, double scale, void *after,
+                         void *h2d, void *comm, void *d2h);
 
     // Knobs of the session (register_min_bytes) and of its world (see
     // DeviceWorld::set_knob).  register_min_bytes: collectives on ordinary device
@@ -158,6 +166,7 @@ class DeviceSession
     void *last_stream_ = nullptr;
     bool have_last_stream_ = false;
     void *order_ev_ = nullptr;
+    std::vector<void *> host_ev_;  // host_all_reduce: two events per piece and one more, kept
     size_t register_min_bytes_ = SIZE_MAX;     // STDML_COLLECTIVE_REGISTER_MIN_BYTES
     int chunk_push_blocks_ = 128;   // grid of a chunk's push while the previous chunk is unpacked (knob;
                                     // 8 GPUs, 64 MB per rank: 128 / 96 gave 850 us where 64 / 0 gave 956)
