@@ -45,6 +45,29 @@ inline size_t nvls_oneshot_limit(const AlgoTuning &t)
     return 2u << 20;
 }
 
+// Vectors of the largest message that goes through the mailboxes (kernels_ll.cu).  They
+// carry twice the bytes, so over links the exchange pays only while the time is its
+// latency (64 KB, where protocols of this kind usually end).  Between ranks of one GPU
+// doubled bytes are L2 traffic; the limit is one vector per thread, two blocks of 512 per SM.
+inline size_t ll_capacity(int world, int vranks, int num_sms)
+{
+    if (world < 2) { return 0; }
+    if (vranks <= 1) { return (64u << 10) / 16; }
+    return std::min<size_t>((512u << 10) / 16,
+                            static_cast<size_t>(std::max(1, 2 * num_sms / vranks)) * kThreads);
+}
+
+// The same for one call.  Against the two barriers of an in-place two-shot the exchange
+// wins at every size that fits (8 ranks, 160 KB: 14.4 us both, below that up to half).
+// Against the one barrier of a one-shot, on one GPU, by ranks (us, barrier / mailboxes):
+// 2: 512 KB 8.3 / 6.2; 4: 160 KB 8.3 / 6.2, 300 KB 8.3 / 8.2, 400 KB 8.3 / 10.0;
+// 8: 12 B 7.5 / 5.0, 16 KB 8.3 / 9.1, 160 KB 10.3 / 14.4.
+inline size_t ll_limit(int world, int vranks, size_t capacity, bool in_place_symmetric)
+{
+    if (vranks <= 1 || in_place_symmetric || world <= 2) { return capacity; }
+    return std::min(capacity, world <= 4 ? (256u << 10) / 16 : size_t{kThreads});
+}
+
 // need_owner: the result must stay in the symmetric buffer (in place), which
 // only the owner algorithms (two-shot, NVLS) can do.
 inline int select_algo(const AlgoTuning &t, size_t bytes, bool nvls_defined_for_op,

@@ -241,6 +241,18 @@ struct StagedArgs {
     int debug_checks;               // as in AllReduceArgs
 };
 
+// All-reduce in one exchange through the mailboxes of the arena (kernels_ll.cu).
+struct LlArgs {
+    const void *src[kMaxRanks];  // per virtual rank
+    void *dst[kMaxRanks];
+    unsigned long long off;    // arena offset of the mailboxes
+    unsigned int capacity;     // vectors of one mailbox
+    unsigned int nvec;
+    unsigned long long count;  // elements
+    int has_scale;
+    double scale;
+};
+
 enum : int { kPhasePack = 1, kPhaseReduce = 2, kPhaseUnpack = 4, kPhaseAll = 7 };
 
 struct GatherArgs {
@@ -300,6 +312,8 @@ int launch_unpack_blocks(const void *region, void *dst, unsigned long long bytes
 int launch_all_reduce(const CommCtx &ctx, const AllReduceArgs &a, int dt, int op,
                       int blocks, int vranks, void *stream);
 bool nvls_supported(int dt, int op);
+// kernels_ll.cu: the same contract; one vector per thread
+int launch_ll(const CommCtx &ctx, const LlArgs &a, int dt, int op, int vranks, void *stream);
 // kernels_st_*.cu: the same contract; blocks and rounds from staged_geometry()
 int launch_staged(const CommCtx &ctx, const StagedArgs &a, int dt, int op, int blocks, int vranks,
                   void *stream);

@@ -296,6 +296,11 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
         symmetric = world_->offset_of(in[v], v) == off;
         in_place = in_place && (in[v] == out[v]);
     }
+    if (algo < 0 && world_->small_all_reduce(in, out, count, dt, op, c.has_scale, scale,
+                                             symmetric && in_place, stream)) {
+        ++launches_;
+        return;
+    }
     if (symmetric && in_place) {
         c.off = off;
         c.count = count;
@@ -811,6 +816,13 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         if (flat) { total = expect - first; }
     }
     if (flat && total > 0) {
+        void *at[kMaxRanks];
+        for (int v = 0; v < vr; ++v) { at[v] = world_->ptr(world_->rank() + v, first); }
+        if (algo < 0 && world_->small_all_reduce(at, at, total / es, dt, op, scale != 1.0, scale, true,
+                                                 stream)) {
+            ++launches_;
+            return;
+        }
         AllReduceCall c;
         c.dt = dt;
         c.op = op;

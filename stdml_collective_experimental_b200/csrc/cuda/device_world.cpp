@@ -134,6 +134,9 @@ class World final : public DeviceWorld
     int vranks_;
     size_t arena_bytes_ = 0;
     size_t staging_off_[2] = {0, 0};
+    // mailboxes of the small all-reduce: offset, vectors of one, bytes of all
+    size_t ll_off_ = 0, ll_capacity_ = 0, ll_bytes_ = 0;
+    size_t ll_max_ = SIZE_MAX;  // knob ll_max_bytes: largest message that may use them
     unsigned long long staged_ops_ = 0;
     OffsetHeap heap_;
     double setup_ms_[4] = {0, 0, 0, 0};
@@ -257,7 +260,10 @@ class World final : public DeviceWorld
         const size_t staging = round_up(std::max<size_t>(o.staging_bytes, 4096), 4096);
         staging_off_[0] = kDataOffset;
         staging_off_[1] = kDataOffset + staging;
-        const size_t heap_off = kDataOffset + 2 * staging;
+        ll_off_ = kDataOffset + 2 * staging;
+        ll_capacity_ = ll_capacity(o.world, vranks_, num_sms_);
+        ll_bytes_ = 2 * static_cast<size_t>(o.world) * ll_capacity_ * 32;  // two per source
+        const size_t heap_off = ll_off_ + ll_bytes_;
         arena_bytes_ = heap_off + round_up(o.heap_bytes, 4096);
         opt_.staging_bytes = staging;
 
@@ -416,6 +422,8 @@ class World final : public DeviceWorld
             bcast_piece_vec_ = static_cast<size_t>(std::max<long long>(32, value));
         } else if (name == "bcast_pipelined_min_bytes") {
             bcast_pipelined_min_ = value < 0 ? SIZE_MAX : static_cast<size_t>(value);
+        } else if (name == "ll_max_bytes") {
+            ll_max_ = value < 0 ? SIZE_MAX : static_cast<size_t>(value);
         } else if (name == "bcast_push_min_bytes") {
             bcast_push_min_ = value < 0 ? SIZE_MAX : static_cast<size_t>(value);
         } else if (name == "gather_push_min_bytes") {
@@ -741,6 +749,13 @@ class World final : public DeviceWorld
         }
         int algo = c.algo;
         if (algo < 0) { algo = pick_algo(bytes, c.dt, c.op, any_dst_null); }
+        if (c.algo < 0 && c.staged && c.table != nullptr && algo == kAlgoOneShot &&
+            c.ntable > 4 * pick_blocks(nvec, algo)) {
+            // The one-shot walks the tensors of a block's span one after the other, about
+            // a microsecond each; the staged kernel lets every vector find its own (158
+            // tensors, 1.1 MB, 4 ranks: 57 us one-shot, 22 us so).
+            algo = kAlgoTwoShot;
+        }
         if (algo >= kAlgoCount) { throw std::invalid_argument("all_reduce: unknown algorithm"); }
         const bool owner = is_owner_algo(algo);
         const bool nvls =
@@ -892,6 +907,40 @@ class World final : public DeviceWorld
         const int rc = launch_staged(make_ctx(), a, c.dt, c.op, g.blocks, vranks_, stream);
         if (rc < 0) { throw std::invalid_argument("all_reduce: (dtype, op) not built"); }
         return rc;
+    }
+
+    bool small_all_reduce(const void *const *in, void *const *out, size_t count, int dt, int op,
+                          bool has_scale, double scale, bool symmetric, void *stream) override
+    {
+        static const size_t sizes[12] = {1, 2, 4, 8, 1, 2, 4, 8, 2, 2, 4, 8};
+        if (dt < 0 || dt > DT_F64_ || op < 0 || op > 4 || (op == 4 && dt >= 8)) { return false; }
+        const size_t bytes = count * sizes[dt];
+        const size_t nvec = (bytes + 15) / 16;
+        if (nvec == 0 || nvec > ll_limit(opt_.world, vranks_, ll_capacity_, symmetric) ||
+            bytes > ll_max_ || debug_checks_ || debug_inject_ != 0) {
+            return false;
+        }
+        // from three GPUs up the switch has small messages (measured: 11-14 us up to 256 KB)
+        if (has_nvls() && nvls_supported(dt, op) && opt_.world > 2) { return false; }
+        LlArgs a;
+        std::memset(&a, 0, sizeof(a));
+        for (int v = 0; v < vranks_; ++v) {
+            if (in[v] == nullptr || out[v] == nullptr) { return false; }
+            a.src[v] = in[v];
+            a.dst[v] = out[v];
+        }
+        a.off = ll_off_;
+        a.capacity = static_cast<unsigned int>(ll_capacity_);
+        a.nvec = static_cast<unsigned int>(nvec);
+        a.count = count;
+        a.has_scale = has_scale ? 1 : 0;
+        a.scale = scale;
+        const int rc = launch_ll(make_ctx(), a, dt, op, vranks_, stream);
+        if (rc != 0) {
+            throw std::runtime_error(std::string("device world: launch of the small all_reduce failed: ") +
+                                     cudaGetErrorString(static_cast<cudaError_t>(rc)));
+        }
+        return true;
     }
 
     // How a block travels (see kGather* / kBcast*).
@@ -1093,10 +1142,10 @@ class World final : public DeviceWorld
         if (rdv_) { rdv_->barrier(); }
         if (opt_.loopback) {
             for (int r = 0; r < opt_.world; ++r) {
-                rt_check(cudaMemset(base_[r], 0, kDataOffset), "cudaMemset(pad)");
+                clear_signals(r);
             }
         } else {
-            rt_check(cudaMemset(base_[opt_.rank], 0, kDataOffset), "cudaMemset(pad)");
+            clear_signals(opt_.rank);
         }
         rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
         std::memset(status_host_, 0, sizeof(StatusBlock));
@@ -1107,6 +1156,16 @@ class World final : public DeviceWorld
   private:
     static constexpr int DT_F64_ = 11;
 
+    // Flags that no wait takes for an arrival: pad and mailboxes start from zero (epochs
+    // count from one).
+    void clear_signals(int r)
+    {
+        rt_check(cudaMemset(base_[r], 0, kDataOffset), "cudaMemset(pad)");
+        if (ll_bytes_ > 0) {
+            rt_check(cudaMemset(base_[r] + ll_off_, 0, ll_bytes_), "cudaMemset(mailboxes)");
+        }
+    }
+
     void setup_loopback()
     {
         backend_ = "loopback";
@@ -1114,8 +1173,8 @@ class World final : public DeviceWorld
             void *p = nullptr;
             rt_check(cudaMalloc(&p, arena_bytes_), "cudaMalloc(arena)");
             owned_.push_back(p);
-            rt_check(cudaMemset(p, 0, kDataOffset), "cudaMemset(pad)");
             base_[r] = static_cast<char *>(p);
+            clear_signals(r);
         }
         rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
     }
@@ -1241,7 +1300,7 @@ class World final : public DeviceWorld
         me.mapped = true;
         map_rw(me.va, size);
         base_[opt_.rank] = reinterpret_cast<char *>(me.va);
-        rt_check(cudaMemset(base_[opt_.rank], 0, kDataOffset), "cudaMemset(pad)");
+        clear_signals(opt_.rank);
         rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
         return true;
     }
@@ -1421,9 +1480,9 @@ class World final : public DeviceWorld
         void *p = nullptr;
         rt_check(cudaMalloc(&p, arena_bytes_), "cudaMalloc(arena)");
         owned_.push_back(p);
-        rt_check(cudaMemset(p, 0, kDataOffset), "cudaMemset(pad)");
-        rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
         base_[opt_.rank] = static_cast<char *>(p);
+        clear_signals(opt_.rank);
+        rt_check(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
         if (opt_.world == 1) { return; }
         cudaIpcMemHandle_t h;
         rt_check(cudaIpcGetMemHandle(&h, p), "cudaIpcGetMemHandle");

@@ -168,6 +168,12 @@ class DeviceWorld
     // Launches.  Return 0 or a cudaError_t; throw std::invalid_argument on
     // arguments that the kernels could not run.
     virtual int all_reduce(const AllReduceCall &c, void *stream) = 0;
+    // Small all-reduce in one exchange, between any tensors (in and out: vranks() entries).
+    // False, with nothing done: the message is too large for it or has a faster way.
+    // symmetric: the other way is the in-place two-shot in the arena.
+    virtual bool small_all_reduce(const void *const *in, void *const *out, size_t count, int dt,
+                                  int op, bool has_scale, double scale, bool symmetric,
+                                  void *stream) = 0;
     virtual int gather(const GatherCall &c, void *stream) = 0;
     // Whether a staged all_gather (root < 0) or broadcast of `bytes` per block goes by
     // pull through a ring in the slot: then one call of any length will do.

@@ -521,6 +521,42 @@ def test_all_gather_push_and_pull_agree(sess, algo_knob):
         sess.set_knob("gather_push_min_bytes", 64 << 10)
 
 
+@pytest.mark.parametrize("dtype,op", [(torch.float32, "sum"), (torch.bfloat16, "sum"),
+                                      (torch.int8, "bit_xor"), (torch.float64, "max")])
+def test_small_all_reduce_in_one_exchange(sess, dtype, op):
+    """Messages that go through the mailboxes: one vector, around a block of threads, the
+    largest that fits and one more; twice and more in a row (both mailboxes), between
+    other collectives, in the heap, off vector boundaries."""
+    if sess.world == 1:
+        pytest.skip("needs peers")
+    es = torch.empty((), dtype=dtype).element_size()
+    lanes = 16 // es
+    most = min(32768, 2 * 148 // sess.world * 512) * lanes
+    for n in (1, lanes - 1 or 1, 511 * lanes + 1, 512 * lanes, 513 * lanes - 1, most - 1, most, most + 1):
+        host = make_inputs(sess.world, n, dtype, seed=n)
+        want = reduce_many(host, op, 1.0)
+        dev = [h.cuda() for h in host]
+        odd = [torch.zeros(n + 1, dtype=dtype, device="cuda")[1:] for _ in host]
+        sym = sess.symm_empty(n, dtype)
+        for r, h in enumerate(host):
+            odd[r].copy_(h)
+            sym[r].copy_(h)
+        outs = [[torch.empty_like(d) for d in dev] for _ in range(3)]
+        sess.all_reduce(dev, out=outs[0], op=op)
+        sess.all_reduce(odd, out=outs[1], op=op)
+        sess.barrier()
+        sess.all_reduce(sym, op=op)
+        sess.all_reduce(dev, out=outs[2], op=op)
+        sess.all_reduce(odd, op=op)
+        torch.cuda.synchronize()
+        sess.check()
+        for r in range(sess.world):
+            for got in [o[r] for o in outs] + [sym[r], odd[r]]:
+                assert same(got.cpu(), want), (n, r)
+            assert same(dev[r].cpu(), host[r])
+        sess.symm_free(sym)
+
+
 @pytest.mark.parametrize("shift", [0, 4, 5])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 4097, 70_001, 3_000_001])
 def test_pull_ring_at_every_alignment(sess, n, shift):
