@@ -835,7 +835,9 @@ class World final : public DeviceWorld
         a.scale = c.scale;
         a.phases = c.phases;
         a.dynamic = !staged && !any_dst && (algo == kAlgoTwoShot || algo == kAlgoTwoShotTma) &&
-                            c.phases == kPhaseAll && nvec < (1ull << 36)
+                            c.phases == kPhaseAll && nvec < (1ull << 36) &&
+                            // (with a tile or two per block there is nothing to balance)
+                            nvec > 2ull * blocks * opt_.world * kThreads * 4
                         ? 1
                         : 0;
         a.nvls_variant = nvls_variant_;

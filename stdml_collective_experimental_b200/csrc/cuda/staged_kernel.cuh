@@ -117,6 +117,7 @@ __device__ __forceinline__ void store_fast(char *dst, unsigned int i, bool user_
 // would weigh on the loops of the many.
 struct SlowTile {
     const GroupEntry *tab;
+    const unsigned int *starts;  // first vectors of the entries, in shared memory (or null)
     const void *src;
     void *dst;
     unsigned long long count;
@@ -124,13 +125,31 @@ struct SlowTile {
     int user_f32;
 };
 
+// Entry that holds vector v, between the tile's first and last.
+__device__ __forceinline__ const GroupEntry &slow_entry(const SlowTile &t, unsigned long long v)
+{
+    if (t.starts == nullptr) {
+        return t.tab[t.first + find_entry(t.tab + t.first, t.last - t.first + 1, v)];
+    }
+    int lo = t.first, hi = t.last;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (t.starts[mid] <= static_cast<unsigned int>(v)) {
+            lo = mid;
+        } else {
+            hi = mid - 1;
+        }
+    }
+    return t.tab[lo];
+}
+
 template <int DT>
 static __device__ __noinline__ uint4 load_slow(const SlowTile &t, unsigned long long v)
 {
     if (t.tab == nullptr) {
         return load_user_vec<DT>(t.src, t.user_f32 != 0, v, t.count, ptr_aligned16(t.src));
     }
-    const GroupEntry &e = t.tab[t.first + find_entry(t.tab + t.first, t.last - t.first + 1, v)];
+    const GroupEntry &e = slow_entry(t, v);
     return load_user_vec<DT>(e.src, t.user_f32 != 0, v - e.voff, e.count, ptr_aligned16(e.src));
 }
 
@@ -141,7 +160,7 @@ static __device__ __noinline__ void store_slow(const SlowTile &t, unsigned long 
         store_user_vec<DT>(t.dst, t.user_f32 != 0, v, t.count, ptr_aligned16(t.dst), x);
         return;
     }
-    const GroupEntry &e = t.tab[t.first + find_entry(t.tab + t.first, t.last - t.first + 1, v)];
+    const GroupEntry &e = slow_entry(t, v);
     store_user_vec<DT>(e.dst, t.user_f32 != 0, v - e.voff, e.count, ptr_aligned16(e.dst), x);
 }
 
@@ -149,8 +168,11 @@ static __device__ __noinline__ void store_slow(const SlowTile &t, unsigned long 
 // others move bytes.  Measured, 102 MB of f32 in 161 tensors, 4 ranks, us per call
 // (vectors per block and round over all shards): 256 threads 403 (1024), 354 (2048),
 // 388 (4096: the rings, 117 MB, no longer fit the L2); 512 threads, two blocks: 368 (4096).
-// The three-phase kernel took 457; with every vector looking for its own tensor (no tile
-// descriptors) this one took 432.
+// Those with four vectors of a thread in flight in pack and unpack, whose registers spill
+// around the out-of-line calls; two in flight 310, one (no spills) 300: the other 31 warps
+// of the SM's share hide a load better than spilled registers do.  Three, five and six blocks
+// per SM: 333, 367, 445.  The three-phase kernel took 457; with every vector looking for
+// its own tensor (no tile descriptors) this one took 432.
 template <int DT, int OP>
 __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
     staged_kernel(const __grid_constant__ CommCtx ctx, const __grid_constant__ StagedArgs a)
@@ -185,6 +207,7 @@ __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
     slow.user_f32 = user_f32 ? 1 : 0;
 
     const bool searchable = tab != nullptr && a.ntable <= kStagedStarts && a.nvec >> 32 == 0;
+    slow.starts = searchable ? starts : nullptr;
     auto entry_at = [&](unsigned long long v) {
         if (!searchable) { return find_entry(tab, a.ntable, v); }
         int lo = 0, hi = a.ntable - 1;
@@ -275,23 +298,12 @@ __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
             // ---- pack tile k of every shard but the own one
             char *to = mine + walk.piece(k, 0);
             const TileDesc *ds = descs[k & 3];
-            for (int q0 = 0; q0 < steps; q0 += 4) {
-                uint4 x[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (q0 + u < steps) {
-                        const TileDesc &d = ds[shard_at(q0 + u)];
-                        const unsigned int i = vector_at(q0 + u);
-                        if (i < d.fast) { x[u] = load_fast<DT>(d.src, i, user_f32, policy); }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (q0 + u < steps) {
-                        const int s = shard_at(q0 + u);
-                        const unsigned int i = vector_at(q0 + u);
-                        if (i < ds[s].fast) { st_arena_v4(to + piece_byte(s, i), x[u]); }
-                    }
+            for (int q = 0; q < steps; ++q) {
+                const int s = shard_at(q);
+                const TileDesc &d = ds[s];
+                const unsigned int i = vector_at(q);
+                if (i < d.fast) {
+                    st_arena_v4(to + piece_byte(s, i), load_fast<DT>(d.src, i, user_f32, policy));
                 }
             }
             for (int q = 0; slow_shards[k & 3] != 0u && q < steps; ++q) {
@@ -357,23 +369,12 @@ __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
             // ---- unpack tile k-2 of every shard but the own one
             const char *from = mine + walk.piece(k - 2, 0);
             const TileDesc *ds = descs[(k - 2) & 3];
-            for (int q0 = 0; q0 < steps; q0 += 4) {
-                uint4 x[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (q0 + u < steps) {
-                        const int s = shard_at(q0 + u);
-                        const unsigned int i = vector_at(q0 + u);
-                        if (i < ds[s].fast) { x[u] = ld_arena_v4(from + piece_byte(s, i)); }
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    if (q0 + u < steps) {
-                        const TileDesc &d = ds[shard_at(q0 + u)];
-                        const unsigned int i = vector_at(q0 + u);
-                        if (i < d.fast) { store_fast<DT>(d.dst, i, user_f32, x[u], policy); }
-                    }
+            for (int q = 0; q < steps; ++q) {
+                const int s = shard_at(q);
+                const TileDesc &d = ds[s];
+                const unsigned int i = vector_at(q);
+                if (i < d.fast) {
+                    store_fast<DT>(d.dst, i, user_f32, ld_arena_v4(from + piece_byte(s, i)), policy);
                 }
             }
             for (int q = 0; slow_shards[(k - 2) & 3] != 0u && q < steps; ++q) {
