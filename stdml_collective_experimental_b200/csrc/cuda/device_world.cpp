@@ -249,6 +249,9 @@ class World final : public DeviceWorld
             // staging pass is HBM traffic: all sizes are pulled (8 ranks, 2.5 MB blocks:
             // 518 us pushed and unpacked; 94 MB broadcast among 4: 345 us).
             gather_push_min_ = bcast_push_min_ = bcast_pipelined_min_ = SIZE_MAX;
+            // Registered groups, plain loads against bulk copies, 8 ranks, us: 6.5 MB 22 / 33,
+            // 11 MB 44 / 63, 20 MB 77 / 82, 51 MB 199 / 155; the same order with 2 and 4.
+            group_bulk_min_ = 24u << 20;
         }
         env_bytes("STDML_COLLECTIVE_GATHER_PUSH_MIN_BYTES", gather_push_min_);
         env_bytes("STDML_COLLECTIVE_BCAST_PIPELINED_MIN_BYTES", bcast_pipelined_min_);
@@ -1089,6 +1092,11 @@ class World final : public DeviceWorld
             unsigned int smem = 0;
             tma_geometry(opt_.world, tma_tile_vec_, &a.tma_stages, &a.tma_tile_vec, &smem);
             blocks = std::min(blocks, num_sms_);
+        } else {
+            // one vector per thread as far as the grid goes: its time is a chain of loads
+            const size_t work = (nvec + opt_.world - 1) / static_cast<size_t>(opt_.world);
+            blocks = static_cast<int>(std::min<size_t>((work + kThreads - 1) / kThreads,
+                                                       static_cast<size_t>(max_blocks_)));
         }
         if (vranks_ > 1) { blocks = std::min(blocks, std::max(1, num_sms_ / vranks_)); }
         blocks = std::min(blocks, kMaxBlocks);

@@ -4,7 +4,7 @@
 // (rank-ascending reduce in registers, scale fused) and stores the result into
 // every rank's output tensor.  Nothing is packed or unpacked, so loose gradient
 // tensors cost one launch and no extra HBM pass.  Two ways of loading: 16-byte
-// peer loads (small sets), or bulk asynchronous copies into a shared-memory
+// peer loads, each vector finding its own tensor (small sets), or bulk asynchronous copies into a shared-memory
 // ring whose tiles run on across tensor boundaries, so that the copy pipeline
 // never drains between tensors (BULK).
 //
@@ -44,7 +44,8 @@ constexpr int kWalkThreads = kThreads + 32;
 template <int DT, int OP>
 __device__ __forceinline__ bool bulk_walk(const CommCtx &ctx, const GroupPeerArgs &a, int rank,
                                           unsigned char *ring, unsigned long long *full,
-                                          unsigned long long *empty, SlotTile *slots, unsigned int *starts, BlockSync *sync)
+                                          unsigned long long *empty, SlotTile *slots, const unsigned int *starts,
+                                          bool searchable, BlockSync *sync)
 {
     constexpr unsigned long long N = lanes_of<DT>();
     const int world = ctx.world;
@@ -53,12 +54,6 @@ __device__ __forceinline__ bool bulk_walk(const CommCtx &ctx, const GroupPeerArg
     const unsigned int tile_bytes = tile_vec * 16u;
     const uint32_t ring_s = smem_addr(ring);
     const uint32_t full_s = smem_addr(full), empty_s = smem_addr(empty);
-    const bool searchable = a.ntable <= kPeerStarts && a.nvec >> 32 == 0;
-    if (searchable) {
-        for (int i = static_cast<int>(threadIdx.x); i < a.ntable; i += kWalkThreads) {
-            starts[i] = static_cast<unsigned int>(a.table[i].voff);
-        }
-    }
     if (threadIdx.x == 0) {
         for (int s = 0; s < stages; ++s) {
             mbar_init(full_s + 8u * s, 1u);
@@ -200,70 +195,121 @@ __device__ __forceinline__ bool bulk_walk(const CommCtx &ctx, const GroupPeerArg
     return true;
 }
 
+// Elements [e0, count) of an entry, one by one: the ragged last vector of a tensor.
+template <int DT, int OP>
+static __device__ __noinline__ void reduce_tail(const PeerEntry *e, unsigned long long e0, int world,
+                                                double scale, bool has_scale)
+{
+    using S = typename Tr<DT>::storage;
+    for (unsigned long long j = e0; j < e->count; ++j) {
+        typename Tr<DT>::acc acc =
+            Tr<DT>::widen(*reinterpret_cast<const volatile S *>(e->in[0] + j * sizeof(S)));
+        for (int r = 1; r < world; ++r) {
+            acc = combine<OP>(acc, Tr<DT>::widen(*reinterpret_cast<const volatile S *>(
+                                       e->in[r] + j * sizeof(S))));
+        }
+        if constexpr (Tr<DT>::is_float) {
+            if (has_scale) { acc = acc * static_cast<typename Tr<DT>::acc>(scale); }
+        }
+        const S res = Tr<DT>::narrow(acc);
+        for (int r = 0; r < world; ++r) {
+            *reinterpret_cast<volatile S *>(e->out[r] + j * sizeof(S)) = res;
+        }
+    }
+}
+
 template <int DT, int OP, bool BULK>
 __global__ void __launch_bounds__(BULK ? kWalkThreads : kThreads)
     group_peer_kernel(const __grid_constant__ CommCtx ctx, const __grid_constant__ GroupPeerArgs a)
 {
-    using S = typename Tr<DT>::storage;
     constexpr unsigned long long N = lanes_of<DT>();
     extern __shared__ __align__(128) unsigned char ring[];
     __shared__ BlockSync sync;
     __shared__ __align__(8) unsigned long long full[BULK ? kTmaMaxStages : 1];
     __shared__ __align__(8) unsigned long long empty[BULK ? kTmaMaxStages : 1];
     __shared__ SlotTile slots[BULK ? kTmaMaxStages : 1];
-    __shared__ unsigned int starts[BULK ? kPeerStarts : 1];
+    __shared__ unsigned int starts[kPeerStarts];
     const int rank = ctx.rank + static_cast<int>(blockIdx.y);
     const int world = ctx.world;
     const int nb = static_cast<int>(gridDim.x);
     const int b = static_cast<int>(blockIdx.x);
     sync_begin(ctx, rank, &sync);
+    const bool searchable = a.ntable <= kPeerStarts && a.nvec >> 32 == 0;
+    if (searchable) {
+        for (int i = static_cast<int>(threadIdx.x); i < a.ntable; i += static_cast<int>(blockDim.x)) {
+            starts[i] = static_cast<unsigned int>(a.table[i].voff);
+        }
+    }
     // every rank is here: its inputs are final, its outputs may be written
     if (!peer_barrier(ctx, rank, &sync)) { return; }
 
     const Span sp = span_of(a.nvec, world, rank, nb, b);
     if constexpr (BULK) {
-        if (!bulk_walk<DT, OP>(ctx, a, rank, ring, full, empty, slots, starts, &sync)) { return; }
-    }
-    if (sp.lo < sp.hi) {
-        for (int i = find_peer_entry(a.table, a.ntable, sp.lo); i < a.ntable; ++i) {
-            const PeerEntry *e = &a.table[i];
-            const unsigned long long voff = e->voff;
-            if (voff >= sp.hi) { break; }
-            const unsigned long long count = e->count;
-            const unsigned long long full = count / N;            // whole vectors
-            const unsigned long long nv = (count + N - 1) / N;    // with the ragged one
-            const unsigned long long lo = (sp.lo > voff ? sp.lo : voff) - voff;
-            unsigned long long hi = (sp.hi < voff + nv ? sp.hi : voff + nv);
-            if (hi <= voff + lo) { continue; }
-            hi -= voff;
-            const unsigned long long hi_full = hi < full ? hi : full;
-            if (!BULK && lo < hi_full) {
-                reduce_span<DT, OP>(ctx, e->in, lo, hi_full, a.scale, a.has_scale != 0,
-                                    [&](unsigned long long v, const uint4 &x) {
-                                        for (int k = 0; k < world; ++k) {
-                                            const int r = (rank + k) % world;
-                                            st_arena_v4(e->out[r] + v * 16ull, x);
-                                        }
-                                    });
+        if (!bulk_walk<DT, OP>(ctx, a, rank, ring, full, empty, slots, starts, searchable, &sync)) {
+            return;
+        }
+        // the ragged last vectors in this block's span, a tensor per thread
+        if (sp.lo < sp.hi) {
+            for (int i = find_peer_entry(a.table, a.ntable, sp.lo) + static_cast<int>(threadIdx.x);
+                 i < a.ntable; i += kWalkThreads) {
+                const PeerEntry *e = &a.table[i];
+                const unsigned long long voff = e->voff;
+                if (voff >= sp.hi) { break; }
+                const unsigned long long whole = e->count / N;
+                const unsigned long long tail = voff + whole;
+                if (whole * N < e->count && tail >= sp.lo && tail < sp.hi) {
+                    reduce_tail<DT, OP>(e, whole * N, world, a.scale, a.has_scale != 0);
+                }
             }
-            // the ragged last vector of a tensor: element by element, one thread
-            if (full < nv && lo <= full && full < hi && threadIdx.x == 0) {
-                const unsigned long long e0 = full * N;
-                for (unsigned long long j = e0; j < count; ++j) {
-                    typename Tr<DT>::acc acc = Tr<DT>::widen(
-                        *reinterpret_cast<const volatile S *>(e->in[0] + j * sizeof(S)));
-                    for (int r = 1; r < world; ++r) {
-                        acc = combine<OP>(acc, Tr<DT>::widen(*reinterpret_cast<const volatile S *>(
-                                                   e->in[r] + j * sizeof(S))));
-                    }
-                    if constexpr (Tr<DT>::is_float) {
-                        if (a.has_scale != 0) { acc = acc * static_cast<typename Tr<DT>::acc>(a.scale); }
-                    }
-                    const S res = Tr<DT>::narrow(acc);
-                    for (int r = 0; r < world; ++r) {
-                        *reinterpret_cast<volatile S *>(e->out[r] + j * sizeof(S)) = res;
+        }
+    } else {
+        // Small sets: a vector per thread, which looks for its own tensor.  (Walking the
+        // tensors of the span one after the other costs their latency each: 158 tensors,
+        // 0.55 MB, 8 ranks on one GPU: 103 us, so 17 us.)
+        for (unsigned long long v = sp.lo + threadIdx.x; v < sp.hi; v += kThreads) {
+            int i;
+            if (searchable) {
+                int lo = 0, hi = a.ntable - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (starts[mid] <= static_cast<unsigned int>(v)) {
+                        lo = mid;
+                    } else {
+                        hi = mid - 1;
                     }
                 }
+                i = lo;
+            } else {
+                i = find_peer_entry(a.table, a.ntable, v);
+            }
+            const PeerEntry *e = &a.table[i];
+            const unsigned long long lv = v - e->voff;
+            if ((lv + 1) * N > e->count) {
+                reduce_tail<DT, OP>(e, lv * N, world, a.scale, a.has_scale != 0);
+                continue;
+            }
+            Accum<DT> acc;
+            for (int r0 = 0; r0 < world; r0 += 4) {
+                uint4 x[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (r0 + j < world) { x[j] = ld_arena_v4(e->in[r0 + j] + lv * 16ull); }
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    if (r0 + j < world) {
+                        if (r0 + j == 0) {
+                            acc.init(x[j]);
+                        } else {
+                            acc.template add<OP>(x[j]);
+                        }
+                    }
+                }
+            }
+            const uint4 res = acc.finish(a.scale, a.has_scale != 0);
+            for (int k = 0; k < world; ++k) {
+                const int r = rank + k < world ? rank + k : rank + k - world;
+                st_arena_v4(e->out[r] + lv * 16ull, res);
             }
         }
     }
