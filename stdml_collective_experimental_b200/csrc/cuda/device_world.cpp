@@ -839,6 +839,8 @@ class World final : public DeviceWorld
         a.phases = c.phases;
         a.dynamic = !staged && !any_dst && (algo == kAlgoTwoShot || algo == kAlgoTwoShotTma) &&
                             c.phases == kPhaseAll && nvec < (1ull << 36) &&
+                            // (a root that unpacks on its own relies on the tiles by index)
+                            (c.root < 0 || registered) &&
                             // (with a tile or two per block there is nothing to balance)
                             nvec > 2ull * blocks * opt_.world * kThreads * 4
                         ? 1

@@ -70,6 +70,7 @@ __device__ __forceinline__ bool bulk_walk(const CommCtx &ctx, const GroupPeerArg
     bool ok = true;
     int issued = 0;  // walker only
     if (walker) {
+        fence_async_proxy();  // the barriers it has passed against the copies it issues
         // on one GPU every block may serve every shard
         const bool any = ctx.one_gpu != 0;
         const Span shard = any ? Span{0ull, a.nvec} : span_of(a.nvec, world, rank, 1, 0);

@@ -184,7 +184,9 @@ class DeviceSession:
     def set_knob(self, name, value):
         """Named tuning knob, same value on every rank: nvls_variant (0..3),
         nvls_blocks, tma_blocks, tma_tile_vec, tma_min_bytes,
-        tma_over_nvls_min_bytes (negative: never), gather_push_min_bytes, gather_mc,
+        tma_over_nvls_min_bytes (negative: never), gather_push_min_bytes,
+        bcast_push_min_bytes (below: pull through a ring), gather_mc, ll_max_bytes
+        (largest all_reduce that may go through the mailboxes; 0: never),
         pipeline_min_bytes, debug_checks, group_bulk_min_bytes (registered groups of
         at least that many bytes load their operands with bulk asynchronous copies;
         negative: never), register_verify (0: a registered group trusts its tensors'
