@@ -31,6 +31,13 @@ __device__ __forceinline__ void st_stream_v4(void *p, const uint4 &v, unsigned l
                  : "memory");
 }
 
+// Asks for [p, p + bytes) of this GPU's own memory in the L2, ahead of the loads that
+// want it: one instruction of one thread.  16-byte aligned, a multiple of 16 bytes.
+__device__ __forceinline__ void prefetch_l2(const void *p, unsigned int bytes)
+{
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
 // Bytes [a, a + 16) of the 32 bytes lo, hi (0 <= a < 16).
 __device__ __forceinline__ uint4 shift_bytes(const uint4 &lo, const uint4 &hi, unsigned int a)
 {
