@@ -78,6 +78,18 @@ struct ShiftedSource {
     {
     }
 
+    // Vectors [v, v + n) into the L2, as far as they are the tensor's (whole aligned 16 bytes).
+    __device__ __forceinline__ void prefetch(unsigned long long v, unsigned long long n) const
+    {
+        const char *lo = begin + 16ull * v - phase;
+        const char *hi = lo + 16ull * n;
+        lo = lo > begin ? lo : begin;
+        hi = hi < end ? hi : end;
+        const unsigned long long a = (reinterpret_cast<unsigned long long>(lo) + 15ull) & ~15ull;
+        const unsigned long long b = reinterpret_cast<unsigned long long>(hi) & ~15ull;
+        if (a < b) { prefetch_l2(reinterpret_cast<const void *>(a), static_cast<unsigned int>(b - a)); }
+    }
+
     // A vector all of whose bytes are the tensor's: no look at the ends.
     __device__ __forceinline__ uint4 load_inside(unsigned long long v, unsigned long long policy) const
     {

@@ -148,6 +148,17 @@ __device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src,
     }
 }
 
+// arrive_all (below) behind a block sync that the caller has made.
+__device__ __forceinline__ void tell_all(const CommCtx &ctx, int rank, BlockSync *s, int nth)
+{
+    const int p = static_cast<int>(threadIdx.x);
+    if (p < ctx.world) {
+        fence_ranks(ctx);
+        st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank],
+                           s->epoch + static_cast<uint32_t>(nth));
+    }
+}
+
 // The two halves of a barrier between the blocks with the same blockIdx.x on every
 // rank; `nth` counts from the kernel's current epoch, starting at 1.
 // arrive_all: thread p (p < world) tells rank p, with a fence and a store, that this
@@ -158,12 +169,7 @@ __device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src,
 __device__ __forceinline__ void arrive_all(const CommCtx &ctx, int rank, BlockSync *s, int nth)
 {
     __syncthreads();
-    const int p = static_cast<int>(threadIdx.x);
-    if (p < ctx.world) {
-        fence_ranks(ctx);
-        st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank],
-                           s->epoch + static_cast<uint32_t>(nth));
-    }
+    tell_all(ctx, rank, s, nth);
 }
 
 __device__ __forceinline__ bool wait_all(const CommCtx &ctx, int rank, BlockSync *s, int nth)
