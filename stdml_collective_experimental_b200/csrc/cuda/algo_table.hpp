@@ -58,13 +58,18 @@ inline size_t ll_capacity(int world, int vranks, int num_sms)
 }
 
 // The same for one call.  Against the two barriers of an in-place two-shot the exchange
-// wins at every size that fits (8 ranks, 160 KB: 14.4 us both, below that up to half).
+// wins at every size that fits with up to four ranks (4 ranks, 400 KB: 9.2 us, 10.3 with
+// barriers), and up to 1 MB over all ranks with more (8 ranks, us, barriers / mailboxes:
+// 16 KB 12.4 / 9.0, 160 KB 14.4 both, 240 KB 14.4 / 16.5).
 // Against the one barrier of a one-shot, on one GPU, by ranks (us, barrier / mailboxes):
 // 2: 512 KB 8.3 / 6.2; 4: 160 KB 8.3 / 6.2, 300 KB 8.3 / 8.2, 400 KB 8.3 / 10.0;
 // 8: 12 B 7.5 / 5.0, 16 KB 8.3 / 9.1, 160 KB 10.3 / 14.4.
 inline size_t ll_limit(int world, int vranks, size_t capacity, bool in_place_symmetric)
 {
-    if (vranks <= 1 || in_place_symmetric || world <= 2) { return capacity; }
+    if (vranks <= 1 || world <= 2) { return capacity; }
+    if (in_place_symmetric) {
+        return world <= 4 ? capacity : std::min(capacity, (1u << 20) / 16 / static_cast<size_t>(world));
+    }
     return std::min(capacity, world <= 4 ? (256u << 10) / 16 : size_t{kThreads});
 }
 
@@ -92,7 +97,12 @@ inline int select_blocks(const AlgoTuning &t, size_t nvec, int algo)
 {
     const bool owner = is_owner_algo(algo);
     const size_t work = owner ? (nvec + t.world - 1) / t.world : nvec;
-    const size_t per_block = static_cast<size_t>(kThreads) * 4;
+    // Vectors of a block where the message is small.  Over links four per thread: every
+    // block costs a flag per peer.  Between ranks of one GPU flags are cheap and a
+    // thread's vectors follow one another: one-shots take one each, as far as the grid goes
+    // (8 ranks, 80-240 KB: 10.3 us with four, 8.3 so).  Two-shots, which have world times
+    // fewer each and two barriers, gain nothing.
+    const size_t per_block = static_cast<size_t>(kThreads) * (t.vranks > 1 && !owner ? 1 : 4);
     size_t b = (work + per_block - 1) / per_block;
     size_t cap = static_cast<size_t>(t.max_blocks);
     if (algo == kAlgoNvls || algo == kAlgoNvlsOneShot) {
