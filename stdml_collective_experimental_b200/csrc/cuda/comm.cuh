@@ -276,8 +276,9 @@ struct GatherArgs {
 };
 
 struct PullArgs {
-    const void *src[kMaxRanks];  // per virtual rank (broadcast: root's only)
-    void *dst[kMaxRanks];        // per virtual rank
+    const void *src[kMaxRanks];  // per virtual rank (broadcast: root's only); nullptr: the rank
+                                 // packs nothing, its block is undefined
+    void *dst[kMaxRanks];        // per virtual rank; nullptr: the rank stores nothing
     unsigned long long off;      // arena offset of the staging slot
     unsigned long long bytes;    // per rank block
     unsigned long long stride;   // all_gather: distance between blocks in dst

@@ -4,6 +4,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <set>
+#include <type_traits>
 
 #include <cuda_runtime.h>
 
@@ -140,6 +141,14 @@ bool DeviceSession::registered_path(size_t bytes, void *stream) const
 
 namespace
 {
+// p + bytes; null stays null (a rank without a tensor has none in any chunk)
+template <typename T>
+T *advanced(T *p, size_t bytes)
+{
+    using Byte = std::conditional_t<std::is_const_v<T>, const char, char>;
+    return p == nullptr ? nullptr : static_cast<Byte *>(p) + bytes;
+}
+
 bool all_aligned16(void *const *p, int n, bool allow_null = false)
 {
     for (int i = 0; i < n; ++i) {
@@ -940,11 +949,13 @@ void DeviceSession::run_gather_chunks(std::vector<GatherCall> &calls,
         ++launches_;
         rt_check(cudaEventRecord(ev(reduced_ev_[slot]), main_s), "cudaEventRecord");
         rt_check(cudaStreamWaitEvent(unpack_s, ev(reduced_ev_[slot]), 0), "cudaStreamWaitEvent");
-        launch_check(world_->unpack_blocks(world_->ptr(rank, g.off), dsts[k][0], g.bytes,
-                                           g.sym_stride, stride, blocks_n, unpack_s,
-                                           chunk_unpack_blocks_),
-                     "unpack (chunk)");
-        ++launches_;
+        if (dsts[k][0] != nullptr) {
+            launch_check(world_->unpack_blocks(world_->ptr(rank, g.off), dsts[k][0], g.bytes,
+                                               g.sym_stride, stride, blocks_n, unpack_s,
+                                               chunk_unpack_blocks_),
+                         "unpack (chunk)");
+            ++launches_;
+        }
         rt_check(cudaEventRecord(ev(unpacked_ev_[slot]), unpack_s), "cudaEventRecord");
         used[slot] = true;
     }
@@ -1015,9 +1026,9 @@ void DeviceSession::all_gather(const void *const *in, void *const *out, size_t c
     // staged: a slot holds one block of every rank
     const bool in_capture = capturing(stream);
     const size_t slot = world_->staging_bytes();
-    const size_t chunk = world_->pulls_staged(bytes, -1)
-                             ? bytes
-                             : std::max<size_t>(16, slot / static_cast<size_t>(world) / 16 * 16);
+    const bool ring = world_->pulls_staged(bytes, -1);
+    const size_t chunk = ring ? bytes
+                              : std::max<size_t>(16, slot / static_cast<size_t>(world) / 16 * 16);
     std::vector<GatherCall> calls;
     std::vector<std::vector<const void *>> srcs;
     std::vector<std::vector<void *>> dsts;
@@ -1025,10 +1036,11 @@ void DeviceSession::all_gather(const void *const *in, void *const *out, size_t c
         srcs.emplace_back(vr);
         dsts.emplace_back(vr);
         for (int v = 0; v < vr; ++v) {
-            srcs.back()[v] = static_cast<const char *>(in[v]) + done;
-            dsts.back()[v] = static_cast<char *>(out[v]) + done;
+            srcs.back()[v] = advanced(in[v], done);
+            dsts.back()[v] = advanced(out[v], done);
         }
         GatherCall g;
+        g.ring = ring;
         g.bytes = std::min(chunk, bytes - done);
         g.sym_stride = (g.bytes + 15) / 16 * 16;
         g.stride = bytes;
@@ -1101,7 +1113,8 @@ void DeviceSession::broadcast(const void *const *in, void *const *out, size_t co
     }
 
     const bool in_capture = capturing(stream);
-    const size_t slot = world_->pulls_staged(bytes, root) ? bytes : world_->staging_bytes();
+    const bool ring = world_->pulls_staged(bytes, root);
+    const size_t slot = ring ? bytes : world_->staging_bytes();
     std::vector<GatherCall> calls;
     std::vector<std::vector<const void *>> srcs;
     std::vector<std::vector<void *>> dsts;
@@ -1109,12 +1122,11 @@ void DeviceSession::broadcast(const void *const *in, void *const *out, size_t co
         srcs.emplace_back(vr);
         dsts.emplace_back(vr);
         for (int v = 0; v < vr; ++v) {
-            srcs.back()[v] = (in != nullptr && in[v] != nullptr)
-                                 ? static_cast<const char *>(in[v]) + done
-                                 : nullptr;
-            dsts.back()[v] = static_cast<char *>(out[v]) + done;
+            srcs.back()[v] = in != nullptr ? advanced(in[v], done) : nullptr;
+            dsts.back()[v] = advanced(out[v], done);
         }
         GatherCall g;
+        g.ring = ring;
         g.bytes = std::min(slot, bytes - done);
         g.root = root;
         g.end_barrier = in_capture;

@@ -14,6 +14,7 @@
 #include <unistd.h>
 
 #include "algo_table.hpp"
+#include "arena_layout.hpp"
 #include "local_rendezvous.hpp"
 #include "offset_heap.hpp"
 #include "pull_walk.hpp"
@@ -133,9 +134,8 @@ class World final : public DeviceWorld
     DeviceWorldOptions opt_;
     int vranks_;
     size_t arena_bytes_ = 0;
-    size_t staging_off_[2] = {0, 0};
-    // mailboxes of the small all-reduce: offset, vectors of one, bytes of all
-    size_t ll_off_ = 0, ll_capacity_ = 0, ll_bytes_ = 0;
+    ArenaLayout layout_;
+    size_t ll_capacity_ = 0;   // vectors of one mailbox of the small all-reduce
     size_t ll_max_ = SIZE_MAX;  // knob ll_max_bytes: largest message that may use them
     unsigned long long staged_ops_ = 0;
     OffsetHeap heap_;
@@ -261,13 +261,10 @@ class World final : public DeviceWorld
         }
 
         const size_t staging = round_up(std::max<size_t>(o.staging_bytes, 4096), 4096);
-        staging_off_[0] = kDataOffset;
-        staging_off_[1] = kDataOffset + staging;
-        ll_off_ = kDataOffset + 2 * staging;
+        layout_.staging = staging;
         ll_capacity_ = ll_capacity(o.world, vranks_, num_sms_);
-        ll_bytes_ = 2 * static_cast<size_t>(o.world) * ll_capacity_ * 32;  // two per source
-        const size_t heap_off = ll_off_ + ll_bytes_;
-        arena_bytes_ = heap_off + round_up(o.heap_bytes, 4096);
+        layout_.mail = 2 * static_cast<size_t>(o.world) * ll_capacity_ * 32;  // two per source
+        arena_bytes_ = layout_.heap_off() + round_up(o.heap_bytes, 4096);
         opt_.staging_bytes = staging;
 
         rt_check(cudaHostAlloc(reinterpret_cast<void **>(&status_host_), sizeof(StatusBlock),
@@ -294,7 +291,8 @@ class World final : public DeviceWorld
             teardown();
             throw;
         }
-        heap_.reset(heap_off, arena_bytes_ - heap_off);
+        layout_.end = arena_bytes_;
+        heap_.reset(layout_.heap_off(), arena_bytes_ - layout_.heap_off());
     }
 
     ~World() override { teardown(); }
@@ -393,7 +391,7 @@ class World final : public DeviceWorld
         }
     }
 
-    size_t next_staging_slot() override { return staging_off_[(staged_ops_++) & 1ull]; }
+    size_t next_staging_slot() override { return layout_.slot(static_cast<int>((staged_ops_++) & 1ull)); }
 
     void set_wait_timeout_ms(unsigned long long ms) override { wait_timeout_ns_ = ms * 1000000ull; }
 
@@ -711,9 +709,8 @@ class World final : public DeviceWorld
         const size_t bytes = c.count * esize;
         const size_t nvec = (bytes + 15) / 16;
         const bool registered = c.peer_data != nullptr;
-        if (!registered &&
-            (c.off % 16 != 0 || c.off < kDataOffset || c.off + nvec * 16 > arena_bytes_)) {
-            throw std::invalid_argument("all_reduce: symmetric buffer outside the arena");
+        if (!registered && !layout_.holds(c.off, nvec * 16)) {
+            throw std::invalid_argument("all_reduce: symmetric buffer outside its slot or heap");
         }
         if (registered) {
             for (int r = 0; r < opt_.world; ++r) {
@@ -811,10 +808,8 @@ class World final : public DeviceWorld
                             ? static_cast<char *>(c.peer_push[r])
                             : ((!registered && c.push_off != 0) ? base_[r] + c.push_off : a.data[r]);
         }
-        if (!registered && c.push_off != 0 &&
-            (c.push_off % 16 != 0 || c.push_off < kDataOffset ||
-             c.push_off + nvec * 16 > arena_bytes_)) {
-            throw std::invalid_argument("all_reduce: result region outside the arena");
+        if (!registered && c.push_off != 0 && !layout_.holds(c.push_off, nvec * 16)) {
+            throw std::invalid_argument("all_reduce: result region outside its slot or heap");
         }
         if (registered && c.peer_push != nullptr) {
             for (int r = 0; r < opt_.world; ++r) {
@@ -936,7 +931,7 @@ class World final : public DeviceWorld
             a.src[v] = in[v];
             a.dst[v] = out[v];
         }
-        a.off = ll_off_;
+        a.off = layout_.mail_off();
         a.capacity = static_cast<unsigned int>(ll_capacity_);
         a.nvec = static_cast<unsigned int>(nvec);
         a.count = count;
@@ -985,9 +980,8 @@ class World final : public DeviceWorld
     int pull(const GatherArgs &g, int want_blocks, void *stream)
     {
         const PullGeometry geo = geometry_of_pull(g.bytes, g.root, want_blocks);
-        if (geo.blocks == 0) { return -1; }
-        if (g.off % 16 != 0 || g.off < kDataOffset || g.off + opt_.staging_bytes > arena_bytes_) {
-            throw std::invalid_argument("gather: staging slot outside the arena");
+        if (geo.blocks == 0 || !layout_.holds(g.off, geo.ring_bytes())) {
+            throw std::invalid_argument("gather: the ring does not fit the staging slot");
         }
         PullArgs a;
         std::memset(&a, 0, sizeof(a));
@@ -1038,18 +1032,9 @@ class World final : public DeviceWorld
         // against 640 GB/s for plain stores at 256 MB)
         const bool mc_possible = has_nvls() && !registered && opt_.world > 2;
         a.algo = c.algo >= 0 ? c.algo : pick_gather(c.bytes, c.root, mc_possible);
-        bool staged = !registered && !c.start_barrier;  // and every destination is a tensor
-        for (int v = 0; v < vranks_; ++v) {
-            staged = staged && a.dst[v] != nullptr &&
-                     (a.src[v] != nullptr || (!all_gather && a.root != rank() + v));
-        }
-        if (a.algo == kBcastPull && staged && opt_.world > 1) {
-            const int rc = pull(a, c.blocks, stream);
-            if (rc >= 0) { return rc; }  // else: the slot is too small for a ring
-        }
-        if (!registered &&
-            (c.off % 16 != 0 || c.off < kDataOffset || c.off + span > arena_bytes_)) {
-            throw std::invalid_argument("gather: symmetric region outside the arena");
+        if (c.ring) { return pull(a, c.blocks, stream); }
+        if (!registered && !layout_.holds(c.off, span)) {
+            throw std::invalid_argument("gather: region outside its slot or heap");
         }
         if (a.algo == kBcastNvls && !mc_possible) {
             throw std::invalid_argument("broadcast: NVLS needs the multicast mapping of the arena");
@@ -1173,8 +1158,8 @@ class World final : public DeviceWorld
     void clear_signals(int r)
     {
         rt_check(cudaMemset(base_[r], 0, kDataOffset), "cudaMemset(pad)");
-        if (ll_bytes_ > 0) {
-            rt_check(cudaMemset(base_[r] + ll_off_, 0, ll_bytes_), "cudaMemset(mailboxes)");
+        if (layout_.mail > 0) {
+            rt_check(cudaMemset(base_[r] + layout_.mail_off(), 0, layout_.mail), "cudaMemset(mailboxes)");
         }
     }
 

@@ -98,6 +98,9 @@ struct GatherCall {
     int use_mc = -1;     // -1 pick; push through the switch (needs NVLS and an arena region)
     bool start_barrier = false;  // the region is live memory of its owner (zero-copy)
     bool end_barrier = false;
+    // `off` is a staging slot in which the call keeps a ring only (pulls_staged() said so
+    // for the whole message): any length, and a rank without a destination takes part.
+    bool ring = false;
 };
 
 class DeviceWorld
@@ -176,7 +179,8 @@ class DeviceWorld
                                   void *stream) = 0;
     virtual int gather(const GatherCall &c, void *stream) = 0;
     // Whether a staged all_gather (root < 0) or broadcast of `bytes` per block goes by
-    // pull through a ring in the slot: then one call of any length will do.
+    // pull through a ring in the slot: then one call of any length will do (GatherCall::ring).
+    // Every rank gets the same answer: it depends on nothing that a rank passes of its own.
     virtual bool pulls_staged(size_t bytes, int root) const = 0;
     // Two-shot all-reduce over a table of registered tensors (see PeerEntry).
     virtual int group_peer(const PeerEntry *table, int ntable, size_t nvec, int dt, int op,

@@ -52,7 +52,8 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
     const int rank = ctx.rank + vr;
     const int world = ctx.world;
     const bool bcast = a.root >= 0;
-    const bool packs = !bcast || a.root == rank;
+    const bool packs = (!bcast || a.root == rank) && a.src[vr] != nullptr;
+    const bool stores = a.dst[vr] != nullptr;
     const PullWalk walk{a.bytes, a.stride, static_cast<int>(gridDim.x),
                         static_cast<int>(blockIdx.x), a.tile_shift};
     sync_begin(ctx, rank, &sync);
@@ -73,10 +74,10 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
 
     const PullBlock &own = blocks[rank];
     const ShiftedSource src(a.src[vr], a.bytes, own.phase);
-    const bool in_place = own.base + own.phase == a.src[vr];
+    const bool ring_only = !stores || own.base + own.phase == a.src[vr];  // own block: packed, not stored
     char *ring = ctx.base[rank] + a.off;
     const int per_tile = a.tile_shift - kPullStepShift;  // log2 of the steps in a tile
-    const int sources = bcast ? (a.root == rank ? 0 : 1) : world - 1;
+    const int sources = !stores ? 0 : bcast ? (a.root == rank ? 0 : 1) : world - 1;
     const int steps = sources << per_tile;
     // steps go through one source after the other, starting with the next rank so that
     // peers do not all read the same GPU first; everything about a step but the
@@ -112,7 +113,7 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
                         const unsigned int i = (static_cast<unsigned int>(q0 + u) << kPullStepShift) + threadIdx.x;
                         if (q0 + u >= 1 << per_tile || v0 + i >= own.nvec) { continue; }
                         st_arena_v4(to + i * 16u, x[u]);
-                        if (in_place) { continue; }
+                        if (ring_only) { continue; }
                         if (own.inside(v0 + i - threadIdx.x)) {
                             st_stream_v4(own.base + (v0 + i) * 16ull, x[u], policy);
                         } else {
@@ -200,7 +201,8 @@ __global__ void __launch_bounds__(kPullLongThreads, kPullPerSm)
     const int rank = ctx.rank + vr;
     const int world = ctx.world;
     const bool bcast = a.root >= 0;
-    const bool packs = !bcast || a.root == rank;
+    const bool packs = (!bcast || a.root == rank) && a.src[vr] != nullptr;
+    const bool stores = a.dst[vr] != nullptr;
     const PullWalk walk{a.bytes, a.stride, static_cast<int>(gridDim.x),
                         static_cast<int>(blockIdx.x), a.tile_shift};
     sync_begin(ctx, rank, &sync);
@@ -226,12 +228,12 @@ __global__ void __launch_bounds__(kPullLongThreads, kPullPerSm)
 
     const PullBlock &own = blocks[rank];
     const ShiftedSource src(a.src[vr], a.bytes, own.phase);
-    const bool in_place = own.base + own.phase == a.src[vr];
+    const bool ring_only = !stores || own.base + own.phase == a.src[vr];  // own block: packed, not stored
     const bool by_bulk = own.aligned;  // alike for all blocks of a destination
     char *ring = ctx.base[rank] + a.off;
     const unsigned long long tile = 1ull << a.tile_shift;
     const int steps = 1 << (a.tile_shift - kPullStepShift);
-    const int sources = bcast ? (a.root == rank ? 0 : 1) : world - 1;
+    const int sources = !stores ? 0 : bcast ? (a.root == rank ? 0 : 1) : world - 1;
     auto source_at = [&](int i) {
         if (bcast) { return a.root; }
         const int p = rank + 1 + i;
@@ -268,7 +270,7 @@ __global__ void __launch_bounds__(kPullLongThreads, kPullPerSm)
                     const unsigned int i = (static_cast<unsigned int>(q0 + u) << kPullStepShift) + threadIdx.x;
                     if (q0 + u >= steps || v0 + i >= own.nvec) { continue; }
                     st_arena_v4(to + i * 16u, x[u]);
-                    if (in_place) { continue; }
+                    if (ring_only) { continue; }
                     if (own.inside(v0 + i - threadIdx.x)) {
                         st_stream_v4(own.base + (v0 + i) * 16ull, x[u], policy);
                     } else {

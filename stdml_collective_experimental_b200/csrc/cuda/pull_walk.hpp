@@ -35,6 +35,11 @@ struct PullWalk {
 struct PullGeometry {
     int blocks = 0;  // 0: the slot cannot hold the ring of even one block
     int tile_shift = kPullStepShift, rounds = 1;
+    // of the staging slot, for all blocks
+    size_t ring_bytes() const
+    {
+        return ((static_cast<size_t>(blocks) * kPullRing) << tile_shift) * 16;
+    }
 };
 
 // Grid and tile for blocks of `bytes` bytes read from `sources` ranks: a tile gives

@@ -12,6 +12,7 @@
 #include "../cuda/group_walk.cuh"
 #include "../cuda/device_session.hpp"
 #include "../cuda/algo_table.hpp"
+#include "../cuda/arena_layout.hpp"
 #include "../cuda/offset_heap.hpp"
 #include "../cuda/pull_walk.hpp"
 #include "../cuda/staged_walk.hpp"
@@ -103,7 +104,7 @@ int main()
             continue;
         }
         const unsigned long long ring = (static_cast<unsigned long long>(kPullRing) << g.tile_shift) * 16;
-        EXPECT(ring * g.blocks <= slot);
+        EXPECT(ring * g.blocks == g.ring_bytes() && g.ring_bytes() <= slot);
         unsigned long long expect = 0;
         for (int k = 0; k < g.rounds; ++k) {
             for (int b = 0; b < g.blocks; ++b) {
@@ -218,6 +219,22 @@ int main()
             EXPECT(fill <= cap);
         }
         for (size_t i = 0; i < n; ++i) { EXPECT(covered[i] == counts[i]); }
+    }
+    // arena: a buffer ends with the slot or the heap in which it starts, and none starts in the
+    // pad or among the mailboxes
+    for (const size_t staging : {size_t{4096}, size_t{1} << 20}) {
+        ArenaLayout a;
+        a.staging = staging;
+        a.mail = 8192;
+        a.end = a.heap_off() + 65536;
+        for (int i = 0; i < 2; ++i) {
+            EXPECT(a.holds(a.slot(i), staging) && !a.holds(a.slot(i), staging + 1));
+            EXPECT(a.holds(a.slot(i) + staging - 16, 16) && !a.holds(a.slot(i) + staging - 16, 17));
+            EXPECT(!a.holds(a.slot(i) + 8, 8) && !a.holds(a.slot(i), ~size_t{0}));
+        }
+        EXPECT(!a.holds(0, 1) && !a.holds(kDataOffset - 16, 16));
+        EXPECT(!a.holds(a.mail_off(), 16) && !a.holds(a.heap_off() - 16, 16));
+        EXPECT(a.holds(a.heap_off(), 65536) && !a.holds(a.heap_off() + 16, 65536) && !a.holds(a.end, 0));
     }
     // symmetric heap: deterministic first fit, 256-byte granules, coalescing
     {

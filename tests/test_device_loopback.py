@@ -595,6 +595,43 @@ def test_pull_ring_at_every_alignment(sess, n, shift):
         sess.set_knob("bcast_push_min_bytes", 256 << 10)
 
 
+@pytest.mark.parametrize("push", [False, True])
+@pytest.mark.parametrize("n", [17, 70_001, 3_000_001])
+def test_ranks_without_a_destination_take_part(sess, n, push):
+    """all_gather and broadcast where some ranks pass no output: the others get theirs, at
+    sizes from one vector to several slots, and nothing beside the staging slot in use
+    changes (a heap tensor between its guard bands, the mailboxes)."""
+    if sess.world == 1:
+        pytest.skip("needs peers")
+    w = sess.world
+    with DeviceSession.loopback(w, heap_bytes=1 << 20, staging_bytes=1 << 20) as s:
+        for knob in ("gather_push_min_bytes", "bcast_push_min_bytes") if push else ():
+            s.set_knob(knob, 0)
+        sym = s.symm_empty(70_000, torch.uint8)
+        for t in sym:
+            t.fill_(9)
+        host = make_inputs(w, n, torch.uint8, seed=n)
+        ins = [h.cuda() for h in host]
+        for absent in ({w - 1}, set(range(1, w))):
+            outs = [None if r in absent else torch.zeros(n * w, dtype=torch.uint8, device="cuda")
+                    for r in range(w)]
+            bouts = [None if r in absent else torch.zeros(n, dtype=torch.uint8, device="cuda")
+                     for r in range(w)]
+            s.all_gather(ins, outs)
+            s.broadcast(ins, out=bouts, root=w - 1)
+            small = [torch.ones(3, device="cuda") for _ in range(w)]
+            s.all_reduce(small)
+            torch.cuda.synchronize()
+            s.check()
+            for r in set(range(w)) - absent:
+                assert torch.equal(outs[r].cpu(), torch.cat(host)), r
+                assert torch.equal(bouts[r].cpu(), host[w - 1]), r
+            for r in range(w):
+                assert torch.equal(ins[r].cpu(), host[r])
+                assert bool((small[r] == w).all()) and bool((sym[r] == 9).all())
+        s.symm_free(sym)  # reads the guard bands
+
+
 def test_kernels_against_plain_pytorch_arithmetic(sess):
     """An oracle that shares nothing with the library: the same reductions done by
     PyTorch in float32 / float64 on the host.  all_reduce (every algorithm), the
