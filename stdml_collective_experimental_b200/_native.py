@@ -1,7 +1,8 @@
 """Loader of the native runtime (``libstdml_collective_b200.so``).
 
 The library is built in-tree by ``make -C csrc`` (``build()`` below runs it) and
-is loaded with ctypes.  Nothing in this package works without it: a missing
+is loaded with ctypes; ``make -C csrc python`` builds ``_fastcall.so``, which only
+DeviceSession needs.  Nothing in this package works without it: a missing
 library is an ImportError with the build command, never a silent Python
 fallback.
 """
@@ -9,6 +10,7 @@ import ctypes
 import importlib.util
 import os
 import subprocess
+import sys
 import threading
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -23,9 +25,10 @@ _fastcall = None
 
 
 def build(jobs=None, verbose=False, target="all"):
-    """Compile the native runtime and its programs for sm_100a (needs nvcc, no GPU)."""
+    """Run one target of csrc/Makefile: ``all``, the library and its programs for sm_100a
+    (needs nvcc, no GPU); ``lib``; ``python``, the module behind DeviceSession."""
     jobs = jobs or max(2, (os.cpu_count() or 4))
-    cmd = ["make", "-C", CSRC, f"-j{jobs}", target]
+    cmd = ["make", "-C", CSRC, f"-j{jobs}", target, f"PYTHON={sys.executable}"]
     res = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if verbose or res.returncode != 0:
         print(res.stdout)
@@ -60,10 +63,10 @@ def fastcall():
         if _fastcall is None:
             if not os.path.exists(FASTCALL_PATH):
                 try:
-                    build(target="lib")
+                    build(target="python")
                 except Exception as e:
                     raise ImportError(f"{FASTCALL_PATH} is missing and could not be built ({e}); "
-                                      f"build it with `make -C {CSRC}`") from e
+                                      f"build it with `make -C {CSRC} python`") from e
             spec = importlib.util.spec_from_file_location(
                 __package__ + "._fastcall", FASTCALL_PATH)
             module = importlib.util.module_from_spec(spec)

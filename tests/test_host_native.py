@@ -39,6 +39,22 @@ def run(prog, *args, env=None, timeout=600, want_rc=0):
     return res.stdout
 
 
+def test_the_library_builds_without_python_and_the_module_without_nvcc():
+    """`make` is for C++ users too: no target but `python` may ask for an interpreter or
+    PyTorch, and a library that CMake built is all that `python` needs beside it."""
+    def plan(target):  # every command of the target, whatever is up to date
+        res = subprocess.run(["make", "-n", "-B", "-C", _native.CSRC, target, "PYTHON=no-python"],
+                             stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+        assert res.returncode == 0, res.stdout[-2000:]
+        return res.stdout
+    for target in ("all", "lib", "programs"):
+        out = plan(target)
+        assert "libstdml_collective_b200.so" in out
+        assert "no-python" not in out and "torch" not in out and "fastcall" not in out, target
+    out = plan("python")
+    assert "fastcall.cpp" in out and "nvcc" not in out
+
+
 def test_unit():
     assert "test-unit: OK" in run("test_unit")
 
