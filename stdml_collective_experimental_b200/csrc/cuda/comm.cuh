@@ -226,7 +226,7 @@ struct GroupPeerArgs {
 struct StagedArgs {
     // Per virtual rank (index blockIdx.y); real multi-GPU launches use [0].
     const void *src[kMaxRanks];
-    void *dst[kMaxRanks];
+    void *dst[kMaxRanks];  // nullptr: the rank stores nothing
     const GroupEntry *table[kMaxRanks];  // non-null: fused group, src/dst unused
     unsigned long long off;    // arena offset of the staging slot
     unsigned long long count;  // elements (single buffer)
@@ -244,7 +244,7 @@ struct StagedArgs {
 // All-reduce in one exchange through the mailboxes of the arena (kernels_ll.cu).
 struct LlArgs {
     const void *src[kMaxRanks];  // per virtual rank
-    void *dst[kMaxRanks];
+    void *dst[kMaxRanks];        // nullptr: the rank stores nothing
     unsigned long long off;    // arena offset of the mailboxes
     unsigned int capacity;     // vectors of one mailbox
     unsigned int nvec;

@@ -377,8 +377,8 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
             srcs.emplace_back(vr);
             dsts.emplace_back(vr);
             for (int v = 0; v < vr; ++v) {
-                srcs.back()[v] = static_cast<const char *>(in[v]) + done * es;
-                dsts.back()[v] = static_cast<char *>(out[v]) + done * es;
+                srcs.back()[v] = advanced(in[v], done * es);
+                dsts.back()[v] = advanced(out[v], done * es);
             }
             AllReduceCall k = c;
             k.count = std::min(chunk, count - done);
@@ -397,8 +397,8 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
     for (size_t done = 0; done < count; done += slot_elems) {
         const size_t n = std::min(slot_elems, count - done);
         for (int v = 0; v < vr; ++v) {
-            src[v] = static_cast<const char *>(in[v]) + done * es;
-            dst[v] = static_cast<char *>(out[v]) + done * es;
+            src[v] = advanced(in[v], done * es);
+            dst[v] = advanced(out[v], done * es);
         }
         AllReduceCall k = c;
         k.off = world_->next_staging_slot();
@@ -446,9 +446,7 @@ void DeviceSession::reduce(const void *const *in, void *const *out, size_t count
         for (size_t done = 0; done < count; done += small ? count : slot_elems) {
             const size_t n = small ? count : std::min(slot_elems, count - done);
             for (int v = 0; v < vr; ++v) {
-                dsts[v] = (out != nullptr && out[v] != nullptr)
-                              ? static_cast<char *>(out[v]) + done * es
-                              : nullptr;
+                dsts[v] = out != nullptr ? advanced(out[v], done * es) : nullptr;
             }
             AllReduceCall k;
             k.dt = dt;
@@ -546,10 +544,8 @@ void DeviceSession::reduce(const void *const *in, void *const *out, size_t count
         srcs.emplace_back(vr);
         dsts.emplace_back(vr);
         for (int v = 0; v < vr; ++v) {
-            srcs.back()[v] = static_cast<const char *>(in[v]) + done * es;
-            dsts.back()[v] = (out != nullptr && out[v] != nullptr)
-                                 ? static_cast<char *>(out[v]) + done * es
-                                 : nullptr;
+            srcs.back()[v] = advanced(in[v], done * es);
+            dsts.back()[v] = out != nullptr ? advanced(out[v], done * es) : nullptr;
         }
         AllReduceCall k;
         k.dt = dt;

@@ -886,8 +886,8 @@ class World final : public DeviceWorld
             a.src[v] = c.src != nullptr ? c.src[v] : nullptr;
             a.dst[v] = c.dst != nullptr ? c.dst[v] : nullptr;
             a.table[v] = c.table != nullptr ? c.table[v] : nullptr;
-            if (a.table[v] == nullptr && (a.src[v] == nullptr || a.dst[v] == nullptr)) {
-                throw std::invalid_argument("all_reduce: staged calls need a source and a destination");
+            if (a.table[v] == nullptr && a.src[v] == nullptr) {
+                throw std::invalid_argument("all_reduce: every rank needs a source");
             }
         }
         a.off = c.off;
@@ -927,7 +927,7 @@ class World final : public DeviceWorld
         LlArgs a;
         std::memset(&a, 0, sizeof(a));
         for (int v = 0; v < vranks_; ++v) {
-            if (in[v] == nullptr || out[v] == nullptr) { return false; }
+            if (in[v] == nullptr) { return false; }
             a.src[v] = in[v];
             a.dst[v] = out[v];
         }

@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(kThreads, 2)
                 }
             }
         }
-        if (ok) {
+        if (ok && a.dst[vr] != nullptr) {
             store_user_vec<DT>(a.dst[vr], false, v, a.count, ptr_aligned16(a.dst[vr]),
                                acc.finish(a.scale, a.has_scale != 0));
         }

@@ -205,6 +205,8 @@ __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
     slow.count = a.count;
     slow.first = slow.last = 0;
     slow.user_f32 = user_f32 ? 1 : 0;
+    // a rank without a destination serves its shard for the others and stores nothing of its own
+    const bool stores = tab != nullptr || slow.dst != nullptr;
 
     const bool searchable = tab != nullptr && a.ntable <= kStagedStarts && a.nvec >> 32 == 0;
     slow.starts = searchable ? starts : nullptr;
@@ -362,6 +364,7 @@ __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
                 for (int r = 0; r < world; ++r) {
                     if (r != rank) { st_arena_v4(ctx.base[r] + byte, res); }
                 }
+                if (!stores) { continue; }
                 if (fast) {
                     store_fast<DT>(d.dst, i, user_f32, res, policy);
                 } else {
@@ -370,7 +373,7 @@ __global__ void __launch_bounds__(kStagedThreads, kStagedPerSm)
             }
         }
         if (k <= rounds) { arrive_all(ctx, rank, &sync, k + 1); }
-        if (k > 1) {
+        if (k > 1 && stores) {
             // ---- unpack tile k-2 of every shard but the own one
             const char *from = mine + walk.piece(k - 2, 0);
             const TileDesc *ds = descs[(k - 2) & 3];

@@ -598,9 +598,9 @@ def test_pull_ring_at_every_alignment(sess, n, shift):
 @pytest.mark.parametrize("push", [False, True])
 @pytest.mark.parametrize("n", [17, 70_001, 3_000_001])
 def test_ranks_without_a_destination_take_part(sess, n, push):
-    """all_gather and broadcast where some ranks pass no output: the others get theirs, at
-    sizes from one vector to several slots, and nothing beside the staging slot in use
-    changes (a heap tensor between its guard bands, the mailboxes)."""
+    """all_gather, broadcast and all_reduce where some ranks pass no output: the others get
+    theirs, at sizes from one vector to several slots, and nothing beside the staging slot in
+    use changes (a heap tensor between its guard bands, the mailboxes)."""
     if sess.world == 1:
         pytest.skip("needs peers")
     w = sess.world
@@ -619,6 +619,9 @@ def test_ranks_without_a_destination_take_part(sess, n, push):
                      for r in range(w)]
             s.all_gather(ins, outs)
             s.broadcast(ins, out=bouts, root=w - 1)
+            routs = [None if r in absent else torch.zeros(n, dtype=torch.uint8, device="cuda")
+                     for r in range(w)]
+            s.all_reduce(ins, out=routs, op="bit_xor")
             small = [torch.ones(3, device="cuda") for _ in range(w)]
             s.all_reduce(small)
             torch.cuda.synchronize()
@@ -626,6 +629,7 @@ def test_ranks_without_a_destination_take_part(sess, n, push):
             for r in set(range(w)) - absent:
                 assert torch.equal(outs[r].cpu(), torch.cat(host)), r
                 assert torch.equal(bouts[r].cpu(), host[w - 1]), r
+                assert torch.equal(routs[r].cpu(), reduce_many(host, "bit_xor")), r
             for r in range(w):
                 assert torch.equal(ins[r].cpu(), host[r])
                 assert bool((small[r] == w).all()) and bool((sym[r] == 9).all())
