@@ -45,10 +45,12 @@ inline size_t nvls_oneshot_limit(const AlgoTuning &t)
     return 2u << 20;
 }
 
-// Vectors of the largest message that goes through the mailboxes (kernels_ll.cu).  They
-// carry twice the bytes, so over links the exchange pays only while the time is its
-// latency (64 KB, where protocols of this kind usually end).  Between ranks of one GPU
-// doubled bytes are L2 traffic; the limit is one vector per thread, two blocks of 512 per SM.
+// Vectors of one mailbox, the most that a message may have (kernels_ll.cu).  Between ranks
+// of one GPU: one vector per thread, two blocks of 512 per SM, 512 KB at most.  Over links
+// 64 KB; that is an estimate, no measurement (the exchange sends the bytes twice, 64 KB more
+// to each of up to 7 peers, 0.6 us at 770 GB/s, and spares a fence, a flag and the round
+// trip of the peer loads, 2 us between ranks of one GPU and no less over links).  The knob
+// ll_max_bytes moves it, 0 gives the kernels with barriers back.
 inline size_t ll_capacity(int world, int vranks, int num_sms)
 {
     if (world < 2) { return 0; }
@@ -57,20 +59,27 @@ inline size_t ll_capacity(int world, int vranks, int num_sms)
                             static_cast<size_t>(std::max(1, 2 * num_sms / vranks)) * kThreads);
 }
 
-// The same for one call.  Against the two barriers of an in-place two-shot the exchange
-// wins at every size that fits with up to four ranks (4 ranks, 400 KB: 9.2 us, 10.3 with
-// barriers), and up to 1 MB over all ranks with more (8 ranks, us, barriers / mailboxes:
-// 16 KB 12.4 / 9.0, 160 KB 14.4 both, 240 KB 14.4 / 16.5).
-// Against the one barrier of a one-shot, on one GPU, by ranks (us, barrier / mailboxes):
-// 2: 512 KB 8.3 / 6.2; 4: 160 KB 8.3 / 6.2, 300 KB 8.3 / 8.2, 400 KB 8.3 / 10.0;
-// 8: 12 B 7.5 / 5.0, 16 KB 8.3 / 9.1, 160 KB 10.3 / 14.4.
+// Vectors of the largest message that goes through the mailboxes.  Between ranks of one GPU,
+// f32, us per call (barriers / mailboxes; a call's time moves in steps of 2 us).
+// In place in the heap, against a two-shot and its two barriers:
+//   2 ranks: 16 KB 8.2 / 4.4, 512 KB 10.0 / 6.2; 4: 16 KB 8.2 / 6.2, 400 KB 10.3 / 9.5, 512 KB 10.3 both;
+//   6: 16 KB 8.4 / 8.2, 147 KB 11.6 / 8.3; 7: 147 KB 11.1 / 10.3;
+//   8: 4 KB 8.2 / 6.3, 6 KB 8.2 both, 24 KB 8.5 / 10.1, 115 KB 10.3 both;
+//   10: 4 KB 9.4 / 8.2, 6 KB 8.7 / 10.3; 16: 3 KB 10.3 / 8.2, 6 KB 10.3 / 12.3.
+// Out of place, against a one-shot and its one barrier:
+//   2 ranks: 512 KB 7.2 / 6.2; 3: 400 KB 8.2 / 6.9; 4: 262 KB 8.2 / 6.9, 307 KB 8.2 both, 400 KB 8.2 / 9.5;
+//   6: 4 KB 6.2 both, 115 KB 8.2 both; 8: 12 B 6.8 / 4.1, 4 KB 6.2-7.6 / 6.3, 6 KB 7.3 / 8.2;
+//   12: 2 KB 8.2 / 6.5, 6 KB 8.2 / 10.3; 16: 1.5 KB 8.2 / 6.2, 4 KB 8.2 / 10.3.
 inline size_t ll_limit(int world, int vranks, size_t capacity, bool in_place_symmetric)
 {
     if (vranks <= 1 || world <= 2) { return capacity; }
+    const auto over_all_ranks = [&](size_t kb) {
+        return std::min(capacity, (kb << 10) / 16 / static_cast<size_t>(world));
+    };
     if (in_place_symmetric) {
-        return world <= 4 ? capacity : std::min(capacity, (1u << 20) / 16 / static_cast<size_t>(world));
+        return world <= 4 ? capacity : over_all_ranks(world < 8 ? 1024 : 48);
     }
-    return std::min(capacity, world <= 4 ? (256u << 10) / 16 : size_t{kThreads});
+    return world <= 4 ? std::min(capacity, size_t{256u << 10} / 16) : over_all_ranks(32);
 }
 
 // need_owner: the result must stay in the symmetric buffer (in place), which

@@ -355,6 +355,19 @@ int main()
             }
         }
     }
+    {   // mailboxes: a message never outgrows one, and with more ranks none has a higher limit
+        for (int w = 2; w <= kMaxRanks; ++w) {
+            for (const bool sym : {false, true}) {
+                const size_t cap = ll_capacity(w, w, 148), most = ll_limit(w, w, cap, sym);
+                EXPECT(most >= 1 && most <= cap && cap <= 2u * 148u / w * kThreads);
+                EXPECT(w == 2 || most <= ll_limit(w - 1, w - 1, ll_capacity(w - 1, w - 1, 148), sym));
+                EXPECT(ll_limit(w, 1, ll_capacity(w, 1, 148), sym) == (64u << 10) / 16);
+            }
+        }
+        EXPECT(ll_capacity(1, 1, 148) == 0);
+        EXPECT(ll_limit(8, 8, ll_capacity(8, 8, 148), false) == (4u << 10) / 16);
+        EXPECT(ll_limit(8, 8, ll_capacity(8, 8, 148), true) == (6u << 10) / 16);
+    }
     {   // the rules of the in-kernel argument checks
         EXPECT(buffer_offset_ok(kDataOffset) && buffer_offset_ok(kDataOffset + 4096) && buffer_offset_ok(0));
         EXPECT(!buffer_offset_ok(kDataOffset + 8) && !buffer_offset_ok(64) && !buffer_offset_ok(kDataOffset - 16));
