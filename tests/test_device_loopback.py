@@ -38,6 +38,20 @@ def sess(request):
     s.close()
 
 
+@pytest.fixture
+def tuned(sess):
+    """The same kind of session for one test alone: it may turn any knob."""
+    with DeviceSession.loopback(sess.world, heap_bytes=32 << 20, staging_bytes=1 << 20) as s:
+        yield s
+
+
+@pytest.fixture(params=[2, 3, 4, 8])
+def job(request):
+    """The staging slots of a job (64 MB): tiles of several steps, rings of the full grid."""
+    with DeviceSession.loopback(request.param, heap_bytes=20 << 20, staging_bytes=64 << 20) as s:
+        yield s
+
+
 def same(a, b):
     if a.dtype.is_floating_point:
         return torch.equal(a.view(torch.uint8), b.view(torch.uint8)) or torch.equal(a, b)
@@ -255,71 +269,69 @@ def test_group_all_reduce_fused(sess, dtype):
     sess.check()
 
 
-@pytest.mark.parametrize("bulk", [False, True])
+@pytest.mark.parametrize("bulk", [False, True, "short tiles"])
 @pytest.mark.parametrize("dtype,op,scale", [
     (torch.float32, "sum", 0.125), (torch.bfloat16, "sum", None), (torch.int32, "max", None),
     (torch.float64, "prod", 1.0 / 3.0), (torch.int8, "bit_xor", None), (torch.float16, "min", None),
 ])
-def test_group_all_reduce_on_registered_loose_tensors(sess, dtype, op, scale, bulk):
+def test_group_all_reduce_on_registered_loose_tensors(tuned, dtype, op, scale, bulk):
     """Separately allocated tensors, reduced where they lie: one launch, no staging.
     `bulk`: operands come in by bulk asynchronous copies into a shared-memory ring
     (the default from 4 MB up), else by 16-byte peer loads."""
-    if sess.world == 1:
+    if tuned.world == 1:
         pytest.skip("needs peers")
-    sess.set_knob("group_bulk_min_bytes", 0 if bulk else -1)
+    tuned.set_knob("group_bulk_min_bytes", 0 if bulk else -1)
+    if bulk == "short tiles":  # more chunks of tiles than blocks: most are drawn by ticket
+        tuned.set_knob("tma_tile_vec", 32)
     sizes = [1, 7, 768, 3, 2304, 590_000, 5, 64, 1000, 123_457, 2, 768]
     host = [[make_inputs(1, n, dtype, seed=31 * r + i, small=op == "prod")[0]
-             for i, n in enumerate(sizes)] for r in range(sess.world)]
-    want = [reduce_many([host[r][i] for r in range(sess.world)], op, scale)
+             for i, n in enumerate(sizes)] for r in range(tuned.world)]
+    want = [reduce_many([host[r][i] for r in range(tuned.world)], op, scale)
             for i in range(len(sizes))]
-    sess.set_knob("register_min_bytes", 0)
-    try:
-        # in place, twice (the second call reuses the table of peer pointers)
-        for _ in range(2):
-            dev = [[t.cuda() for t in host[r]] for r in range(sess.world)]
-            before = sess.launches
-            sess.group_all_reduce(dev if sess.vranks > 1 else dev[0], op=op, scale=scale)
-            torch.cuda.synchronize()
-            sess.check()
-            assert sess.launches == before + 1
-            for r in range(sess.world):
-                for i in range(len(sizes)):
-                    assert same(dev[r][i].cpu(), want[i]), (r, i)
-        # out of place: inputs stay, outputs carry the result and nothing beyond their end
-        dev = [[t.cuda() for t in host[r]] for r in range(sess.world)]
-        pad = 16
-        outs = [[torch.full((n + pad,), 3, dtype=dtype, device="cuda") for n in sizes]
-                for _ in range(sess.world)]
-        views = [[o[:n] for o, n in zip(outs[r], sizes)] for r in range(sess.world)]
-        before = sess.launches
-        sess.group_all_reduce(dev if sess.vranks > 1 else dev[0],
-                              outs=views if sess.vranks > 1 else views[0], op=op, scale=scale)
+    tuned.set_knob("register_min_bytes", 0)
+    # in place, twice (the second call reuses the table of peer pointers)
+    for _ in range(2):
+        dev = [[t.cuda() for t in host[r]] for r in range(tuned.world)]
+        before = tuned.launches
+        tuned.group_all_reduce(dev if tuned.vranks > 1 else dev[0], op=op, scale=scale)
         torch.cuda.synchronize()
-        sess.check()
-        assert sess.launches == before + 1
-        for r in range(sess.world):
-            for i, n in enumerate(sizes):
-                assert same(views[r][i].cpu(), want[i]), (r, i)
-                assert bool((outs[r][i][n:] == 3).all()), "wrote past the end of a tensor"
-                assert torch.equal(dev[r][i].cpu(), host[r][i]), "inputs must stay untouched"
-        # a tensor that does not start on a 16-byte boundary sends the set the staged way
-        dev = [[t.cuda() for t in host[r]] for r in range(sess.world)]
-        for r in range(sess.world):
-            odd = torch.empty(sizes[5] + 1, dtype=dtype, device="cuda")[1:]
-            if odd.data_ptr() % 16 != 0:
-                odd.copy_(host[r][5])
-                dev[r][5] = odd
-        before = sess.launches
-        sess.group_all_reduce(dev if sess.vranks > 1 else dev[0], op=op, scale=scale)
-        torch.cuda.synchronize()
-        sess.check()
-        assert sess.launches > before
-        for r in range(sess.world):
+        tuned.check()
+        assert tuned.launches == before + 1
+        for r in range(tuned.world):
             for i in range(len(sizes)):
                 assert same(dev[r][i].cpu(), want[i]), (r, i)
-    finally:
-        sess.set_knob("register_min_bytes", -1)
-        sess.set_knob("group_bulk_min_bytes", 4 << 20)
+    # out of place: inputs stay, outputs carry the result and nothing beyond their end
+    dev = [[t.cuda() for t in host[r]] for r in range(tuned.world)]
+    pad = 16
+    outs = [[torch.full((n + pad,), 3, dtype=dtype, device="cuda") for n in sizes]
+            for _ in range(tuned.world)]
+    views = [[o[:n] for o, n in zip(outs[r], sizes)] for r in range(tuned.world)]
+    before = tuned.launches
+    tuned.group_all_reduce(dev if tuned.vranks > 1 else dev[0],
+                          outs=views if tuned.vranks > 1 else views[0], op=op, scale=scale)
+    torch.cuda.synchronize()
+    tuned.check()
+    assert tuned.launches == before + 1
+    for r in range(tuned.world):
+        for i, n in enumerate(sizes):
+            assert same(views[r][i].cpu(), want[i]), (r, i)
+            assert bool((outs[r][i][n:] == 3).all()), "wrote past the end of a tensor"
+            assert torch.equal(dev[r][i].cpu(), host[r][i]), "inputs must stay untouched"
+    # a tensor that does not start on a 16-byte boundary sends the set the staged way
+    dev = [[t.cuda() for t in host[r]] for r in range(tuned.world)]
+    for r in range(tuned.world):
+        odd = torch.empty(sizes[5] + 1, dtype=dtype, device="cuda")[1:]
+        if odd.data_ptr() % 16 != 0:
+            odd.copy_(host[r][5])
+            dev[r][5] = odd
+    before = tuned.launches
+    tuned.group_all_reduce(dev if tuned.vranks > 1 else dev[0], op=op, scale=scale)
+    torch.cuda.synchronize()
+    tuned.check()
+    assert tuned.launches > before
+    for r in range(tuned.world):
+        for i in range(len(sizes)):
+            assert same(dev[r][i].cpu(), want[i]), (r, i)
 
 
 def test_group_all_reduce_bf16_wire_for_f32_grads(sess):
@@ -472,53 +484,47 @@ def test_zero_copy_all_gather_broadcast_reduce_on_symmetric_buffers(sess, n):
         sess.symm_free(sym)
 
 
-def test_broadcast_in_rounds(sess):
+def test_broadcast_in_rounds(tuned):
     """The pipelined broadcast (root sends in rounds and signals, holders forward
     while root goes on) at sizes from one vector to many rounds, staged and on
     symmetric buffers, from both ends of the rank range."""
-    if sess.world < 3:
+    if tuned.world < 3:
         pytest.skip("used from three ranks up")
-    sess.set_knob("bcast_pipelined_min_bytes", 0)
-    try:
-        for n in (1, 17, 5000, 300_001, 2_000_003):
-            host = make_inputs(sess.world, n, torch.float32, seed=n + 1)
-            for root in sorted({0, sess.world - 1}):
-                dev = [h.cuda() for h in host]
-                sess.broadcast(dev, root=root)
+    tuned.set_knob("bcast_pipelined_min_bytes", 0)
+    for n in (1, 17, 5000, 300_001, 2_000_003):
+        host = make_inputs(tuned.world, n, torch.float32, seed=n + 1)
+        for root in sorted({0, tuned.world - 1}):
+            dev = [h.cuda() for h in host]
+            tuned.broadcast(dev, root=root)
+            if n * 4 <= (4 << 20):
+                sym = tuned.symm_empty(n, torch.float32)
+                for r in range(tuned.world):
+                    sym[r].copy_(host[r])
+                tuned.broadcast(sym, root=root)
+            torch.cuda.synchronize()
+            tuned.check()
+            for r in range(tuned.world):
+                assert torch.equal(dev[r].cpu(), host[root]), (n, root, r)
                 if n * 4 <= (4 << 20):
-                    sym = sess.symm_empty(n, torch.float32)
-                    for r in range(sess.world):
-                        sym[r].copy_(host[r])
-                    sess.broadcast(sym, root=root)
-                torch.cuda.synchronize()
-                sess.check()
-                for r in range(sess.world):
-                    assert torch.equal(dev[r].cpu(), host[root]), (n, root, r)
-                    if n * 4 <= (4 << 20):
-                        assert torch.equal(sym[r].cpu(), host[root]), (n, root, r, "symmetric")
-                if n * 4 <= (4 << 20):
-                    sess.symm_free(sym)
-    finally:
-        sess.set_knob("bcast_pipelined_min_bytes", 8 << 20)
+                    assert torch.equal(sym[r].cpu(), host[root]), (n, root, r, "symmetric")
+            if n * 4 <= (4 << 20):
+                tuned.symm_free(sym)
 
 
 @pytest.mark.parametrize("algo_knob", [0, 1 << 40])
-def test_all_gather_push_and_pull_agree(sess, algo_knob):
-    sess.set_knob("gather_push_min_bytes", algo_knob)  # 0: always push; huge: always pull
-    try:
-        for n in (3, 1000, 70_001):
-            host = make_inputs(sess.world, n, torch.int16, seed=n)
-            outs = [torch.empty(n * sess.world, dtype=torch.int16, device="cuda")
-                    for _ in range(sess.world)]
-            ins = [h.cuda() for h in host]
-            sess.all_gather(ins if sess.vranks > 1 else ins[0],
-                            outs if sess.vranks > 1 else outs[0])
-            torch.cuda.synchronize()
-            sess.check()
-            for r in range(sess.world):
-                assert torch.equal(outs[r].cpu(), torch.cat(host)), (n, r)
-    finally:
-        sess.set_knob("gather_push_min_bytes", 64 << 10)
+def test_all_gather_push_and_pull_agree(tuned, algo_knob):
+    tuned.set_knob("gather_push_min_bytes", algo_knob)  # 0: always push; huge: always pull
+    for n in (3, 1000, 70_001):
+        host = make_inputs(tuned.world, n, torch.int16, seed=n)
+        outs = [torch.empty(n * tuned.world, dtype=torch.int16, device="cuda")
+                for _ in range(tuned.world)]
+        ins = [h.cuda() for h in host]
+        tuned.all_gather(ins if tuned.vranks > 1 else ins[0],
+                        outs if tuned.vranks > 1 else outs[0])
+        torch.cuda.synchronize()
+        tuned.check()
+        for r in range(tuned.world):
+            assert torch.equal(outs[r].cpu(), torch.cat(host)), (n, r)
 
 
 @pytest.mark.parametrize("dtype,op", [(torch.float32, "sum"), (torch.bfloat16, "sum"),
@@ -559,40 +565,35 @@ def test_small_all_reduce_in_one_exchange(sess, dtype, op):
 
 @pytest.mark.parametrize("shift", [0, 4, 5])
 @pytest.mark.parametrize("n", [1, 15, 16, 17, 4097, 70_001, 3_000_001])
-def test_pull_ring_at_every_alignment(sess, n, shift):
+def test_pull_ring_at_every_alignment(tuned, n, shift):
     """Staged all_gather and broadcast by pull: sizes around a vector, a tile and many
     rounds, sources and destinations that start `shift` bytes off a vector boundary;
     nothing beyond a destination's own bytes may change."""
-    if sess.world == 1:
+    if tuned.world == 1:
         pytest.skip("needs peers")
-    w = sess.world
-    sess.set_knob("gather_push_min_bytes", -1)
-    sess.set_knob("bcast_pipelined_min_bytes", -1)
-    sess.set_knob("bcast_push_min_bytes", -1)
-    try:
-        host = make_inputs(w, n, torch.uint8, seed=n)
-        ins = [torch.zeros(n + 16, dtype=torch.uint8, device="cuda")[shift:shift + n] for _ in range(w)]
-        for t, h in zip(ins, host):
-            t.copy_(h)
-        pads = [torch.full((n * w + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
-        outs = [p[16 + shift:16 + shift + n * w] for p in pads]
-        sess.all_gather(ins, outs)
-        bpads = [torch.full((n + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
-        bouts = [p[16 + shift:16 + shift + n] for p in bpads]
-        sess.broadcast(ins, out=bouts, root=w - 1)
-        sess.broadcast(ins, root=0)  # in place
-        torch.cuda.synchronize()
-        sess.check()
-        for r in range(w):
-            assert torch.equal(outs[r].cpu(), torch.cat(host)), r
-            assert bool((pads[r][:16 + shift] == 7).all() and (pads[r][16 + shift + n * w:] == 7).all())
-            assert torch.equal(bouts[r].cpu(), host[w - 1]), r
-            assert bool((bpads[r][:16 + shift] == 7).all() and (bpads[r][16 + shift + n:] == 7).all())
-            assert torch.equal(ins[r].cpu(), host[0]), r
-    finally:
-        sess.set_knob("gather_push_min_bytes", 64 << 10)
-        sess.set_knob("bcast_pipelined_min_bytes", 8 << 20)
-        sess.set_knob("bcast_push_min_bytes", 256 << 10)
+    w = tuned.world
+    tuned.set_knob("gather_push_min_bytes", -1)
+    tuned.set_knob("bcast_pipelined_min_bytes", -1)
+    tuned.set_knob("bcast_push_min_bytes", -1)
+    host = make_inputs(w, n, torch.uint8, seed=n)
+    ins = [torch.zeros(n + 16, dtype=torch.uint8, device="cuda")[shift:shift + n] for _ in range(w)]
+    for t, h in zip(ins, host):
+        t.copy_(h)
+    pads = [torch.full((n * w + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
+    outs = [p[16 + shift:16 + shift + n * w] for p in pads]
+    tuned.all_gather(ins, outs)
+    bpads = [torch.full((n + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
+    bouts = [p[16 + shift:16 + shift + n] for p in bpads]
+    tuned.broadcast(ins, out=bouts, root=w - 1)
+    tuned.broadcast(ins, root=0)  # in place
+    torch.cuda.synchronize()
+    tuned.check()
+    for r in range(w):
+        assert torch.equal(outs[r].cpu(), torch.cat(host)), r
+        assert bool((pads[r][:16 + shift] == 7).all() and (pads[r][16 + shift + n * w:] == 7).all())
+        assert torch.equal(bouts[r].cpu(), host[w - 1]), r
+        assert bool((bpads[r][:16 + shift] == 7).all() and (bpads[r][16 + shift + n:] == 7).all())
+        assert torch.equal(ins[r].cpu(), host[0]), r
 
 
 @pytest.mark.parametrize("push", [False, True])
@@ -634,6 +635,123 @@ def test_ranks_without_a_destination_take_part(sess, n, push):
                 assert torch.equal(ins[r].cpu(), host[r])
                 assert bool((small[r] == w).all()) and bool((sym[r] == 9).all())
         s.symm_free(sym)  # reads the guard bands
+
+
+def scattered(world, dtype, aligned, seed):
+    """A set of 1100 small tensors among three large ones, 5.3 M elements in all: more entries
+    than the kernels search in shared memory, several steps per tile with 64 MB slots; unless
+    `aligned`, some tensors start off a vector boundary.  Host copies and device tensors."""
+    sizes = [1 + 37 * i % 900 for i in range(1100)]
+    sizes[0:0], sizes[500:500], sizes[1100:1100] = [1_500_001], [1_600_000], [1_700_003]
+    host = [make_inputs(1, sum(sizes), dtype, seed=seed + r)[0] for r in range(world)]
+    dev = []
+    for h in host:
+        flat = torch.empty(sum(sizes) + 16 * len(sizes), dtype=dtype, device="cuda")
+        lanes, at, row = 16 // flat.element_size(), 0, []
+        for i, part in enumerate(torch.split(h, sizes)):
+            at = -(-at // lanes) * lanes + (0 if aligned or i % 7 else 1)
+            row.append(flat[at:at + part.numel()])
+            at += part.numel()
+            row[-1].copy_(part)
+        dev.append(row)
+    return host, dev
+
+
+@pytest.mark.parametrize("dtype,wire", [(torch.float32, None), (torch.float32, torch.bfloat16),
+                                        (torch.bfloat16, None)])
+def test_staged_group_at_the_slots_of_a_job(job, dtype, wire):
+    host, dev = scattered(job.world, dtype, aligned=False, seed=5)
+    job.group_all_reduce(dev, scale=0.5, wire_dtype=wire)
+    torch.cuda.synchronize()
+    job.check()
+    want = reduce_many([h.to(wire or dtype) for h in host], "sum", 0.5).to(dtype)
+    for r in range(job.world):
+        assert same(torch.cat(dev[r]).cpu(), want), r
+
+
+def test_staged_buffer_at_the_slots_of_a_job(job):
+    n = 5_300_003
+    host = make_inputs(job.world, n, torch.int32, seed=8)
+    for odd in (0, 1):
+        dev = [torch.empty(n + 1, dtype=torch.int32, device="cuda")[odd:n + odd] for _ in host]
+        out = [torch.full((n + 2,), 7, dtype=torch.int32, device="cuda") for _ in host]
+        for d, h in zip(dev, host):
+            d.copy_(h)
+        job.all_reduce(dev, out=[o[odd:n + odd] for o in out], op="max")
+        torch.cuda.synchronize()
+        job.check()
+        for r in range(job.world):
+            assert torch.equal(out[r][odd:n + odd].cpu(), reduce_many(host, "max")), (odd, r)
+            assert bool((out[r][:odd] == 7).all()) and bool((out[r][n + odd:] == 7).all())
+
+
+@pytest.mark.parametrize("bulk", [False, True])
+def test_registered_set_of_many_tensors(job, bulk):
+    """More entries than are searched in shared memory; by bulk copies, most chunks by ticket."""
+    job.set_knob("register_min_bytes", 0)
+    job.set_knob("group_bulk_min_bytes", 0 if bulk else -1)
+    job.set_knob("tma_tile_vec", 64)
+    host, dev = scattered(job.world, torch.bfloat16, aligned=True, seed=6)
+    before = job.launches
+    job.group_all_reduce(dev, scale=0.5)
+    torch.cuda.synchronize()
+    job.check()
+    assert job.launches == before + 1
+    want = reduce_many(host, "sum", 0.5)
+    for r in range(job.world):
+        assert same(torch.cat(dev[r]).cpu(), want), r
+
+
+@pytest.mark.parametrize("algo", [None, "twoshot", "twoshot_tma"])
+def test_tiles_drawn_by_ticket(job, algo):
+    """In place, 16 MB per rank: past the size from which blocks draw their tiles; three
+    calls in a row, whose counters each call has to leave at zero."""
+    n = 4_000_003
+    host = make_inputs(job.world, n, torch.float32, seed=12)
+    sym = job.symm_empty(n, torch.float32)
+    for t, h in zip(sym, host):
+        t.copy_(h)
+    for _ in range(3):
+        job.all_reduce(sym, op="max", algo=algo)
+    torch.cuda.synchronize()
+    job.check()
+    for t in sym:
+        assert same(t.cpu(), reduce_many(host, "max"))
+    for t, h in zip(sym, host):
+        t.copy_(h)
+    job.all_reduce(sym, scale=0.5, algo=algo)
+    torch.cuda.synchronize()
+    job.check()
+    for t in sym:
+        assert same(t.cpu(), reduce_many(host, "sum", 0.5))
+    job.symm_free(sym)
+
+
+@pytest.mark.parametrize("shift", [0, 5])
+def test_pull_at_the_slots_of_a_job(job, shift):
+    """all_gather and broadcast of three rounds, tiles of several steps (from three ranks up
+    the kernel of long messages), from and to addresses `shift` bytes off a vector boundary."""
+    w = job.world
+    for op, n in (("all_gather", {2: 20_000_003, 3: 14_000_001, 4: 7_000_001, 8: 2_000_003}[w]),
+                  ("broadcast", {2: 20_000_003, 3: 27_000_005, 4: 20_000_003, 8: 11_000_001}[w])):
+        host = make_inputs(w, n, torch.uint8, seed=n)
+        ins = [torch.zeros(n + 16, dtype=torch.uint8, device="cuda")[shift:shift + n] for _ in range(w)]
+        for t, h in zip(ins, host):
+            t.copy_(h)
+        want = (torch.cat(host) if op == "all_gather" else host[w - 1]).cuda()
+        pads = [torch.full((want.numel() + 48,), 7, dtype=torch.uint8, device="cuda") for _ in range(w)]
+        outs = [p[16 + shift:16 + shift + want.numel()] for p in pads]
+        if op == "all_gather":
+            job.all_gather(ins, outs)
+        else:
+            job.broadcast(ins, out=outs, root=w - 1)
+        torch.cuda.synchronize()
+        job.check()
+        for r in range(w):
+            assert torch.equal(outs[r], want), (op, r)
+            assert bool((pads[r][:16 + shift] == 7).all()), (op, r)
+            assert bool((pads[r][16 + shift + want.numel():] == 7).all()), (op, r)
+            assert torch.equal(ins[r].cpu(), host[r]), (op, r)
 
 
 def test_kernels_against_plain_pytorch_arithmetic(sess):
