@@ -81,8 +81,7 @@ DeviceSession::~DeviceSession()
             (void)cudaEventDestroy(static_cast<cudaEvent_t>(unpacked_ev_[i]));
         }
     }
-    for (void *p : table_mem_) { (void)cudaFree(p); }
-    table_mem_.clear();
+    plans_.clear();
     forget_peer_plans();
     for (void *e : host_ev_) { (void)cudaEventDestroy(static_cast<cudaEvent_t>(e)); }
     if (order_ev_ != nullptr) { (void)cudaEventDestroy(static_cast<cudaEvent_t>(order_ev_)); }
@@ -607,7 +606,7 @@ std::vector<std::vector<GroupPiece>> plan_group_pieces(size_t n, const size_t *c
 const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *const *ins,
                                                           void *const *outs,
                                                           const size_t *counts, int dt,
-                                                          int user_dt)
+                                                          int user_dt, bool in_capture)
 {
     const int vr = world_->vranks();
     std::string key;
@@ -618,12 +617,14 @@ const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *
     key.append(reinterpret_cast<const char *>(&dt), sizeof(dt));
     key.append(reinterpret_cast<const char *>(&user_dt), sizeof(user_dt));
     auto it = plans_.find(key);
-    if (it != plans_.end()) { return it->second; }
-    if (plans_.size() >= 64) {  // bounded cache; cudaFree waits for work in flight
-        for (void *p : table_mem_) { (void)cudaFree(p); }
-        table_mem_.clear();
-        plans_.clear();
+    if (it != plans_.end()) {
+        it->second.captured = it->second.captured || in_capture;
+        return it->second;
     }
+    // bounded, but for the plans whose tables a graph reads at every replay; cudaFree
+    // waits for work in flight
+    const auto loose = [](const auto &kv) { return !kv.second.captured; };
+    if (std::count_if(plans_.begin(), plans_.end(), loose) >= 64) { std::erase_if(plans_, loose); }
 
     const size_t es = elem_size(dt);                          // wire element
     const size_t ues = user_dt >= 0 ? elem_size(user_dt) : es;  // user element
@@ -636,6 +637,7 @@ const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *
     const std::vector<std::vector<Piece>> chunks = plan_group_pieces(n, counts, lanes, cap);
 
     GroupPlan plan;
+    plan.captured = in_capture;
     for (const auto &pieces : chunks) {
         if (pieces.empty()) { continue; }
         std::vector<Table> per_rank(vr);
@@ -668,7 +670,7 @@ const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *
                         first_of_tile.size() * sizeof(int));
             void *dev = nullptr;
             rt_check(cudaMalloc(&dev, image.size()), "cudaMalloc(table)");
-            table_mem_.push_back(dev);
+            plan.mem.emplace_back(dev, [](void *p) { (void)cudaFree(p); });
             rt_check(cudaMemcpy(dev, image.data(), image.size(), cudaMemcpyHostToDevice),
                      "cudaMemcpy(table)");
             per_rank[v].dev = static_cast<GroupEntry *>(dev);
@@ -852,11 +854,12 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         }
     }
 
-    const GroupPlan &plan = plan_group(n, ins, outs, counts, dt, user_dt);
+    const bool in_capture = capturing(stream);
+    const GroupPlan &plan = plan_group(n, ins, outs, counts, dt, user_dt, in_capture);
     size_t plan_bytes = 0;
     for (const auto &chunk : plan.chunks) { plan_bytes += chunk[0].nvec * 16; }
     if (world_->world() > 1 && plan.chunks.size() >= 2 && plan_bytes >= pipeline_min_bytes_ &&
-        !capturing(stream) && (algo < 0 || is_owner_algo(algo))) {
+        !in_capture && (algo < 0 || is_owner_algo(algo))) {
         std::vector<std::vector<const GroupEntry *>> all_tabs;
         std::vector<AllReduceCall> calls;
         for (const auto &chunk : plan.chunks) {
@@ -878,7 +881,6 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         return;
     }
     std::vector<const GroupEntry *> tabs(vr);
-    const bool in_capture = capturing(stream);
     for (const auto &chunk : plan.chunks) {
         for (int v = 0; v < vr; ++v) { tabs[v] = chunk[v].dev; }
         AllReduceCall c;

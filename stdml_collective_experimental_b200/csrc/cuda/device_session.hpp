@@ -111,6 +111,8 @@ class DeviceSession
     };
     struct GroupPlan {
         std::vector<std::vector<Table>> chunks;  // [chunk][vrank]
+        std::vector<std::shared_ptr<void>> mem;  // device memory of the tables
+        bool captured = false;    // a graph may hold its tables: kept as long as the session
     };
 
     void launch_ar(AllReduceCall &c, void *stream);
@@ -124,7 +126,7 @@ class DeviceSession
                            const std::vector<std::vector<void *>> &dsts, int blocks_n,
                            size_t stride, void *stream);
     const GroupPlan &plan_group(size_t n, const void *const *ins, void *const *outs,
-                                const size_t *counts, int dt, int user_dt);
+                                const size_t *counts, int dt, int user_dt, bool in_capture);
 
     // Every public call holds this from its first look at the session's state
     // to its last launch: calls from several threads of one rank are serialised
@@ -156,7 +158,6 @@ class DeviceSession
     // Returns false when the set has to be staged (decided alike on every rank).
     bool group_registered(size_t n, const void *const *ins, void *const *outs,
                           const size_t *counts, int dt, int op, double scale, void *stream);
-    std::vector<void *> table_mem_;
     unsigned long long launches_ = 0;
     // One signal pad serves the whole session, so its collectives must run on
     // the GPU one after the other, in the order issued.  On one stream that is

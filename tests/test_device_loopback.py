@@ -862,6 +862,28 @@ def test_cuda_graph_capture_and_replay():
             assert torch.all(sym == (4.0 + it) / 2) and torch.all(user == 2.0 * (1.0 + it))
 
 
+def test_captured_group_outlives_the_plans_of_other_sets():
+    """A graph reads its set's descriptor table at every replay; however many other sets
+    follow, the bounded cache of plans must not free it."""
+    with DeviceSession.loopback(1, heap_bytes=1 << 20, staging_bytes=1 << 20) as s:
+        tensors = [torch.zeros(k, device="cuda") for k in (1000, 3, 70_001)]
+        s.group_all_reduce(tensors, scale=2.0)  # its table is made outside the capture
+        torch.cuda.synchronize()
+        g, cap = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(g, stream=cap):
+            s.group_all_reduce(tensors, scale=2.0, stream=cap)
+        others = [[torch.ones(17 + k, device="cuda"), torch.ones(5, device="cuda")] for k in range(200)]
+        for o in others:
+            s.group_all_reduce(o, scale=3.0)
+        for t in tensors:
+            t.fill_(1.5)
+        g.replay()
+        torch.cuda.synchronize()
+        s.check()
+        assert all(bool((t == 3.0).all()) for o in others for t in o)
+        assert all(bool((t == 3.0).all()) for t in tensors)
+
+
 @pytest.mark.parametrize("world", [2, 4])
 def test_large_staged_messages_are_pipelined_on_three_streams(world, monkeypatch):
     """Above a size threshold staged calls run pack / reduce / unpack of successive
