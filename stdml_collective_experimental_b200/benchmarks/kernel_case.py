@@ -76,7 +76,8 @@ def other_collective(args, sess, dtype, es, n):
     times = [e[i].elapsed_time(e[i + 1]) for i in range(args.iters)]
     best = min(times[1:]) if len(times) > 1 else times[0]
     nbytes = n * es
-    # all_gather: pack (r+w) per rank, then every rank reads w blocks and writes w blocks
+    # push: pack (r+w) per rank, then every rank reads w blocks and writes w blocks (by pull
+    # most of this stays in the L2: a block is read once and written once per rank)
     hbm = {"all_gather": w * nbytes * (2 + 2 * w), "broadcast": nbytes * (2 + 2 * w),
            "barrier": 0}[args.collective]
     print(json.dumps({"collective": args.collective, "world": w, "mb_per_rank": args.mb,
@@ -102,6 +103,9 @@ def main():
                     help="with --staged-group: register the tensors instead of staging them")
     ap.add_argument("--bulk-min-bytes", type=int, default=None,
                     help="with --registered: the group_bulk_min_bytes knob (-1: peer loads only)")
+    ap.add_argument("--knob", action="append", default=[], metavar="NAME=VALUE",
+                    help="a knob of the session, e.g. gather_push_min_bytes=0 (the push form of "
+                         "all_gather, which a loopback session does not choose by itself)")
     args = ap.parse_args()
     dtype = {"f32": torch.float32, "bf16": torch.bfloat16}[args.dtype]
     es = 4 if args.dtype == "f32" else 2
@@ -110,6 +114,9 @@ def main():
                                   staging_bytes=(args.mb + 1) << 20
                                   if (args.staged_group or args.collective != "all_reduce")
                                   else 1 << 20)
+    for knob in args.knob:
+        name, value = knob.split("=")
+        sess.set_knob(name, int(value))
     if args.blocks:
         sess.set_tuning(max_blocks=args.blocks)
     if args.staged_group > 0:

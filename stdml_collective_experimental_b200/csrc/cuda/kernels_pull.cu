@@ -16,9 +16,10 @@
 // data by that much (two aligned loads and a funnel shift per vector), so that
 // the world - 1 copies of each tile are aligned 16-byte accesses; only the vectors
 // at a block's ends are moved byte by byte.
-// Measured, us: all_gather of 8 x 2.47 MB (an odd size) 518 -> 65, broadcast of 94 MB
-// to 3 others 345 -> 117.  By vectors per thread and round over all sources, four in
-// flight: 8: 68 / 128, 16: 65 / 117, 32: 76 / 117; eight in flight at 80 registers: 73 / 139.
+// Measured, us: all_gather of 8 x 2.47 MB (an odd size) 518 -> 58, broadcast of 94 MB
+// to 3 others 345 -> 111 (108 by the second kernel).  By vectors per thread and round over all
+// sources, four in flight, when 16 took 65 / 117: 8: 68 / 128, 32: 76 / 117; eight in flight at 80
+// registers: 73 / 139.
 //
 // The reference's counterparts are its full-mesh exchange
 // (src/stdml/collective/all_gather.cpp:16-56 there) and its broadcast walk
@@ -175,8 +176,7 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
 // and tile k packed side by side; arrive; wait for the others.  (An arrival then also says that
 // tile k-1 has been read.)  Vectors at a block's ends are stored byte by byte; a
 // destination that is not 16-byte aligned is written by the packing warps.
-// Against the kernel above, us: all_gather of 8 x 2.47 MB 65 -> 58, 8 x 8 MB 177 -> 162,
-// 4 x 8 MB 54 -> 49; broadcast of 94 MB to 3 117 -> 113, 16 MB to 7 56 -> 51.
+// launch_pull says which messages it is for.
 constexpr int kPullBufs = 5;  // of kPullBufVec vectors: four blocks of an SM fit
 constexpr unsigned int kPullBufVec = 512;
 constexpr int kPullLongThreads = kPullThreads + 32;
@@ -245,7 +245,7 @@ __global__ void __launch_bounds__(kPullLongThreads, kPullPerSm)
     for (int k = 0; k <= a.rounds; ++k) {
         bool ok = true;
         // broadcast: root's pack is what the others wait for, from an eighth or so of the
-        // grid (120 us without, 113 with it; all_gather, where every rank packs, 58 and 61)
+        // grid (94 MB to 3 others: 116 us without, 108 with it); in an all_gather every rank packs
         if (is_sync_thread() && bcast && packs && k + 1 < a.rounds) {
             src.prefetch(walk.first_vector(k + 1), tile);
         }
@@ -395,9 +395,15 @@ int launch_pull(const CommCtx &ctx, const PullArgs &a, int blocks, int vranks, v
 {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid(blocks, vranks, 1);
-    // one or two rounds are a matter of latency, to which the way through shared memory adds
-    // (with two ranks the registers keep up: 96 MB broadcast 68 us, 74 the other way)
-    const bool lng = a.rounds > 2 && ctx.world > 2;
+    // One or two rounds are a matter of latency, to which the way through shared memory adds.
+    // From three on, us, pull_kernel / pull_long_kernel, tensors not in the L2: broadcast of
+    // 100 MB to 3 121 / 117, 34 MB to 5 70 / 66, 100 MB to 7 228 / 216, 17 MB to 7 49 / 48.
+    // all_gather, in which every rank copies and packs the whole time: 3 x 34 MB 110 / 103,
+    // 4 x 17 MB 78 / 83, 4 x 100 MB 442 / 437, 8 x 2.47 MB 58 both, 8 x 8 MB 150 / 160.
+    // Two ranks: the registers keep up (broadcast 100 MB 70 / 74, all_gather 34 MB 57 both).
+    // (Destinations off a vector boundary do better in pull_kernel throughout, 34 MB to 3: 293 / 325,
+    // but a rank does not know the others', and all have to run the same kernel.)
+    const bool lng = a.rounds > 2 && ctx.world > 2 && (a.root >= 0 || ctx.world == 3);
     const void *kernel = lng ? reinterpret_cast<const void *>(&pull_long_kernel)
                              : reinterpret_cast<const void *>(&pull_kernel);
     const dim3 block(lng ? kPullLongThreads : kPullThreads);

@@ -729,8 +729,9 @@ def test_tiles_drawn_by_ticket(job, algo):
 
 @pytest.mark.parametrize("shift", [0, 5])
 def test_pull_at_the_slots_of_a_job(job, shift):
-    """all_gather and broadcast of three rounds, tiles of several steps (from three ranks up
-    the kernel of long messages), from and to addresses `shift` bytes off a vector boundary."""
+    """all_gather and broadcast of three rounds, tiles of several steps (by the kernel of long
+    messages: broadcast from three ranks up, all_gather among three), from and to addresses
+    `shift` bytes off a vector boundary."""
     w = job.world
     for op, n in (("all_gather", {2: 20_000_003, 3: 14_000_001, 4: 7_000_001, 8: 2_000_003}[w]),
                   ("broadcast", {2: 20_000_003, 3: 27_000_005, 4: 20_000_003, 8: 11_000_001}[w])):
