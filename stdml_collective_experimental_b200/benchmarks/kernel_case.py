@@ -40,9 +40,9 @@ def staged_group(args, sess, dtype, es):
     sess.check()
     times = [e[i].elapsed_time(e[i + 1]) for i in range(args.iters)]
     nbytes = sum(sizes) * es
-    # per rank: pack (read + write), reduce (read world, write world, amortised: read + write), unpack (read + write);
-    # registered: the reduce alone
-    hbm = (2 if args.registered else 6) * args.world * nbytes
+    # what has to move: every tensor is read once and written once (the staging ring stays
+    # mostly in the L2)
+    hbm = 2 * args.world * nbytes
     best = min(times[1:]) if len(times) > 1 else times[0]
     want = sum(range(1, args.world + 1)) / args.world
     assert args.iters > 1 or all(abs(float(t[-1]) - want) < 1e-3 for t in ranks[0]), "wrong result"
@@ -76,9 +76,8 @@ def other_collective(args, sess, dtype, es, n):
     times = [e[i].elapsed_time(e[i + 1]) for i in range(args.iters)]
     best = min(times[1:]) if len(times) > 1 else times[0]
     nbytes = n * es
-    # push: pack (r+w) per rank, then every rank reads w blocks and writes w blocks (by pull
-    # most of this stays in the L2: a block is read once and written once per rank)
-    hbm = {"all_gather": w * nbytes * (2 + 2 * w), "broadcast": nbytes * (2 + 2 * w),
+    # what has to move: every block is read once and written once per rank
+    hbm = {"all_gather": w * nbytes * (1 + w), "broadcast": nbytes * (1 + w),
            "barrier": 0}[args.collective]
     print(json.dumps({"collective": args.collective, "world": w, "mb_per_rank": args.mb,
                       "ms_per_launch": times, "best_ms": best, "hbm_bytes_per_launch": hbm,

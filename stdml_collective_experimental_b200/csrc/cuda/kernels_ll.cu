@@ -6,8 +6,8 @@
 // memory or to a peer; with the flag inside every 8-byte word the data is its own
 // signal, and the chain is one store and one poll.  The price is twice the bytes, so
 // this is for messages whose time is the chain (see ll_limit in algo_table.hpp).
-// Three f32 elements, 8 ranks on one GPU: 6.8 us per call with a barrier, 4.1 us so (kernel
-// 6.2 / 3.6); 16 KB in the heap, 2 ranks: 8.2 us per call in place, 4.4 us so.
+// Three f32 elements, 8 ranks on one GPU: 6.8 us per call with a barrier, 4.1 us so;
+// 16 KB in the heap, 2 ranks: 8.2 us per call in place, 4.4 us so.
 //
 // One vector per thread.  The flag is the block's epoch + 1, so a word from an earlier
 // call never passes for this one's, and the two mailboxes of a block alternate with the
