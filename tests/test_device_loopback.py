@@ -863,6 +863,74 @@ def test_cuda_graph_capture_and_replay():
             assert torch.all(sym == (4.0 + it) / 2) and torch.all(user == 2.0 * (1.0 + it))
 
 
+@pytest.mark.parametrize("staging", [4096, 20_000, 300_000])
+@pytest.mark.parametrize("world", [3, 8, 16])
+def test_slots_too_small_for_a_ring(world, staging):
+    """Every staged collective with slots of a few KB: too small for any ring, for the ring of
+    several blocks, for a whole message."""
+    with DeviceSession.loopback(world, heap_bytes=1 << 20, staging_bytes=staging) as s:
+        for n in (1, 1000, 300_007):
+            host = make_inputs(world, n, torch.int32, seed=n)
+            want = reduce_many(host, "sum")
+            ins = [h.cuda() for h in host]
+            out, bc, red = ([torch.zeros_like(t) for t in ins] for _ in range(3))
+            ag = [torch.zeros(n * world, dtype=torch.int32, device="cuda") for _ in ins]
+            group = [list(torch.split(t.clone(), n // 7 + 1)) for t in ins]
+            s.all_reduce(ins, out=out)
+            s.all_gather(ins, ag)
+            s.broadcast(ins, out=bc, root=world - 1)
+            s.reduce(ins, out=red, root=1)
+            s.group_all_reduce(group)
+            torch.cuda.synchronize()
+            s.check()
+            assert torch.equal(red[1].cpu(), want), n
+            for r in range(world):
+                assert torch.equal(out[r].cpu(), want), (n, r)
+                assert torch.equal(ag[r].cpu(), torch.cat(host)), (n, r)
+                assert torch.equal(bc[r].cpu(), host[world - 1]), (n, r)
+                assert torch.equal(torch.cat(group[r]).cpu(), want), (n, r)
+
+
+@pytest.mark.parametrize("n", [3, 70_001, 2_000_003])
+def test_staged_collectives_of_several_ranks_in_a_graph(n):
+    """Mailboxes, staged rounds and the pull rings replayed from a graph, between ordinary
+    calls that use the same slots and mailboxes."""
+    w = 4
+    with DeviceSession.loopback(w, heap_bytes=1 << 20, staging_bytes=1 << 20) as s:
+        ins, out, bc = ([torch.zeros(n, device="cuda") for _ in range(w)] for _ in range(3))
+        ag = [torch.zeros(n * w, device="cuda") for _ in range(w)]
+        group = [list(torch.split(torch.zeros(n, device="cuda"), n // 3 + 1)) for _ in range(w)]
+
+        def calls(stream=None):
+            s.all_reduce(ins, out=out, stream=stream)
+            s.all_gather(ins, ag, stream=stream)
+            s.broadcast(ins, out=bc, root=2, stream=stream)
+            s.group_all_reduce(group, stream=stream)
+
+        calls()  # the group's table is made outside the capture
+        torch.cuda.synchronize()
+        g, cap = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(g, stream=cap):
+            calls(cap)
+        for it in range(3):
+            for r in range(w):
+                ins[r].fill_(r + it)
+                for t in group[r]:
+                    t.fill_(r + it)
+            g.replay()
+            torch.cuda.synchronize()
+            s.check()
+            total = float(sum(r + it for r in range(w)))
+            for r in range(w):
+                assert bool((out[r] == total).all()) and bool((bc[r] == 2.0 + it).all()), (it, r)
+                assert torch.equal(ag[r], torch.cat(ins)), (it, r)
+                assert all(bool((t == total).all()) for t in group[r]), (it, r)
+            s.all_reduce(ins, out=out)
+            s.broadcast(ins, out=bc)
+        torch.cuda.synchronize()
+        s.check()
+
+
 def test_captured_group_outlives_the_plans_of_other_sets():
     """A graph reads its set's descriptor table at every replay; however many other sets
     follow, the bounded cache of plans must not free it."""
