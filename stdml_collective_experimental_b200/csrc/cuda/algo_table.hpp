@@ -68,7 +68,8 @@ inline size_t ll_capacity(int world, int vranks, int num_sms)
 //   10: 4 KB 9.4 / 8.2, 6 KB 8.7 / 10.3; 16: 3 KB 10.3 / 8.2, 6 KB 10.3 / 12.3.
 // Out of place, against a one-shot and its one barrier:
 //   2 ranks: 512 KB 7.2 / 6.2; 3: 400 KB 8.2 / 6.9; 4: 262 KB 8.2 / 6.9, 307 KB 8.2 both, 400 KB 8.2 / 9.5;
-//   6: 4 KB 6.2 both, 115 KB 8.2 both; 8: 12 B 6.8 / 4.1, 4 KB 6.2-7.6 / 6.3, 6 KB 7.3 / 8.2;
+//   5: 8 KB 8.2 / 7.1, 147 KB 8.2 both; 6: 6 KB 6.6 / 6.5, 8 KB and 115 KB 8.2 both;
+//   7: 4 KB 7.6 / 6.2, 6 KB 7.2 / 8.2; 8: 12 B 6.8 / 4.1, 4 KB 6.2-7.6 / 6.3, 6 KB 7.3 / 8.2;
 //   12: 2 KB 8.2 / 6.5, 6 KB 8.2 / 10.3; 16: 1.5 KB 8.2 / 6.2, 4 KB 8.2 / 10.3.
 inline size_t ll_limit(int world, int vranks, size_t capacity, bool in_place_symmetric)
 {
@@ -79,7 +80,8 @@ inline size_t ll_limit(int world, int vranks, size_t capacity, bool in_place_sym
     if (in_place_symmetric) {
         return world <= 4 ? capacity : over_all_ranks(world < 8 ? 1024 : 48);
     }
-    return world <= 4 ? std::min(capacity, size_t{256u << 10} / 16) : over_all_ranks(32);
+    if (world <= 6) { return std::min(capacity, size_t{world <= 4 ? 256u << 10 : 8u << 10} / 16); }
+    return over_all_ranks(32);
 }
 
 // need_owner: the result must stay in the symmetric buffer (in place), which
