@@ -244,7 +244,7 @@ struct StagedArgs {
 // All-reduce in one exchange through the mailboxes of the arena (kernels_ll.cu).
 struct LlArgs {
     const void *src[kMaxRanks];  // per virtual rank
-    void *dst[kMaxRanks];        // nullptr: the rank stores nothing
+    void *dst[kMaxRanks];
     unsigned long long off;    // arena offset of the mailboxes
     unsigned int capacity;     // vectors of one mailbox
     unsigned int nvec;

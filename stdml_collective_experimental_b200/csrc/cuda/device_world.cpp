@@ -929,7 +929,10 @@ class World final : public DeviceWorld
         for (int v = 0; v < vranks_; ++v) {
             if (in[v] == nullptr) { return false; }
             a.src[v] = in[v];
-            a.dst[v] = out[v];
+            // A rank without a destination stores into its mailbox for its own data, which
+            // nobody writes or reads (a look at the pointer in the kernel cost 0.02-0.3 us).
+            const int r = rank() + v;
+            a.dst[v] = out[v] != nullptr ? out[v] : base_[r] + layout_.mail_off() + r * ll_capacity_ * 32;
         }
         a.off = layout_.mail_off();
         a.capacity = static_cast<unsigned int>(ll_capacity_);

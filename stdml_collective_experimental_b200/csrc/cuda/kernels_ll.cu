@@ -62,8 +62,6 @@ __global__ void __launch_bounds__(kThreads, 2)
     SignalPad *pad = pad_of(ctx, rank);
     const unsigned int v = blockIdx.x * kThreads + threadIdx.x;
     const bool mine = v < a.nvec;
-    void *const dst = a.dst[vr];
-    const unsigned long long count = dst != nullptr ? a.count : 0ull;  // elements to store
     const uint32_t epoch = ld_relaxed_sys_u32(&pad->epoch[blockIdx.x]);
     uint4 own = make_uint4(0, 0, 0, 0);
     if (mine) { own = load_user_vec<DT>(a.src[vr], false, v, a.count, ptr_aligned16(a.src[vr])); }
@@ -129,7 +127,7 @@ __global__ void __launch_bounds__(kThreads, 2)
             }
         }
         if (ok) {
-            store_user_vec<DT>(dst, false, v, count, ptr_aligned16(dst),
+            store_user_vec<DT>(a.dst[vr], false, v, a.count, ptr_aligned16(a.dst[vr]),
                                acc.finish(a.scale, a.has_scale != 0));
         }
     }
