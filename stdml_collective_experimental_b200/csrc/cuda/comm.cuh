@@ -125,15 +125,30 @@ inline void tma_geometry(int world, unsigned int want_tile_vec, int *stages,
     *smem_bytes = st * static_cast<unsigned int>(world) * tv * 16u;
 }
 
-// The staged all-reduce (staged_kernel.cuh): pieces of its ring per block, and
-// vectors that a block packs, reduces and unpacks per round over all shards.
-constexpr int kStagedRing = 3;
-constexpr int kStagedThreads = 256;
-constexpr int kStagedPerSm = 4;
-constexpr int kStagedStepShift = 8;  // smallest tile: one vector per thread
-static_assert(1 << kStagedStepShift == kStagedThreads, "a step is one vector per thread");
+// The staged all-reduce (staged_kernel.cuh): workers and threads of a block, blocks per SM.
+constexpr int kStagedThreads = 192;
+constexpr int kStagedBlock = kStagedThreads + 96;  // and a warp each that loads, tells, fetches
+constexpr int kStagedMinPerSm = 3;  // that the registers allow
+constexpr int kStagedLag = 3;       // passes from a tile's pack to its reduce, and on to its unpack
+constexpr int kStagedRing = 2 * kStagedLag + 1;  // pieces of a block's ring, per shard
+constexpr int kStagedMinShift = 5;  // smallest tile: one vector per lane of a warp
 constexpr int kStagedStarts = 1024;  // table entries searched in shared memory
-constexpr unsigned int kStagedRoundVec = 2048;
+constexpr unsigned int kStagedRoundVec = 1024;
+constexpr size_t kStagedSmem = 100u << 10;  // of dynamic shared memory, at most
+constexpr size_t kStagedOtherSmem = 11u << 10;  // of a block beside it, at most
+
+// Bytes of the tile buffers of a block (StagedBuffers in staged_kernel.cuh).
+STDML_HD constexpr size_t staged_smem(int world, int tile_shift, bool user_f32)
+{
+    return static_cast<size_t>((world + 1) * (user_f32 ? 32 : 16) + 3 * (world - 1) * 16) << tile_shift;
+}
+
+// Blocks of which an SM holds so many at once.
+STDML_HD constexpr int staged_per_sm(int world, int tile_shift, bool user_f32)
+{
+    const size_t fit = (size_t{228} << 10) / (staged_smem(world, tile_shift, user_f32) + kStagedOtherSmem);
+    return fit < kStagedMinPerSm ? static_cast<int>(fit) : kStagedMinPerSm;
+}
 
 // all_gather / broadcast by pull (kernels_pull.cu)
 constexpr int kPullRing = 4;

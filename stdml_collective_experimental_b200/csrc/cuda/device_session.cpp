@@ -391,6 +391,10 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
         run_pipelined(calls, stream);
         return;
     }
+    // the staged kernel goes round in a slot: one launch, whatever the length
+    const bool ring = total_bytes > slot_elems * es &&
+                      world_->staged_any_length(count, dt, op, algo, false);
+    if (ring) { slot_elems = count; }
     std::vector<const void *> src(vr);
     std::vector<void *> dst(vr);
     for (size_t done = 0; done < count; done += slot_elems) {
@@ -406,6 +410,7 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
         k.count = n;
         k.end_barrier = in_capture;
         k.staged = true;
+        k.ring = ring;
         launch_ar(k, stream);
     }
 }
@@ -606,16 +611,17 @@ std::vector<std::vector<GroupPiece>> plan_group_pieces(size_t n, const size_t *c
 const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *const *ins,
                                                           void *const *outs,
                                                           const size_t *counts, int dt,
-                                                          int user_dt, bool in_capture)
+                                                          int user_dt, size_t cap, bool in_capture)
 {
     const int vr = world_->vranks();
     std::string key;
-    key.reserve((2 * vr * n + n + 2) * sizeof(void *));
+    key.reserve((2 * vr * n + n + 3) * sizeof(void *));
     key.append(reinterpret_cast<const char *>(ins), sizeof(void *) * n * vr);
     key.append(reinterpret_cast<const char *>(outs), sizeof(void *) * n * vr);
     key.append(reinterpret_cast<const char *>(counts), sizeof(size_t) * n);
     key.append(reinterpret_cast<const char *>(&dt), sizeof(dt));
     key.append(reinterpret_cast<const char *>(&user_dt), sizeof(user_dt));
+    key.append(reinterpret_cast<const char *>(&cap), sizeof(cap));
     auto it = plans_.find(key);
     if (it != plans_.end()) {
         it->second.captured = it->second.captured || in_capture;
@@ -629,10 +635,6 @@ const DeviceSession::GroupPlan &DeviceSession::plan_group(size_t n, const void *
     const size_t es = elem_size(dt);                          // wire element
     const size_t ues = user_dt >= 0 ? elem_size(user_dt) : es;  // user element
     const size_t lanes = 16 / es;
-    // One chunk per staging slot.  (Cutting a pipelined set finer, 1/8 of it per
-    // chunk, was measured slower at 8 GPUs: 605 against 671 GB/s on 438 MB.)
-    const size_t cap = world_->staging_bytes() / 16;  // vectors per slot
-
     using Piece = GroupPiece;
     const std::vector<std::vector<Piece>> chunks = plan_group_pieces(n, counts, lanes, cap);
 
@@ -855,11 +857,18 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
     }
 
     const bool in_capture = capturing(stream);
-    const GroupPlan &plan = plan_group(n, ins, outs, counts, dt, user_dt, in_capture);
-    size_t plan_bytes = 0;
-    for (const auto &chunk : plan.chunks) { plan_bytes += chunk[0].nvec * 16; }
-    if (world_->world() > 1 && plan.chunks.size() >= 2 && plan_bytes >= pipeline_min_bytes_ &&
-        !in_capture && (algo < 0 || is_owner_algo(algo))) {
+    size_t nvec = 0;
+    for (size_t i = 0; i < n; ++i) { nvec += (counts[i] + 16 / es - 1) / (16 / es); }
+    // One chunk per staging slot.  (Cutting a pipelined set finer, 1/8 of it per
+    // chunk, was measured slower at 8 GPUs: 605 against 671 GB/s on 438 MB.)
+    const size_t slot = world_->staging_bytes() / 16;  // vectors
+    const bool pipelined = world_->world() > 1 && nvec > slot && nvec * 16 >= pipeline_min_bytes_ &&
+                           !in_capture && (algo < 0 || is_owner_algo(algo));
+    // Or one chunk in all: the staged kernel goes round in a slot.
+    const bool ring = !pipelined && nvec > slot &&
+                      world_->staged_any_length(nvec * (16 / es), dt, op, algo, user_dt >= 0);
+    const GroupPlan &plan = plan_group(n, ins, outs, counts, dt, user_dt, ring ? nvec : slot, in_capture);
+    if (pipelined) {
         std::vector<std::vector<const GroupEntry *>> all_tabs;
         std::vector<AllReduceCall> calls;
         for (const auto &chunk : plan.chunks) {
@@ -896,6 +905,7 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
         c.algo = algo;
         c.end_barrier = in_capture;
         c.staged = true;
+        c.ring = ring;
         c.first_of_tile = chunk[0].first_of_tile;
         c.chained = &chunk != &plan.chunks.front() && !in_capture;
         launch_ar(c, stream);

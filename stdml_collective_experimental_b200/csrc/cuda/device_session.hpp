@@ -126,7 +126,8 @@ class DeviceSession
                            const std::vector<std::vector<void *>> &dsts, int blocks_n,
                            size_t stride, void *stream);
     const GroupPlan &plan_group(size_t n, const void *const *ins, void *const *outs,
-                                const size_t *counts, int dt, int user_dt, bool in_capture);
+                                const size_t *counts, int dt, int user_dt, size_t cap,
+                                bool in_capture);
 
     // Every public call holds this from its first look at the session's state
     // to its last launch: calls from several threads of one rank are serialised

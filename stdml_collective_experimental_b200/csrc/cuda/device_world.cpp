@@ -709,7 +709,7 @@ class World final : public DeviceWorld
         const size_t bytes = c.count * esize;
         const size_t nvec = (bytes + 15) / 16;
         const bool registered = c.peer_data != nullptr;
-        if (!registered && !layout_.holds(c.off, nvec * 16)) {
+        if (!registered && !c.ring && !layout_.holds(c.off, nvec * 16)) {
             throw std::invalid_argument("all_reduce: symmetric buffer outside its slot or heap");
         }
         if (registered) {
@@ -746,6 +746,11 @@ class World final : public DeviceWorld
             void *to = (c.dst != nullptr && c.dst[0] != nullptr) ? c.dst[0] : sym;
             return launch_local_scale(from, to, c.count, c.dt, c.scale, c.has_scale ? 1 : 0,
                                       stream);
+        }
+        if (c.ring) {
+            const int rc = all_reduce_staged(c, nvec, user_dt, stream);
+            if (rc < 0) { throw std::invalid_argument("all_reduce: the ring does not fit the staging slot"); }
+            return rc;
         }
         int algo = c.algo;
         if (algo < 0) { algo = pick_algo(bytes, c.dt, c.op, any_dst_null); }
@@ -877,6 +882,16 @@ class World final : public DeviceWorld
         return rc;
     }
 
+    bool staged_any_length(size_t count, int dt, int op, int algo, bool user_f32) const override
+    {
+        static const size_t sizes[12] = {1, 2, 4, 8, 1, 2, 4, 8, 2, 2, 4, 8};
+        if (dt < 0 || dt > DT_F64_) { return false; }
+        const size_t bytes = count * sizes[dt], nvec = (bytes + 15) / 16;
+        if (algo < 0) { algo = pick_algo(bytes, dt, op, false); }
+        return opt_.world > 1 && (algo == kAlgoTwoShot || algo == kAlgoTwoShotTma) &&
+               staged_geometry(opt_.world, nvec, opt_.staging_bytes, num_sms_, vranks_, 0, user_f32).full;
+    }
+
     // Peer-load two-shot of memory outside the arena: rounds over a small ring.
     int all_reduce_staged(const AllReduceCall &c, size_t nvec, int user_dt, void *stream)
     {
@@ -899,10 +914,8 @@ class World final : public DeviceWorld
         a.scale = c.scale;
         a.slot_bytes = opt_.staging_bytes;
         a.debug_checks = debug_checks_ ? 1 : 0;
-        // all resident (the kernel's launch bounds)
-        const int most = c.blocks > 0 ? c.blocks
-                                      : std::min(kMaxBlocks, std::max(1, kStagedPerSm * num_sms_ / vranks_));
-        const StagedGeometry g = staged_geometry(opt_.world, nvec, opt_.staging_bytes, most);
+        const StagedGeometry g = staged_geometry(opt_.world, nvec, opt_.staging_bytes, num_sms_, vranks_,
+                                                 c.blocks, user_dt != c.dt);
         if (g.blocks == 0) { return -1; }
         a.tile_shift = g.tile_shift;
         a.rounds = g.rounds;

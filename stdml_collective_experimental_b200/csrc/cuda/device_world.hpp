@@ -80,6 +80,8 @@ struct AllReduceCall {
     // `off` is a staging slot of which the call may make any use: nobody looks for
     // the packed operands or the result there afterwards.
     bool staged = false;
+    // ... and in which it keeps a ring only (staged_any_length() said so for the whole message).
+    bool ring = false;
     int phases = 7;  // kPhasePack | kPhaseReduce | kPhaseUnpack
 };
 
@@ -182,6 +184,9 @@ class DeviceWorld
     // pull through a ring in the slot: then one call of any length will do (GatherCall::ring).
     // Every rank gets the same answer: it depends on nothing that a rank passes of its own.
     virtual bool pulls_staged(size_t bytes, int root) const = 0;
+    // Whether a staged all_reduce of `count` elements in all goes by rounds over a ring in a
+    // staging slot, which takes messages of any length in one launch.  Alike on every rank.
+    virtual bool staged_any_length(size_t count, int dt, int op, int algo, bool user_f32) const = 0;
     // Two-shot all-reduce over a table of registered tensors (see PeerEntry).
     virtual int group_peer(const PeerEntry *table, int ntable, size_t nvec, int dt, int op,
                            double scale, void *stream) = 0;

@@ -49,14 +49,16 @@ struct StagedWalk {
 
 struct StagedGeometry {
     int blocks = 0;  // 0: the slot cannot hold the ring of even one block
-    int tile_shift = kStagedStepShift, rounds = 1;
+    int tile_shift = kStagedMinShift, rounds = 1;
+    bool full = false;  // the slot holds the rings of as many blocks as there may be
 };
 
-// Grid and tile for `nvec` vectors.  A tile is kStagedRoundVec vectors over all shards
-// of a round at most (the block's loads in flight), smaller where the message
-// would otherwise leave blocks without a tile, and never so large that the
-// rings of all blocks outgrow the staging slot.
-inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_bytes, int max_blocks)
+// Grid and tile for `nvec` vectors on `num_sms` SMs that `vranks` ranks share.  A tile is kStagedRoundVec
+// vectors over all shards of a round at most, smaller where its buffers would outgrow the shared
+// memory of a block or the rings of all blocks the staging slot, and where the message would
+// otherwise leave blocks without a tile.
+inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_bytes, int num_sms, int vranks,
+                                      int want_blocks, bool user_f32)
 {
     StagedGeometry g;
     size_t longest = 0;
@@ -64,18 +66,27 @@ inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_byt
         longest = std::max<size_t>(longest, StagedWalk::shard_begin(nvec, world, s + 1) -
                                                 StagedWalk::shard_begin(nvec, world, s));
     }
-    const size_t want = kStagedRoundVec / static_cast<size_t>(world);
-    const size_t most = static_cast<size_t>(max_blocks);
     const auto ring_bytes = [&](int shift) {
         return (static_cast<size_t>(kStagedRing) * world << shift) * 16;
     };
-    while ((size_t{2} << g.tile_shift) <= want && (size_t{2} << g.tile_shift) * most <= longest &&
-           ring_bytes(g.tile_shift + 1) * most <= staging_bytes) {
-        ++g.tile_shift;
-    }
+    // blocks per rank that are resident together
+    const auto most = [&](int shift) {
+        const int resident = std::min(kMaxBlocks, staged_per_sm(world, shift, user_f32) * num_sms / vranks);
+        return static_cast<size_t>(std::max(1, want_blocks > 0 ? std::min(want_blocks, resident) : resident));
+    };
+    const size_t want = std::max<size_t>(kStagedRoundVec / static_cast<size_t>(world), size_t{1} << kStagedMinShift);
+    const auto good = [&](int shift) {
+        const size_t tile = size_t{1} << shift;
+        if (tile > want || staged_smem(world, shift, user_f32) > kStagedSmem) { return false; }
+        // (a short message has fewer blocks, not smaller tiles than this)
+        if (tile <= 256) { return ring_bytes(shift) <= staging_bytes; }
+        return tile * most(shift) <= longest && ring_bytes(shift) * most(shift) <= staging_bytes;
+    };
+    while (good(g.tile_shift + 1)) { ++g.tile_shift; }
     const size_t tiles = (longest + (size_t{1} << g.tile_shift) - 1) >> g.tile_shift;
     const size_t fit = staging_bytes / ring_bytes(g.tile_shift);
-    g.blocks = static_cast<int>(std::min<size_t>({tiles, most, fit}));
+    g.blocks = static_cast<int>(std::min<size_t>({tiles, most(g.tile_shift), fit}));
+    g.full = fit >= most(g.tile_shift);
     if (g.blocks > 0) { g.rounds = static_cast<int>((tiles + g.blocks - 1) / g.blocks); }
     return g;
 }

@@ -61,15 +61,20 @@ int main()
         const unsigned long long nvec = 1 + rng() % (trial % 3 == 0 ? 70 : 3000000);
         const int world = 2 + static_cast<int>(rng() % 15);
         const size_t slot = (size_t{4096} << (rng() % 15)) + 4096;
-        const int most = 1 + static_cast<int>(rng() % 300);
-        const StagedGeometry g = staged_geometry(world, nvec, slot, most);
-        EXPECT(g.blocks <= most && g.tile_shift >= kStagedStepShift);
-        if (g.blocks == 0) {
-            EXPECT(slot < ((static_cast<size_t>(kStagedRing) * world) << kStagedStepShift) * 16);
-            continue;
-        }
+        const bool user_f32 = trial % 2 == 0;
+        const int sms = 1 + static_cast<int>(rng() % 148), rows = trial % 5 < 3 ? world : 1;
+        const int want = trial % 7 == 0 ? 1 + static_cast<int>(rng() % 300) : 0;
+        const StagedGeometry g = staged_geometry(world, nvec, slot, sms, rows, want, user_f32);
+        const int per_sm = staged_per_sm(world, g.tile_shift, user_f32);
+        EXPECT(per_sm >= 1 && (staged_smem(world, g.tile_shift, user_f32) + kStagedOtherSmem) * per_sm <= 228u << 10);
+        EXPECT((g.blocks - 1) * rows < per_sm * sms && (want == 0 || g.blocks <= want) && g.tile_shift >= kStagedMinShift);
         const unsigned long long ring =
             ((static_cast<unsigned long long>(kStagedRing) * world) << g.tile_shift) * 16;
+        EXPECT(staged_smem(world, g.tile_shift, user_f32) <= kStagedSmem);
+        if (g.blocks == 0) {
+            EXPECT(slot < ring);
+            continue;
+        }
         EXPECT(ring * g.blocks <= slot);
         std::vector<unsigned long long> bound(world + 1);
         for (int s = 0; s <= world; ++s) { bound[s] = StagedWalk::shard_begin(nvec, world, s); }

@@ -669,6 +669,37 @@ def test_staged_group_at_the_slots_of_a_job(job, dtype, wire):
         assert same(torch.cat(dev[r]).cpu(), want), r
 
 
+@pytest.mark.parametrize("world,dtype,wire,slot,n", [
+    (3, torch.float32, None, 32, 9_500_003), (8, torch.bfloat16, None, 16, 9_000_001),
+    (2, torch.float32, torch.bfloat16, 32, 17_000_005), (16, torch.int32, None, 16, 4_400_001)])
+def test_staged_message_of_several_slots_is_one_launch(world, dtype, wire, slot, n):
+    """The ring of a full grid fits the slot, so the message may be longer than it."""
+    host = make_inputs(world, n, dtype, seed=12)
+    sizes = [n // 2, 5, n // 3 + 1, n - n // 2 - n // 3 - 6]
+    want = reduce_many([h.to(wire or dtype) for h in host], "sum").to(dtype)
+    with DeviceSession.loopback(world, heap_bytes=1 << 20, staging_bytes=slot << 20) as s:
+        for shift in (0, 1):
+            flat = [torch.empty(n + 1, dtype=dtype, device="cuda")[shift:n + shift] for _ in host]
+            for f, h in zip(flat, host):
+                f.copy_(h)
+            dev = [list(torch.split(f, sizes)) for f in flat]
+            before = s.launches
+            s.group_all_reduce(dev, wire_dtype=wire)
+            assert s.launches == before + 1
+            torch.cuda.synchronize()
+            s.check()
+            for r in range(world):
+                assert same(flat[r].cpu(), want), (shift, r)
+            if shift == 0 and wire is None:
+                for f, h in zip(flat, host):
+                    f.copy_(h)
+                s.all_reduce(flat)
+                torch.cuda.synchronize()
+                s.check()
+                assert s.launches == before + 2
+                assert all(same(f.cpu(), want) for f in flat)
+
+
 def test_staged_buffer_at_the_slots_of_a_job(job):
     n = 5_300_003
     host = make_inputs(job.world, n, torch.int32, seed=8)
