@@ -157,6 +157,27 @@ constexpr int kPullPerSm = 4;
 constexpr int kPullStepShift = 8;  // smallest tile: one vector per thread
 constexpr int kPullVec = 16;            // vectors per thread and round over all sources
 static_assert(1 << kPullStepShift == kPullThreads, "a step is one vector per thread");
+// ... of several rounds: workers and threads of a block, blocks per SM, rounds from pack to copy
+constexpr int kPullLongThreads = 192;
+constexpr int kPullLongBlock = kPullLongThreads + 128;  // and a warp each that loads, tells, fetches, stores
+constexpr int kPullLongPerSm = 2;
+constexpr int kPullLongSources = 7;
+constexpr size_t kPullLongMin = 512;  // vectors per block, at least
+constexpr int kPullLag = 6;
+constexpr int kPullDepth = 2;  // rounds of ring pieces in shared memory
+constexpr int kPullLongRing = 2 * kPullLag + 1;
+constexpr size_t kPullLongSmem = 100u << 10;  // of dynamic shared memory: kPullLongPerSm blocks fit an SM
+STDML_HD constexpr int pull_sources(int world, int root) { return root >= 0 ? 1 : world - 1; }
+// Bytes of a block's tile buffers: two rounds of the tensor, kPullDepth of every source's ring piece.
+STDML_HD constexpr size_t pull_long_smem(int sources, unsigned int tile)
+{
+    return (2 * (static_cast<size_t>(tile) + 1) + kPullDepth * static_cast<size_t>(sources) * tile) * 16;
+}
+// Vectors of the largest tile, of which the buffers fit.
+STDML_HD constexpr unsigned int pull_long_tile(int sources)
+{
+    return static_cast<unsigned int>((kPullLongSmem / 16 - 2) / (2 + kPullDepth * sources)) / 32u * 32u;
+}
 
 // One tensor of a fused group: `count` elements that live at vector offset
 // `voff` (16-byte units) of the flat symmetric region.
@@ -300,6 +321,8 @@ struct PullArgs {
     int root;                    // < 0: all_gather; >= 0: broadcast
     int end_barrier;             // as in GatherArgs
     int tile_shift, rounds;      // from pull_geometry()
+    unsigned int tile;           // pull_long_kernel: instead of tile_shift
+    int lng;                     // pull_long_kernel
 };
 
 enum : int {

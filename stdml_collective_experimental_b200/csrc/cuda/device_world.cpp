@@ -1,6 +1,7 @@
 #include "device_world.hpp"
 
 #include <algorithm>
+#include <bit>
 #include <chrono>
 #include <cstdlib>
 #include <cstring>
@@ -979,11 +980,7 @@ class World final : public DeviceWorld
 
     PullGeometry geometry_of_pull(size_t bytes, int root, int want_blocks) const
     {
-        // all resident (the kernel's launch bounds)
-        const int most = want_blocks > 0
-                             ? want_blocks
-                             : std::min(kMaxBlocks, std::max(1, kPullPerSm * num_sms_ / vranks_));
-        return pull_geometry(root >= 0 ? 1 : opt_.world - 1, bytes, opt_.staging_bytes, most);
+        return pull_geometry(pull_sources(opt_.world, root), bytes, opt_.staging_bytes, num_sms_, vranks_, want_blocks);
     }
 
     bool pulls_staged(size_t bytes, int root) const override
@@ -1008,8 +1005,10 @@ class World final : public DeviceWorld
         a.stride = g.stride;
         a.root = g.root;
         a.end_barrier = g.end_barrier;
-        a.tile_shift = geo.tile_shift;
+        a.tile = geo.tile;
+        a.tile_shift = std::bit_width(geo.tile) - 1;
         a.rounds = geo.rounds;
+        a.lng = geo.lng ? 1 : 0;
         return launch_pull(make_ctx(), a, geo.blocks, vranks_, stream);
     }
 

@@ -16,17 +16,20 @@
 // data by that much (two aligned loads and a funnel shift per vector), so that
 // the world - 1 copies of each tile are aligned 16-byte accesses; only the vectors
 // at a block's ends are moved byte by byte.
-// Measured, us: all_gather of 8 x 2.47 MB (an odd size) 518 -> 58, broadcast of 94 MB
-// to 3 others 345 -> 111 (108 by the second kernel).  By vectors per thread and round over all
+// Measured against a slot-sized region, us: all_gather of 8 x 2.47 MB (an odd size) 518 -> 58, broadcast of 94 MB
+// to 3 others 345 -> 111 (both have gone to the second kernel since).  By vectors per thread and round over all
 // sources, four in flight, when 16 took 65 / 117: 8: 68 / 128, 32: 76 / 117; eight in flight at 80
 // registers: 73 / 139.
 //
 // The reference's counterparts are its full-mesh exchange
 // (src/stdml/collective/all_gather.cpp:16-56 there) and its broadcast walk
 // (src/stdml/collective/session.cpp:49-62 there).
+#include <atomic>
+
 #include "ar_kernel.cuh"
 #include "copy.cuh"
 #include "pull_walk.hpp"
+#include "ring_sync.cuh"
 
 namespace stdml::collective::cuda
 {
@@ -39,9 +42,28 @@ struct PullBlock {
     // all vectors of [v, v + kPullThreads) can be stored whole
     __device__ __forceinline__ bool inside(unsigned long long v) const
     {
-        return aligned && v >= 1 && v + kPullThreads < nvec;
+        return whole(v, kPullThreads);
+    }
+    // so can all of [v, v + n)
+    __device__ __forceinline__ bool whole(unsigned long long v, unsigned int n) const
+    {
+        return aligned && v >= 1 && v + n < nvec;
     }
 };
+
+// Where the data of source p goes (broadcast: the same place for every p).
+__device__ __forceinline__ PullBlock pull_block(const PullArgs &a, const PullLayout &walk, int vr, int p)
+{
+    const bool bcast = a.root >= 0;
+    PullBlock d;
+    d.phase = bcast ? 0u : walk.phase(p);
+    char *first = static_cast<char *>(a.dst[vr]) +
+                  (bcast ? 0ull : static_cast<unsigned long long>(p) * a.stride);
+    d.base = first - d.phase;
+    d.nvec = walk.vectors(d.phase);
+    d.aligned = (reinterpret_cast<unsigned long long>(d.base) & 15ull) == 0ull;
+    return d;
+}
 
 __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
     pull_kernel(const __grid_constant__ CommCtx ctx, const __grid_constant__ PullArgs a)
@@ -55,21 +77,11 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
     const bool bcast = a.root >= 0;
     const bool packs = (!bcast || a.root == rank) && a.src[vr] != nullptr;
     const bool stores = a.dst[vr] != nullptr;
-    const PullWalk walk{a.bytes, a.stride, static_cast<int>(gridDim.x),
-                        static_cast<int>(blockIdx.x), a.tile_shift};
+    const PullWalk walk{{a.bytes, a.stride}, static_cast<int>(gridDim.x), static_cast<int>(blockIdx.x), a.tile_shift};
     sync_begin(ctx, rank, &sync);
     const unsigned long long policy = evict_first_policy();
-    // blocks[p]: where the data of source p goes (broadcast: the same place for every p)
     if (static_cast<int>(threadIdx.x) < world) {
-        const int p = static_cast<int>(threadIdx.x);
-        PullBlock d;
-        d.phase = bcast ? 0u : walk.phase(p);
-        char *first = static_cast<char *>(a.dst[vr]) +
-                      (bcast ? 0ull : static_cast<unsigned long long>(p) * a.stride);
-        d.base = first - d.phase;
-        d.nvec = walk.vectors(d.phase);
-        d.aligned = (reinterpret_cast<unsigned long long>(d.base) & 15ull) == 0ull;
-        blocks[p] = d;
+        blocks[threadIdx.x] = pull_block(a, walk, vr, static_cast<int>(threadIdx.x));
     }
     __syncthreads();
 
@@ -169,245 +181,319 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
     sync_end(ctx, rank, &sync);
 }
 
-// The same for messages of several rounds.  What bounds them is bytes in flight, and
-// registers hold too few: the copies from the rings to the tensors go through shared
-// memory by bulk asynchronous copies in both directions, which one thread of an extra warp
-// keeps under way while the other warps pack the next tile.  Pass k: tile k-1 is copied
-// and tile k packed side by side; arrive; wait for the others.  (An arrival then also says that
-// tile k-1 has been read.)  Vectors at a block's ends are stored byte by byte; a
-// destination that is not 16-byte aligned is written by the packing warps.
-// launch_pull says which messages it is for.
-constexpr int kPullBufs = 5;  // of kPullBufVec vectors: four blocks of an SM fit
-constexpr unsigned int kPullBufVec = 512;
-constexpr int kPullLongThreads = kPullThreads + 32;
-constexpr int kPullLongBatch = 4;  // vectors of a packing thread in flight
+// The same for messages of several rounds.  What bounds them is bytes in flight and the way of a flag
+// (a fence for the block's stores, the flag, its poll, the first load behind it: 4 to 8 us under
+// load, several times what the bytes of a round take).  So four warps of a block look after these
+// (ring_sync.cuh, as in staged_kernel.cuh): the loader brings the tensor's tiles into shared memory by bulk
+// copies, the teller sets the flags, the fetcher polls them and brings the ring pieces of all
+// sources into shared memory, the storer takes them on to the destination, by bulk copies too.  The workers
+// only pack: pass k takes tile k from shared memory to the ring (and to the own block of the destination), and
+// waits for the pieces of tile k - lag.  An odd destination is theirs as well: its vectors are put together
+// from two of the piece's.  Ring of 2 lag + 1: tile k goes over tile k - 2 lag - 1, which its readers had
+// in their shared memory before the flags that the fetcher saw for pass k - 1.
+// Measured among ranks of one GPU, us, against a kernel that copied by bulk copies in lockstep with the pack, or
+// pull_kernel: broadcast of 94 MB to 3 others 108 / 90, 100 MB to 7 220 / 186, 9 MB to 5 27 / 20; all_gather of
+// 8 x 2.47 MB (an odd size) 54 / 42, 8 x 8 MB 142 / 118, 3 x 34 MB 104 / 96, 8 x 0.7 MB 25.5 / 18; to destinations off a
+// vector boundary 8 x 2.47 MB 435 / 51, broadcast of 34 MB to 3 321 / 42.
+// By lag, broadcast of 94 MB: 2: 143, 3: 121, 5: 100, 7: 95 (before there was a storer); no more from there on.
+// Two blocks per SM and 100 KB each, or three and 64: 8 x 2.47 MB 42 / 44, 94 MB 91 / 89; buffers for three or four rounds
+// of pieces, with smaller tiles: 49, 57 and 93, 102.
+struct PullShared {
+    PullBlock blocks[kMaxRanks];
+    // A round's bytes are there: the tensor's, the ring pieces of all sources.
+    Phases<2> tensor;
+    Phases<kPullDepth> pieces;
+    // Workers and storer are done with them.
+    Phases<2> packed;
+    Phases<kPullDepth> stored;
+    Phases<8> done;  // passes: tile k packed, tile k - lag here
+    uint32_t epoch;
+    int dead;  // the block gives up
+};
+static_assert(kPullLag <= 7, "passes that the workers may be ahead of the warp that tells the peers");
 
-__device__ __forceinline__ void bulk_store(void *dst, uint32_t src_smem, uint32_t bytes)
+// n bytes of shared memory to a destination of any alignment: the lanes of `threads` threads that share a run
+// (this one is `me`).  Aligned stores, put together from two vectors where the addresses differ.
+__device__ __forceinline__ void store_run(char *dst, uint32_t src, unsigned int n, unsigned int me,
+                                          unsigned int threads, unsigned long long policy)
 {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-                 "r"(src_smem), "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+    const unsigned int to_vec = static_cast<unsigned int>(-reinterpret_cast<long long>(dst)) & 15u;
+    const unsigned int head = to_vec < n ? to_vec : n;
+    const unsigned int vecs = (n - head) / 16u;
+    const uint32_t from = src + head;
+    const unsigned int odd = from & 15u;
+    for (unsigned int j = me; j < vecs; j += threads) {
+        const uint32_t at = (from & ~15u) + j * 16u;
+        uint4 x = ld_shared_v4(at);
+        if (odd != 0u) { x = shift_bytes(x, ld_shared_v4(at + 16u), odd); }
+        st_stream_v4(dst + head + j * 16ull, x, policy);
+    }
+    const char *bytes = static_cast<const char *>(__cvta_shared_to_generic(src));
+    const unsigned int rest = head + vecs * 16u;
+    for (unsigned int j = me; j < head; j += threads) { dst[j] = bytes[j]; }
+    for (unsigned int j = rest + me; j < n; j += threads) { dst[j] = bytes[j]; }
 }
 
-__global__ void __launch_bounds__(kPullLongThreads, kPullPerSm)
+struct PullLong {
+    const CommCtx &ctx;
+    const PullArgs &a;
+    PullShared &sh;
+    PullLongWalk walk;
+    uint32_t smem;
+    int vr, rank, sources;
+    bool packs, stores;
+
+    __device__ __forceinline__ PullLong(const CommCtx &c, const PullArgs &args, PullShared &shared, uint32_t bufs)
+        : ctx(c), a(args), sh(shared), walk{{args.bytes, args.stride}, static_cast<int>(gridDim.x),
+                                            static_cast<int>(blockIdx.x), args.tile},
+          smem(bufs), vr(static_cast<int>(blockIdx.y)), rank(c.rank + vr)
+    {
+        const bool bcast = a.root >= 0;
+        packs = (!bcast || a.root == rank) && a.src[vr] != nullptr;
+        stores = a.dst[vr] != nullptr;
+        sources = !stores ? 0 : bcast ? (a.root == rank ? 0 : 1) : ctx.world - 1;
+    }
+    // starting with the next rank, so that peers do not all read the same GPU first
+    __device__ __forceinline__ int source_at(int i) const
+    {
+        if (a.root >= 0) { return a.root; }
+        const int p = rank + 1 + i;
+        return p < ctx.world ? p : p - ctx.world;
+    }
+    __device__ __forceinline__ unsigned int vectors(int p, int k) const
+    {
+        const unsigned long long v0 = walk.first_vector(k), end = sh.blocks[p].nvec;
+        return v0 >= end ? 0u : end - v0 < a.tile ? static_cast<unsigned int>(end - v0) : a.tile;
+    }
+    // two rounds of the tensor (a vector more: it may start anywhere in one), kPullDepth of all sources' pieces
+    __device__ __forceinline__ uint32_t tensor(int k) const { return smem + (k & 1) * (a.tile + 1u) * 16u; }
+    __device__ __forceinline__ uint32_t piece(int i, int k) const
+    {
+        return smem + (2u * (a.tile + 1u) + static_cast<unsigned int>(k % kPullDepth * sources + i) * a.tile) * 16u;
+    }
+    // where tile k lies in tensor memory (its first byte), and the aligned address that comes first in tensor(k)
+    __device__ __forceinline__ unsigned long long tensor_at(int k) const
+    {
+        return reinterpret_cast<unsigned long long>(a.src[vr]) + 16ull * walk.first_vector(k) - sh.blocks[rank].phase;
+    }
+
+    __device__ __forceinline__ void load() const
+    {
+        if (!packs || (threadIdx.x & 31u) != 0u) { return; }
+        const unsigned long long policy = evict_first_policy();
+        const unsigned long long begin = reinterpret_cast<unsigned long long>(a.src[vr]) & ~15ull;
+        const unsigned long long end = (reinterpret_cast<unsigned long long>(a.src[vr]) + a.bytes + 15ull) & ~15ull;
+        for (int k = 0; k < a.rounds; ++k) {
+            // whole aligned vectors that hold a byte of the tensor
+            const unsigned int n = vectors(rank, k);
+            const unsigned long long at = tensor_at(k), first = at & ~15ull;
+            const unsigned long long lo = first > begin ? first : begin;
+            const unsigned long long last = first + 16ull * n + (at != first ? 16ull : 0ull);
+            const unsigned long long hi = last < end ? last : end;
+            if (k >= 2 && !ring_wait(ctx, sh.dead, sh.packed, k - 2)) {
+                // its copies in flight end before the block does
+                drain(ctx, sh.tensor, k - 2);
+                drain(ctx, sh.tensor, k - 1);
+                return;
+            }
+            ask_stream(sh.tensor.at(k), tensor(k) + static_cast<uint32_t>(lo - first), reinterpret_cast<const void *>(lo),
+                       n != 0u && lo < hi ? static_cast<unsigned int>(hi - lo) : 0u, policy);
+        }
+    }
+
+    __device__ __forceinline__ void fetch(int told) const
+    {
+        const int i = static_cast<int>(threadIdx.x & 31u);
+        for (int t = 0; t < told; ++t) {
+            const bool more = t < a.rounds;
+            const unsigned int bytes = more && i < sources ? vectors(source_at(i), t) * 16u : 0u;
+            const unsigned int all = __reduce_add_sync(0xffffffffu, bytes);
+            const char *from = ctx.base[i < sources ? source_at(i) : rank] + a.off + walk.piece(t);
+            const uint32_t to = piece(i, t);
+            // (pass r + lag waits for round r)
+            const int before = t - kPullDepth;
+            bool ok = !more || before < 0 || (sources != 0 ? ring_wait(ctx, sh.dead, sh.stored, before)
+                                                           : ring_wait(ctx, sh.dead, sh.done, before + kPullLag));
+            if (ok && i < ctx.world) { ok = poll_acquire(ctx, rank, i, sh.epoch + static_cast<uint32_t>(t) + 1u, 0); }
+            if (!warp_agrees(ok)) {
+                *static_cast<volatile int *>(&sh.dead) = 1;
+                for (int j = 1; j <= kPullDepth; ++j) { drain(ctx, sh.pieces, t - j < a.rounds ? t - j : -1); }
+                return;
+            }
+            if (!more) { continue; }
+            if (i == 0) { mbar_expect_tx(sh.pieces.at(t), all); }
+            if (bytes != 0u) { bulk_load(to, from, bytes, sh.pieces.at(t)); }
+        }
+        if (i == 0) { pad_of(ctx, rank)->epoch[blockIdx.x] = sh.epoch + static_cast<uint32_t>(told); }
+    }
+
+    // Bytes of source p's tile t that its block has: from shared address `piece`, to where.
+    struct Run {
+        char *dst;
+        uint32_t src;
+        unsigned int n;
+        // both start at the same byte of a vector
+        __device__ __forceinline__ bool alike() const
+        {
+            return ((static_cast<uint32_t>(reinterpret_cast<unsigned long long>(dst)) ^ src) & 15u) == 0u;
+        }
+    };
+    __device__ __forceinline__ Run run_of(int p, int t, uint32_t piece) const
+    {
+        const PullBlock &d = sh.blocks[p];
+        const unsigned long long at = 16ull * walk.first_vector(t), end = a.bytes + d.phase;
+        const unsigned long long lo = at < d.phase ? d.phase : at;
+        const unsigned long long to = at + 16ull * a.tile, hi = to < end ? to : end;
+        return Run{d.base + lo, piece + static_cast<uint32_t>(lo - at), lo < hi ? static_cast<unsigned int>(hi - lo) : 0u};
+    }
+
+    // Tile k of the own data: to the ring, and to its place in the own destination.
+    __device__ __forceinline__ void pack(int k) const
+    {
+        const unsigned long long policy = evict_first_policy();
+        const PullBlock &own = sh.blocks[rank];
+        const unsigned long long v0 = walk.first_vector(k);
+        const unsigned int odd = static_cast<unsigned int>(tensor_at(k) & 15ull);
+        const unsigned int n = vectors(rank, k);
+        char *to = ctx.base[rank] + a.off + walk.piece(k);
+        const bool keeps = stores && own.base + own.phase != a.src[vr];  // else the own block is in place
+        // all vectors but the block's ends, stored as they are packed
+        const bool aligned = keeps && own.aligned;
+#pragma unroll 2
+        for (unsigned int i = threadIdx.x; i < n; i += kPullLongThreads) {
+            const uint32_t at = tensor(k) + i * 16u;
+            uint4 x = ld_shared_v4(at);
+            if (odd != 0u) { x = shift_bytes(x, ld_shared_v4(at + 16u), odd); }
+            st_arena_v4(to + i * 16u, x);
+            if (aligned && own.whole(v0 + i, 1)) { st_stream_v4(own.base + (v0 + i) * 16ull, x, policy); }
+        }
+        if (!keeps) { return; }
+        const Run run = run_of(rank, k, tensor(k) + odd);
+        if (!aligned) {
+            store_run(run.dst, run.src, run.n, threadIdx.x, kPullLongThreads, policy);
+        } else if (n != 0u && (v0 == 0 || v0 + n == own.nvec)) {
+            // the ends
+            const unsigned int first = v0 == 0 ? (run.n < 16u - own.phase ? run.n : 16u - own.phase) : 0u;
+            store_run(run.dst, run.src, first, threadIdx.x, kPullLongThreads, policy);
+            if (v0 + n == own.nvec && n + v0 > 1) {
+                const unsigned int last = (static_cast<unsigned int>(a.bytes + own.phase - 1ull) & 15u) + 1u;
+                store_run(run.dst + run.n - last, run.src + run.n - last, last, threadIdx.x, kPullLongThreads, policy);
+            }
+        }
+    }
+
+    // The storer: a lane per source takes its tiles on to the destination.
+    __device__ __forceinline__ void store() const
+    {
+        if (!stores || sources == 0) { return; }
+        const int i = static_cast<int>(threadIdx.x & 31u);
+        const unsigned long long policy = evict_first_policy();
+        for (int t = 0; t < a.rounds; ++t) {
+            if (!warp_agrees(ring_wait(ctx, sh.dead, sh.pieces, t))) { break; }
+            if (i < sources) {
+                const Run run = run_of(source_at(i), t, piece(i, t));
+                if (run.n != 0u && run.alike()) {
+                    const unsigned int to_vec = (16u - (run.src & 15u)) & 15u, head = to_vec < run.n ? to_vec : run.n;
+                    const unsigned int whole = (run.n - head) & ~15u;
+                    if (whole != 0u) {
+                        asm volatile("cp.async.bulk.global.shared::cta.bulk_group.L2::cache_hint [%0], [%1], %2, %3;" ::"l"(
+                                         run.dst + head),
+                                     "r"(run.src + head), "r"(whole), "l"(policy)
+                                     : "memory");
+                    }
+                    const char *bytes = static_cast<const char *>(__cvta_shared_to_generic(run.src));
+                    for (unsigned int j = 0; j < head; ++j) { run.dst[j] = bytes[j]; }
+                    for (unsigned int j = head + whole; j < run.n; ++j) { run.dst[j] = bytes[j]; }
+                }
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+            }
+            warp_arrive(sh.stored.at(t));
+        }
+        asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+
+    __device__ __forceinline__ void work() const
+    {
+        const unsigned long long policy = evict_first_policy();
+#pragma unroll 1
+        for (int k = 0; k < a.rounds + kPullLag; ++k) {
+            if (k < a.rounds && packs) {
+                if (!ring_wait(ctx, sh.dead, sh.tensor, k)) { return; }
+                pack(k);
+                warp_arrive(sh.packed.at(k));
+            }
+            const int t = k - kPullLag;
+            if (t >= 0 && !ring_wait(ctx, sh.dead, sh.pieces, t)) { return; }
+            warp_arrive(sh.done.at(k));
+            if (t >= 0 && sources != 0) {
+                // what the storer cannot do
+                for (int i = 0; i < sources; ++i) {
+                    const Run run = run_of(source_at(i), t, piece(i, t));
+                    if (!run.alike()) { store_run(run.dst, run.src, run.n, threadIdx.x, kPullLongThreads, policy); }
+                }
+                warp_arrive(sh.stored.at(t));
+            }
+        }
+    }
+};
+
+__global__ void __launch_bounds__(kPullLongBlock, kPullLongPerSm)
     pull_long_kernel(const __grid_constant__ CommCtx ctx, const __grid_constant__ PullArgs a)
 {
     extern __shared__ __align__(128) unsigned char bufs[];
-    __shared__ BlockSync sync;
-    __shared__ PullBlock blocks[kMaxRanks];
-    __shared__ __align__(8) unsigned long long bars[kPullBufs];
-    const int vr = static_cast<int>(blockIdx.y);
-    const int rank = ctx.rank + vr;
-    const int world = ctx.world;
-    const bool bcast = a.root >= 0;
-    const bool packs = (!bcast || a.root == rank) && a.src[vr] != nullptr;
-    const bool stores = a.dst[vr] != nullptr;
-    const PullWalk walk{a.bytes, a.stride, static_cast<int>(gridDim.x),
-                        static_cast<int>(blockIdx.x), a.tile_shift};
-    sync_begin(ctx, rank, &sync);
-    const unsigned long long policy = evict_first_policy();
-    const uint32_t bars_s = smem_addr(bars), bufs_s = smem_addr(bufs);
-    if (static_cast<int>(threadIdx.x) < world) {
-        const int p = static_cast<int>(threadIdx.x);
-        PullBlock d;
-        d.phase = bcast ? 0u : walk.phase(p);
-        char *first = static_cast<char *>(a.dst[vr]) +
-                      (bcast ? 0ull : static_cast<unsigned long long>(p) * a.stride);
-        d.base = first - d.phase;
-        d.nvec = walk.vectors(d.phase);
-        d.aligned = (reinterpret_cast<unsigned long long>(d.base) & 15ull) == 0ull;
-        blocks[p] = d;
-    }
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < kPullBufs; ++i) { mbar_init(bars_s + 8u * i, 1u); }
+    __shared__ __align__(16) PullShared sh;
+    const PullLong pull(ctx, a, sh, smem_addr(bufs));
+    const int tid = static_cast<int>(threadIdx.x);
+    if (tid < ctx.world) { sh.blocks[tid] = pull_block(a, pull.walk, pull.vr, tid); }
+    if (tid == 0) {
+        sh.epoch = pad_of(ctx, pull.rank)->epoch[blockIdx.x];
+        sh.dead = 0;
+        sh.tensor.init(1u);
+        sh.pieces.init(1u);
+        sh.packed.init(kPullLongThreads / 32);
+        sh.stored.init(kPullLongThreads / 32 + 1);
+        sh.done.init(kPullLongThreads / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_proxy();
     }
     __syncthreads();
-
-    const PullBlock &own = blocks[rank];
-    const ShiftedSource src(a.src[vr], a.bytes, own.phase);
-    const bool ring_only = !stores || own.base + own.phase == a.src[vr];  // own block: packed, not stored
-    const bool by_bulk = own.aligned;  // alike for all blocks of a destination
-    char *ring = ctx.base[rank] + a.off;
-    const unsigned long long tile = 1ull << a.tile_shift;
-    const int steps = 1 << (a.tile_shift - kPullStepShift);
-    const int sources = !stores ? 0 : bcast ? (a.root == rank ? 0 : 1) : world - 1;
-    auto source_at = [&](int i) {
-        if (bcast) { return a.root; }
-        const int p = rank + 1 + i;
-        return p < world ? p : p - world;
-    };
-    const bool copier = threadIdx.x == kPullThreads;
-    int filled = 0;  // copier only: buffers filled so far
-
-    for (int k = 0; k <= a.rounds; ++k) {
-        bool ok = true;
-        // broadcast: root's pack is what the others wait for, from an eighth or so of the
-        // grid (94 MB to 3 others: 116 us without, 108 with it); in an all_gather every rank packs
-        if (is_sync_thread() && bcast && packs && k + 1 < a.rounds) {
-            src.prefetch(walk.first_vector(k + 1), tile);
-        }
-        if (threadIdx.x < kPullThreads && packs && k < a.rounds) {
-            // ---- pack tile k
-            const unsigned long long v0 = walk.first_vector(k);
-            char *to = ring + walk.piece(k);
-            for (int q0 = 0; q0 < steps; q0 += kPullLongBatch) {
-                uint4 x[kPullLongBatch];
-#pragma unroll
-                for (int u = 0; u < kPullLongBatch; ++u) {
-                    const unsigned int i = (static_cast<unsigned int>(q0 + u) << kPullStepShift) + threadIdx.x;
-                    if (q0 + u >= steps) { continue; }
-                    if (own.inside(v0 + i - threadIdx.x)) {
-                        x[u] = src.load_inside(v0 + i, policy);
-                    } else if (v0 + i < own.nvec) {
-                        x[u] = src.load(v0 + i, policy);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kPullLongBatch; ++u) {
-                    const unsigned int i = (static_cast<unsigned int>(q0 + u) << kPullStepShift) + threadIdx.x;
-                    if (q0 + u >= steps || v0 + i >= own.nvec) { continue; }
-                    st_arena_v4(to + i * 16u, x[u]);
-                    if (ring_only) { continue; }
-                    if (own.inside(v0 + i - threadIdx.x)) {
-                        st_stream_v4(own.base + (v0 + i) * 16ull, x[u], policy);
-                    } else {
-                        store_virtual(own.base + own.phase, a.bytes, own.phase, v0 + i, x[u], policy);
-                    }
-                }
-            }
-            fence_async_proxy();  // the peers read the ring with bulk copies
-        }
-        if (k > 0) {
-            const unsigned long long v0 = walk.first_vector(k - 1);
-            const unsigned long long from = a.off + walk.piece(k - 1);
-            if (!by_bulk) {
-                for (int i = 0; threadIdx.x < kPullThreads && i < sources; ++i) {
-                    const int p = source_at(i);
-                    const PullBlock &d = blocks[p];
-                    for (unsigned long long v = v0 + threadIdx.x; v < v0 + tile && v < d.nvec;
-                         v += kPullThreads) {
-                        store_virtual(d.base + d.phase, a.bytes, d.phase, v,
-                                      ld_arena_v4(ctx.base[p] + from + (v - v0) * 16ull), policy);
-                    }
-                }
-            } else if (copier) {
-                // ---- copy tile k-1 of the other sources: whole vectors by bulk copies
-                fence_async_proxy();
-                int stored = filled;
-                auto span_of_source = [&](const PullBlock &d, unsigned long long *lo, unsigned long long *hi) {
-                    const unsigned long long end = (a.bytes + d.phase) % 16ull != 0ull ? d.nvec - 1 : d.nvec;
-                    *lo = v0 == 0 && d.phase != 0u ? 1ull : v0;
-                    *hi = v0 + tile < end ? v0 + tile : end;
-                };
-                // two walks over the same chunks, the loads ahead of the stores
-                int li = 0, si = 0;
-                unsigned long long lv = 0, lhi = 0, sv = 0, shi = 0;
-                bool lopen = false, sopen = false;
-                auto next = [&](int *i, bool *open, unsigned long long *v, unsigned long long *hi) {
-                    while (*i < sources) {
-                        if (!*open) {
-                            span_of_source(blocks[source_at(*i)], v, hi);
-                            *open = true;
-                        }
-                        if (*v < *hi) { return true; }
-                        *open = false;
-                        ++*i;
-                    }
-                    return false;
-                };
-                for (;;) {
-                    while (ok && filled - stored < kPullBufs - 1 && next(&li, &lopen, &lv, &lhi)) {
-                        const int j = filled % kPullBufs;
-                        // the store of kPullBufs chunks ago must have read this buffer; at
-                        // least one younger store has been issued since, which need not
-                        asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
-                        const unsigned long long n = lhi - lv < kPullBufVec ? lhi - lv : kPullBufVec;
-                        const uint32_t bytes = static_cast<uint32_t>(n) * 16u;
-                        mbar_expect_tx(bars_s + 8u * j, bytes);
-                        bulk_load(bufs_s + j * kPullBufVec * 16u,
-                                  ctx.base[source_at(li)] + from + (lv - v0) * 16ull, bytes,
-                                  bars_s + 8u * j);
-                        lv += n;
-                        ++filled;
-                    }
-                    if (stored == filled) { break; }
-                    const int j = stored % kPullBufs;
-                    ok = mbar_wait(ctx, bars_s + 8u * j, static_cast<uint32_t>((stored / kPullBufs) & 1),
-                                   ctx.timeout_ns) && ok;
-                    if (!ok) {
-                        report_timeout(ctx, rank, -1, 0u, 0u, 64);
-                        // the others already under way: one more bounded chance each
-                        for (int t = stored + 1; t < filled; ++t) {
-                            (void)mbar_wait(ctx, bars_s + 8u * (t % kPullBufs),
-                                            static_cast<uint32_t>((t / kPullBufs) & 1), ctx.timeout_ns / 4);
-                        }
-                        break;
-                    }
-                    (void)next(&si, &sopen, &sv, &shi);
-                    const unsigned long long n = shi - sv < kPullBufVec ? shi - sv : kPullBufVec;
-                    bulk_store(blocks[source_at(si)].base + sv * 16ull, bufs_s + j * kPullBufVec * 16u,
-                               static_cast<uint32_t>(n) * 16u);
-                    sv += n;
-                    ++stored;
-                }
-            } else if (threadIdx.x > kPullThreads) {
-                // the ends of the blocks: lanes of the copier's warp, a source each
-                for (int i = static_cast<int>(threadIdx.x) - kPullThreads - 1; i < sources; i += 31) {
-                    const int p = source_at(i);
-                    const PullBlock &d = blocks[p];
-                    const unsigned long long last = d.nvec - 1;
-                    if (v0 == 0 && d.phase != 0u) {
-                        store_virtual(d.base + d.phase, a.bytes, d.phase, 0,
-                                      ld_arena_v4(ctx.base[p] + from), policy);
-                    }
-                    if ((a.bytes + d.phase) % 16ull != 0ull && last >= v0 && last < v0 + tile &&
-                        !(last == 0 && d.phase != 0u)) {
-                        store_virtual(d.base + d.phase, a.bytes, d.phase, last,
-                                      ld_arena_v4(ctx.base[p] + from + (last - v0) * 16ull), policy);
-                    }
-                }
-            }
-        }
-        if (__syncthreads_and(ok ? 1 : 0) == 0) {
-            if (copier) { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-            return;
-        }
-        if (k < a.rounds) {
-            tell_all(ctx, rank, &sync, k + 1);
-            if (!wait_all(ctx, rank, &sync, k + 1)) {
-                if (copier) { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-                return;
-            }
-        }
+    // (the rings of the last tiles may only be reused when all have read them: the next
+    // call uses the other slot, whose users of the call before this one are done)
+    const int told = a.rounds + (a.end_barrier != 0 ? kPullLag : 0);
+    if (tid < kPullLongThreads) {
+        pull.work();
+    } else if (tid < kPullLongThreads + 32) {
+        pull.load();
+    } else if (tid < kPullLongThreads + 64) {
+        ring_tell(ctx, sh.dead, sh.epoch, sh.done, pull.rank, told);
+    } else if (tid < kPullLongThreads + 96) {
+        pull.fetch(told);
+    } else {
+        pull.store();
     }
-    if (copier) { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-    advance_epoch(&sync, a.rounds);
-    // the rings of the last tiles may only be reused when all have read them: the next
-    // call uses the other slot, whose users of the call before this one are done
-    if (a.end_barrier && !peer_barrier(ctx, rank, &sync)) { return; }
-    sync_end(ctx, rank, &sync);
 }
 
 int launch_pull(const CommCtx &ctx, const PullArgs &a, int blocks, int vranks, void *stream)
 {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const dim3 grid(blocks, vranks, 1);
-    // One or two rounds are a matter of latency, to which the way through shared memory adds.
-    // From three on, us, pull_kernel / pull_long_kernel, tensors not in the L2: broadcast of
-    // 100 MB to 3 121 / 117, 34 MB to 5 70 / 66, 100 MB to 7 228 / 216, 17 MB to 7 49 / 48.
-    // all_gather, in which every rank copies and packs the whole time: 3 x 34 MB 110 / 103,
-    // 4 x 17 MB 78 / 83, 4 x 100 MB 442 / 437, 8 x 2.47 MB 58 both, 8 x 8 MB 150 / 160.
-    // Two ranks: the registers keep up (broadcast 100 MB 70 / 74, all_gather 34 MB 57 both).
-    // (Destinations off a vector boundary do better in pull_kernel throughout, 34 MB to 3: 293 / 325,
-    // but a rank does not know the others', and all have to run the same kernel.)
-    const bool lng = a.rounds > 2 && ctx.world > 2 && (a.root >= 0 || ctx.world == 3);
-    const void *kernel = lng ? reinterpret_cast<const void *>(&pull_long_kernel)
-                             : reinterpret_cast<const void *>(&pull_kernel);
-    const dim3 block(lng ? kPullLongThreads : kPullThreads);
-    const size_t smem = lng ? kPullBufs * kPullBufVec * 16u : 0u;
+    const void *kernel = a.lng != 0 ? reinterpret_cast<const void *>(&pull_long_kernel)
+                                    : reinterpret_cast<const void *>(&pull_kernel);
+    const dim3 block(a.lng != 0 ? kPullLongBlock : kPullThreads);
+    const size_t smem = a.lng != 0 ? pull_long_smem(pull_sources(ctx.world, a.root), a.tile) : 0u;
+    if (smem != 0) {
+        // the opt-in to more than 48 KB is per function and per device
+        static std::atomic<bool> opted_in[64] = {};
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { dev = 0; }
+        if (!opted_in[dev].load(std::memory_order_relaxed)) {
+            const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       static_cast<int>(kPullLongSmem));
+            if (e != cudaSuccess) { return static_cast<int>(e); }
+            opted_in[dev].store(true, std::memory_order_relaxed);
+        }
+    }
     void *params[2] = {const_cast<CommCtx *>(&ctx), const_cast<PullArgs *>(&a)};
     if (vranks > 1) {
         return static_cast<int>(cudaLaunchCooperativeKernel(kernel, grid, block, params, smem, s));

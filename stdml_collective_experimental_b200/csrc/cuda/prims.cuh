@@ -124,16 +124,19 @@ static __device__ __noinline__ void report_timeout(const CommCtx &ctx, int rank,
 
 // One thread waits until rank src's flag for this block has reached `target`,
 // with a time and an iteration limit.  False: the limit was reached (reported).
-template <typename Look>
+template <typename Look, typename Seen>
 __device__ __forceinline__ bool poll_with(const CommCtx &ctx, int rank, int src, uint32_t target,
-                                          int phase, Look look)
+                                          int phase, Look look, Seen then)
 {
     const uint32_t *f = &pad_of(ctx, rank)->flag[blockIdx.x][src];
     unsigned int spins = 0;
     unsigned long long t0 = 0;
     for (;;) {
         const uint32_t seen = look(f);
-        if (static_cast<int32_t>(seen - target) >= 0) { return true; }
+        if (static_cast<int32_t>(seen - target) >= 0) {
+            then();
+            return true;
+        }
         ++spins;
         if ((spins & 127u) == 0u) {
             const unsigned long long now = global_ns();
@@ -149,11 +152,9 @@ __device__ __forceinline__ bool poll_with(const CommCtx &ctx, int rank, int src,
 __device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src, uint32_t target,
                                           int phase)
 {
-    if (!poll_with(ctx, rank, src, target, phase, [](const uint32_t *f) { return ld_relaxed_sys_u32(f); })) {
-        return false;
-    }
-    fence_ranks(ctx);
-    return true;
+    return poll_with(
+        ctx, rank, src, target, phase, [](const uint32_t *f) { return ld_relaxed_sys_u32(f); },
+        [&] { fence_ranks(ctx); });
 }
 
 // The same by acquiring loads, without the fence, which would wait for the SM's own
@@ -161,15 +162,18 @@ __device__ __forceinline__ bool poll_flag(const CommCtx &ctx, int rank, int src,
 __device__ __forceinline__ bool poll_acquire(const CommCtx &ctx, int rank, int src, uint32_t target,
                                              int phase)
 {
-    return poll_with(ctx, rank, src, target, phase, [&](const uint32_t *f) {
-        uint32_t v;
-        if (ctx.one_gpu) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
-        } else {
-            asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
-        }
-        return v;
-    });
+    return poll_with(
+        ctx, rank, src, target, phase,
+        [&](const uint32_t *f) {
+            uint32_t v;
+            if (ctx.one_gpu) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+            } else {
+                asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(f) : "memory");
+            }
+            return v;
+        },
+        [] {});
 }
 
 // arrive_all (below) behind a block sync that the caller has made.

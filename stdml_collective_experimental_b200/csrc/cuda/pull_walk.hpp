@@ -10,17 +10,22 @@
 namespace stdml::collective::cuda
 {
 // A rank's block of `bytes` bytes is seen as vectors of 16 bytes in which it starts
-// `phase` bytes after the beginning of vector 0, as it does in a 16-byte aligned destination.  Block b of the grid moves vectors [k * nb + b) * T, + T) in round k.
-struct PullWalk {
+// `phase` bytes after the beginning of vector 0, as it does in a 16-byte aligned destination.
+struct PullLayout {
     unsigned long long bytes, stride;  // destination blocks start `stride` bytes apart
-    int nb, b;
-    int tile_shift;  // T = 1 << tile_shift vectors
 
     STDML_HD unsigned int phase(int p) const
     {
         return static_cast<unsigned int>(p) * static_cast<unsigned int>(stride & 15ull) & 15u;
     }
     STDML_HD unsigned long long vectors(unsigned int ph) const { return (bytes + ph + 15ull) / 16ull; }
+};
+
+// Block b of the grid moves vectors [k * nb + b) * T, + T) in round k.
+struct PullWalk : PullLayout {
+    int nb, b;
+    int tile_shift;  // T = 1 << tile_shift vectors
+
     STDML_HD unsigned long long first_vector(int k) const
     {
         return (static_cast<unsigned long long>(k) * nb + b) << tile_shift;
@@ -32,33 +37,71 @@ struct PullWalk {
     }
 };
 
-struct PullGeometry {
-    int blocks = 0;  // 0: the slot cannot hold the ring of even one block
-    int tile_shift = kPullStepShift, rounds = 1;
-    // of the staging slot, for all blocks
-    size_t ring_bytes() const
+// The same for pull_long_kernel: tiles of any number of vectors, a longer ring.
+struct PullLongWalk : PullLayout {
+    int nb, b;
+    unsigned int tile;
+
+    STDML_HD unsigned long long first_vector(int k) const
     {
-        return ((static_cast<size_t>(blocks) * kPullRing) << tile_shift) * 16;
+        return (static_cast<unsigned long long>(k) * nb + b) * tile;
+    }
+    STDML_HD unsigned long long piece(int k) const
+    {
+        return (static_cast<unsigned long long>(b) * kPullLongRing + k % kPullLongRing) * tile * 16ull;
     }
 };
 
-// Grid and tile for blocks of `bytes` bytes read from `sources` ranks: a tile gives
-// each thread up to kPullVec vectors to copy per round over all sources, less where the
-// message would otherwise leave blocks without a tile.
-inline PullGeometry pull_geometry(int sources, size_t bytes, size_t staging_bytes, int max_blocks)
+struct PullGeometry {
+    int blocks = 0;  // 0: the slot cannot hold the ring of even one block
+    unsigned int tile = 1u << kPullStepShift;
+    int rounds = 1, ring = kPullRing;
+    bool lng = false;  // for pull_long_kernel
+    // of the staging slot, for all blocks
+    size_t ring_bytes() const { return static_cast<size_t>(blocks) * ring * tile * 16; }
+};
+
+// Grid and tile for blocks of `bytes` bytes read from `sources` ranks, on `num_sms` SMs that `vranks` ranks
+// share.  pull_kernel: a tile gives each thread up to kPullVec vectors to copy per round over
+// all sources, less where the message would otherwise leave blocks without a tile.
+inline PullGeometry pull_geometry(int sources, size_t bytes, size_t staging_bytes, int num_sms, int vranks,
+                                  int want_blocks)
 {
-    PullGeometry g;
-    const size_t most = static_cast<size_t>(max_blocks);
+    const auto resident = [&](int per_sm) {
+        const int n = std::max(1, std::min(kMaxBlocks, per_sm * num_sms / vranks));
+        return static_cast<size_t>(want_blocks > 0 ? std::min(want_blocks, n) : n);
+    };
     const size_t nvec = (bytes + 15 + 15) / 16;  // with the largest shift
+    PullGeometry g;
+    size_t most = resident(kPullPerSm);
     const size_t want = static_cast<size_t>(kPullThreads) * kPullVec / static_cast<size_t>(std::max(1, sources));
-    const auto ring_bytes = [&](int shift) { return (static_cast<size_t>(kPullRing) << shift) * 16; };
-    while ((size_t{2} << g.tile_shift) <= want && (size_t{2} << g.tile_shift) * most <= nvec &&
-           ring_bytes(g.tile_shift + 1) * most <= staging_bytes) {
-        ++g.tile_shift;
+    while (g.tile * 2 <= want && g.tile * 2 * most <= nvec && kPullRing * g.tile * 2 * 16 * most <= staging_bytes) {
+        g.tile *= 2;
     }
-    const size_t tiles = (nvec + (size_t{1} << g.tile_shift) - 1) >> g.tile_shift;
-    g.blocks = static_cast<int>(std::min<size_t>({tiles, most, staging_bytes / ring_bytes(g.tile_shift)}));
-    if (g.blocks > 0) { g.rounds = static_cast<int>((tiles + g.blocks - 1) / g.blocks); }
+    const auto lay_out = [&]() {
+        const size_t tiles = (nvec + g.tile - 1) / g.tile;
+        g.blocks = static_cast<int>(std::min<size_t>({tiles, most, staging_bytes / (static_cast<size_t>(g.ring) * g.tile * 16)}));
+        if (g.blocks > 0) { g.rounds = static_cast<int>((tiles + g.blocks - 1) / g.blocks); }
+    };
+    lay_out();
+    // pull_long_kernel, wherever every block of its grid has some work: broadcast of 1 MB to 1 (422 vectors
+    // per block) 6.2 us and 6.4 so, of 0.5 MB to 7 (844) 9.7 and 8.2, all_gather of 8 x 0.7 MB 25.5 and 18.  From eight
+    // sources on its tiles and bulk copies get small (16 x 1 MB: 74 us, 81 so).
+    const PullGeometry s = g;
+    g.lng = true;
+    g.ring = kPullLongRing;
+    most = resident(kPullLongPerSm);
+    g.tile = pull_long_tile(sources);
+    lay_out();
+    if (sources > kPullLongSources || nvec < kPullLongMin * most ||
+        staging_bytes < static_cast<size_t>(g.ring) * g.tile * 16 * most) {
+        return s;
+    }
+    g.blocks = static_cast<int>(most);
+    // tiles of equal size that just fill their rounds
+    const size_t per_round = static_cast<size_t>(g.rounds) * g.blocks;
+    g.tile = static_cast<unsigned int>((nvec + per_round - 1) / per_round + 31) / 32 * 32;
+    lay_out();
     return g;
 }
 }  // namespace stdml::collective::cuda

@@ -1,0 +1,122 @@
+// How the warps of a block work together where some of them look after flags and loads and the
+// others (the workers) move bytes in rounds: staged_kernel.cuh, kernels_pull.cu.
+#pragma once
+#include "ar_kernel.cuh"
+#include "copy.cuh"
+
+namespace stdml::collective::cuda
+{
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t at)
+{
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "r"(at)
+                 : "memory");
+    return v;
+}
+
+// One phase per round of something, on N barriers in turn: who waits for round k finds it although
+// up to N - 1 later ones are over too.
+template <int N>
+struct Phases {
+    unsigned long long bar[N];
+
+    __device__ __forceinline__ void init(unsigned int count)
+    {
+        for (int i = 0; i < N; ++i) { mbar_init(smem_addr(&bar[i]), count); }
+    }
+    __device__ __forceinline__ uint32_t at(int k) const { return smem_addr(&bar[k % N]); }
+    // (may sleep a while on a round that is not over)
+    __device__ __forceinline__ bool try_wait(int k) const
+    {
+        return mbar_try_wait(at(k), static_cast<uint32_t>(k / N & 1));
+    }
+    __device__ __forceinline__ bool over(int k) const
+    {
+        uint32_t done;
+        asm volatile("{\n\t"
+                     ".reg .pred p;\n\t"
+                     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                     "selp.u32 %0, 1, 0, p;\n\t"
+                     "}"
+                     : "=r"(done)
+                     : "r"(at(k)), "r"(static_cast<uint32_t>(k / N & 1))
+                     : "memory");
+        return done != 0;
+    }
+};
+
+// Waits for round k of something.  False: the block gives up (`dead`, in shared memory).
+template <int N>
+__device__ __forceinline__ bool ring_wait(const CommCtx &ctx, int &dead, const Phases<N> &phases, int k)
+{
+    unsigned long long t0 = 0;
+    for (unsigned int spins = 0; !phases.try_wait(k); ++spins) {
+        if (*static_cast<volatile int *>(&dead) != 0) { return false; }
+        if ((spins & 63u) != 63u) { continue; }
+        const unsigned long long now = global_ns();
+        if (t0 == 0) { t0 = now; }
+        // (twice the limit of a wait for a peer's flag, of whose end `dead` tells)
+        if (now - t0 > 2 * ctx.timeout_ns || spins >= ctx.max_spins) {
+            *static_cast<volatile int *>(&dead) = 1;
+            return false;
+        }
+    }
+    return true;
+}
+
+// A warp that gives up: its copies of round k in flight end before the block does.
+template <int N>
+__device__ __forceinline__ void drain(const CommCtx &ctx, const Phases<N> &phases, int k)
+{
+    if (k >= 0) { (void)mbar_wait(ctx, phases.at(k), static_cast<uint32_t>(k / N & 1), ctx.timeout_ns / 4); }
+}
+
+__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok ? 1 : 0) != 0; }
+
+// One lane of a worker warp for all of it.
+__device__ __forceinline__ void warp_arrive(uint32_t bar)
+{
+    __syncwarp();
+    if ((threadIdx.x & 31u) == 0u) { mbar_arrive(bar); }
+}
+
+// Asks for the first `bytes` bytes at src, of tensor memory, past the L2 as far as it can; every lane
+// of a barrier of 32 calls it.
+__device__ __forceinline__ void ask_stream(uint32_t bar, uint32_t dst, const void *src,
+                                           unsigned int bytes, unsigned long long policy)
+{
+    if (bytes == 0u) {
+        mbar_arrive(bar);
+        return;
+    }
+    mbar_expect_tx(bar, bytes);
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+                 "[%0], [%1], %2, [%3], %4;" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar), "l"(policy)
+                 : "memory");
+}
+
+// The teller: lets the peers know what the passes have stored.  A warp of its own: its fences wait for
+// all of the block's stores.  Over links and within a GPU alike they and the flags' way take
+// longer than a pass, hence the lag.
+// `done`: a phase per pass.
+template <int N>
+__device__ __forceinline__ void ring_tell(const CommCtx &ctx, int &dead, uint32_t epoch, const Phases<N> &done,
+                                          int rank, int passes)
+{
+    const int p = static_cast<int>(threadIdx.x & 31u);
+    for (int k = 0; k < passes; ++k) {
+        if (!warp_agrees(ring_wait(ctx, dead, done, k))) { return; }
+        // (one fence for all that are over by now)
+        while (k + 1 < passes && warp_agrees(done.over(k + 1))) { ++k; }
+        fence_ranks(ctx);
+        fence_async_proxy_global();  // the peers read it by bulk copies
+        if (p < ctx.world) {
+            st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank], epoch + static_cast<uint32_t>(k) + 1u);
+        }
+    }
+}
+
+}  // namespace stdml::collective::cuda

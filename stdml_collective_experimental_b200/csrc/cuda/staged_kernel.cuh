@@ -43,6 +43,7 @@
 #pragma once
 #include "ar_kernel.cuh"
 #include "copy.cuh"
+#include "ring_sync.cuh"
 #include "staged_walk.hpp"
 
 #include <atomic>
@@ -90,16 +91,6 @@ struct TileDesc {
     unsigned int n, fast;
     int first, last;
 };
-
-__device__ __forceinline__ uint4 ld_shared_v4(uint32_t at)
-{
-    uint4 v;
-    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "r"(at)
-                 : "memory");
-    return v;
-}
 
 __device__ __forceinline__ void *generic_of(uint32_t at) { return __cvta_shared_to_generic(at); }
 
@@ -282,37 +273,6 @@ struct StagedBuffers {
     }
 };
 
-// One phase per round of something, on N barriers in turn: who waits for round k finds it although
-// up to N - 1 later ones are over too.
-template <int N>
-struct Phases {
-    unsigned long long bar[N];
-
-    __device__ __forceinline__ void init(unsigned int count)
-    {
-        for (int i = 0; i < N; ++i) { mbar_init(smem_addr(&bar[i]), count); }
-    }
-    __device__ __forceinline__ uint32_t at(int k) const { return smem_addr(&bar[k % N]); }
-    // (may sleep a while on a round that is not over)
-    __device__ __forceinline__ bool try_wait(int k) const
-    {
-        return mbar_try_wait(at(k), static_cast<uint32_t>(k / N & 1));
-    }
-    __device__ __forceinline__ bool over(int k) const
-    {
-        uint32_t done;
-        asm volatile("{\n\t"
-                     ".reg .pred p;\n\t"
-                     "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t"
-                     "}"
-                     : "=r"(done)
-                     : "r"(at(k)), "r"(static_cast<uint32_t>(k / N & 1))
-                     : "memory");
-        return done != 0;
-    }
-};
-
 // What the warps of a block share.
 struct StagedShared {
     TileDesc descs[kStagedDescs][kMaxRanks];
@@ -333,57 +293,6 @@ struct StagedShared {
     unsigned int starts[kStagedStarts];
 };
 static_assert(kStagedLag <= 3, "passes that the workers may be ahead of the warp that tells the peers");
-
-// Waits for round k of something.  False: the block gives up.
-template <int N>
-__device__ __forceinline__ bool staged_wait(const CommCtx &ctx, StagedShared &sh, const Phases<N> &phases, int k)
-{
-    unsigned long long t0 = 0;
-    for (unsigned int spins = 0; !phases.try_wait(k); ++spins) {
-        if (*static_cast<volatile int *>(&sh.dead) != 0) { return false; }
-        if ((spins & 63u) != 63u) { continue; }
-        const unsigned long long now = global_ns();
-        if (t0 == 0) { t0 = now; }
-        // (twice the limit of a wait for a peer's flag, of whose end `dead` tells)
-        if (now - t0 > 2 * ctx.timeout_ns || spins >= ctx.max_spins) {
-            *static_cast<volatile int *>(&sh.dead) = 1;
-            return false;
-        }
-    }
-    return true;
-}
-
-// A warp that gives up: its copies of round k in flight end before the block does.
-template <int N>
-__device__ __forceinline__ void drain(const CommCtx &ctx, const Phases<N> &phases, int k)
-{
-    if (k >= 0) { (void)mbar_wait(ctx, phases.at(k), static_cast<uint32_t>(k / N & 1), ctx.timeout_ns / 4); }
-}
-
-__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok ? 1 : 0) != 0; }
-
-// One lane of a worker warp for all of it.
-__device__ __forceinline__ void warp_arrive(uint32_t bar)
-{
-    __syncwarp();
-    if ((threadIdx.x & 31u) == 0u) { mbar_arrive(bar); }
-}
-
-// Asks for the first `bytes` bytes at src, of tensor memory, past the L2 as far as it can; every lane
-// of a barrier of 32 calls it.
-__device__ __forceinline__ void ask_stream(uint32_t bar, uint32_t dst, const void *src,
-                                           unsigned int bytes, unsigned long long policy)
-{
-    if (bytes == 0u) {
-        mbar_arrive(bar);
-        return;
-    }
-    mbar_expect_tx(bar, bytes);
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
-                 "[%0], [%1], %2, [%3], %4;" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar), "l"(policy)
-                 : "memory");
-}
 
 // The loader warp: a lane per shard finds the tensor of each of its tiles, a chain of dependent
 // loads, and asks for the tile's bytes as soon as the buffer is free.
@@ -445,7 +354,7 @@ __device__ __forceinline__ void staged_load(const CommCtx &ctx, const StagedArgs
             }
         }
         bool ok = true;
-        if (k > 0 && k < a.rounds) { ok = warp_agrees(staged_wait(ctx, sh, sh.packed, k - 1)); }
+        if (k > 0 && k < a.rounds) { ok = warp_agrees(ring_wait(ctx, sh.dead, sh.packed, k - 1)); }
         if (ok && k < a.rounds) {
             if (s < world) { sh.descs[k % kStagedDescs][s] = d; }
             const bool whole = warp_agrees(s >= world || d.fast == 1u << a.tile_shift);
@@ -455,7 +364,7 @@ __device__ __forceinline__ void staged_load(const CommCtx &ctx, const StagedArgs
         // The own tiles, the first two of them at once: pass k - 1 reduced the one that was in the buffer.
         const int t = k < 2 ? k : k - kStagedLag + 1;
         if (ok && t < a.rounds && (k < 2 || t >= 2)) {
-            ok = k < 2 || warp_agrees(staged_wait(ctx, sh, sh.reduced, k - 1));
+            ok = k < 2 || warp_agrees(ring_wait(ctx, sh.dead, sh.reduced, k - 1));
             if (ok && s == rank) {
                 const TileDesc &o = sh.descs[t % kStagedDescs][rank];
                 ask_stream(sh.own.at(t), bufs.own(t), o.src, o.fast * unit, policy);
@@ -466,25 +375,6 @@ __device__ __forceinline__ void staged_load(const CommCtx &ctx, const StagedArgs
             drain(ctx, sh.tensor, k - 1 < a.rounds ? k - 1 : a.rounds - 1);
             for (int i = 1; i <= 2; ++i) { drain(ctx, sh.own, t - i < a.rounds ? t - i : -1); }
             return;
-        }
-    }
-}
-
-// The teller: lets the peers know what the passes have stored.  A warp of its own: its fences wait for
-// all of the block's stores.  Over links and within a GPU alike they and the flags' way take
-// longer than a pass, hence the lag.
-__device__ __forceinline__ void staged_tell(const CommCtx &ctx, const StagedArgs &a, StagedShared &sh, int rank)
-{
-    const int p = static_cast<int>(threadIdx.x & 31u);
-    const int passes = a.rounds + kStagedLag;
-    for (int k = 0; k < passes; ++k) {
-        if (!warp_agrees(staged_wait(ctx, sh, sh.reduced, k))) { return; }
-        // (one fence for all that are over by now)
-        while (k + 1 < passes && warp_agrees(sh.reduced.over(k + 1))) { ++k; }
-        fence_ranks(ctx);
-        fence_async_proxy_global();  // the peers read it by bulk copies
-        if (p < ctx.world) {
-            st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank], sh.epoch + static_cast<uint32_t>(k) + 1u);
         }
     }
 }
@@ -512,7 +402,7 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
         const unsigned int all_res = __reduce_add_sync(0xffffffffu, n_res);
         const char *from_op = theirs + walk.piece(t, rank), *from_res = mine + walk.piece(u < 0 ? 0 : u, peer ? p : rank);
         const uint32_t to_op = bufs.operand(p, t), to_res = bufs.result(p);
-        bool ok = !reduces || t < 2 || staged_wait(ctx, sh, sh.reduced, t - 2 + kStagedLag);
+        bool ok = !reduces || t < 2 || ring_wait(ctx, sh.dead, sh.reduced, t - 2 + kStagedLag);
         if (ok && p < ctx.world) { ok = poll_acquire(ctx, rank, p, sh.epoch + static_cast<uint32_t>(t) + 1u, 0); }
         ok = warp_agrees(ok);
         if (ok && reduces) {
@@ -520,7 +410,7 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
             if (peer && n_op != 0u) { bulk_load(to_op, from_op, n_op, sh.operands.at(t)); }
         }
         if (ok && unpacks) {
-            ok = u < 1 || warp_agrees(staged_wait(ctx, sh, sh.unpacked, u - 1));
+            ok = u < 1 || warp_agrees(ring_wait(ctx, sh.dead, sh.unpacked, u - 1));
             if (ok && p == 0) { mbar_expect_tx(sh.results.at(u), all_res); }
             if (ok && n_res != 0u) { bulk_load(to_res, from_res, n_res, sh.results.at(u)); }
         }
@@ -588,7 +478,7 @@ template <int DT>
 __device__ __forceinline__ bool staged_pack(const CommCtx &ctx, const StagedArgs &a, StagedShared &sh, uint32_t smem,
                                             int k)
 {
-    if (!staged_wait(ctx, sh, sh.tensor, k)) { return false; }
+    if (!ring_wait(ctx, sh.dead, sh.tensor, k)) { return false; }
     const StagedWorker<DT> w(ctx, a, sh, smem);
     char *to = ctx.base[w.rank] + a.off + w.walk().piece(k, 0);
     if (sh.whole[k % kStagedDescs] != 0) {
@@ -649,7 +539,7 @@ template <int DT, int OP>
 __device__ __forceinline__ bool staged_reduce(const CommCtx &ctx, const StagedArgs &a, StagedShared &sh, uint32_t smem,
                                               int t)
 {
-    if (!staged_wait(ctx, sh, sh.operands, t) || !staged_wait(ctx, sh, sh.own, t)) { return false; }
+    if (!ring_wait(ctx, sh.dead, sh.operands, t) || !ring_wait(ctx, sh.dead, sh.own, t)) { return false; }
     const StagedWorker<DT> w(ctx, a, sh, smem);
     const unsigned long long policy = evict_first_policy();
     const TileDesc &d = sh.descs[t % kStagedDescs][w.rank];
@@ -685,7 +575,7 @@ template <int DT>
 __device__ __forceinline__ bool staged_unpack(const CommCtx &ctx, const StagedArgs &a, StagedShared &sh, uint32_t smem,
                                               int t)
 {
-    if (!staged_wait(ctx, sh, sh.results, t)) { return false; }
+    if (!ring_wait(ctx, sh.dead, sh.results, t)) { return false; }
     const StagedWorker<DT> w(ctx, a, sh, smem);
     const unsigned long long policy = evict_first_policy();
     const TileDesc *ds = sh.descs[t % kStagedDescs];
@@ -757,7 +647,7 @@ __global__ void __launch_bounds__(kStagedBlock, kStagedMinPerSm)
     if (tid >= kStagedThreads) {
         const int role = (tid - kStagedThreads) / 32;
         if (role == 0) { staged_load<DT>(ctx, a, sh, walk, bufs, vr); }
-        if (role == 1) { staged_tell(ctx, a, sh, rank); }
+        if (role == 1) { ring_tell(ctx, sh.dead, sh.epoch, sh.reduced, rank, a.rounds + kStagedLag); }
         if (role == 2) { staged_fetch(ctx, a, sh, walk, bufs, stores); }
         return;
     }

@@ -3,6 +3,7 @@
 // the buffer exactly once, and the descriptor-table search lands on the tensor
 // that holds a vector.  compute-sanitizer is not available for the device
 // code, so the arithmetic that decides every address is exercised here.
+#include <bit>
 #include <cstdio>
 #include <cstring>
 #include <random>
@@ -101,26 +102,35 @@ int main()
         const size_t stride = bytes + rng() % 40;
         const int world = 2 + static_cast<int>(rng() % 15);
         const size_t slot = (size_t{4096} << (rng() % 15)) + 4096;
-        const int most = 1 + static_cast<int>(rng() % 300);
-        const PullGeometry g = pull_geometry(trial % 2 == 0 ? 1 : world - 1, bytes, slot, most);
-        EXPECT(g.blocks <= most && g.tile_shift >= kPullStepShift);
+        const int sms = 1 + static_cast<int>(rng() % 148), rows = trial % 5 < 3 ? world : 1;
+        const int want = trial % 7 == 0 ? 1 + static_cast<int>(rng() % 300) : 0;
+        const int sources = pull_sources(world, trial % 2 == 0 ? 0 : -1);
+        const PullGeometry g = pull_geometry(sources, bytes, slot, sms, rows, want);
+        EXPECT((g.blocks - 1) * rows < (g.lng ? kPullLongPerSm : kPullPerSm) * sms && (want == 0 || g.blocks <= want));
+        EXPECT(g.tile % 32 == 0 && g.tile > 0);
         if (g.blocks == 0) {
             EXPECT(slot < (static_cast<size_t>(kPullRing) << kPullStepShift) * 16);
             continue;
         }
-        const unsigned long long ring = (static_cast<unsigned long long>(kPullRing) << g.tile_shift) * 16;
+        if (g.lng) {
+            EXPECT(g.ring == kPullLongRing && pull_long_smem(sources, g.tile) <= kPullLongSmem);
+        } else {
+            EXPECT(g.ring == kPullRing && (g.tile & (g.tile - 1)) == 0 && g.tile >= 1u << kPullStepShift);
+        }
+        const unsigned long long piece = g.tile * 16ull, ring = piece * g.ring;
         EXPECT(ring * g.blocks == g.ring_bytes() && g.ring_bytes() <= slot);
         unsigned long long expect = 0;
         for (int k = 0; k < g.rounds; ++k) {
             for (int b = 0; b < g.blocks; ++b) {
-                const PullWalk w{bytes, stride, g.blocks, b, g.tile_shift};
-                EXPECT(w.first_vector(k) == expect);
-                expect += 1ull << g.tile_shift;
-                EXPECT(w.piece(k) == ring * b + (k % kPullRing) * (ring / kPullRing));
+                const PullWalk w{{bytes, stride}, g.blocks, b, std::bit_width(g.tile) - 1};
+                const PullLongWalk l{{bytes, stride}, g.blocks, b, g.tile};
+                EXPECT((g.lng ? l.first_vector(k) : w.first_vector(k)) == expect);
+                expect += g.tile;
+                EXPECT((g.lng ? l.piece(k) : w.piece(k)) == ring * b + (k % g.ring) * piece);
             }
         }
         for (int p = 0; p < world; ++p) {
-            const PullWalk w{bytes, stride, g.blocks, 0, g.tile_shift};
+            const PullLayout w{bytes, stride};
             EXPECT(w.phase(p) == p * stride % 16);
             EXPECT(expect >= w.vectors(w.phase(p)));
             EXPECT((w.vectors(w.phase(p)) - 1) * 16 < bytes + w.phase(p));

@@ -596,6 +596,31 @@ def test_pull_ring_at_every_alignment(tuned, n, shift):
         assert torch.equal(ins[r].cpu(), host[0]), r
 
 
+@pytest.mark.parametrize("world,root", [(2, None), (3, 1), (8, None), (8, 7), (9, None)])
+def test_long_pull_at_the_edges_of_its_rounds(world, root):
+    """Messages from the smallest of the long kernel's on, one vector around whole rounds, destinations at
+    odd bytes; a ninth rank, whose messages are none of them."""
+    per_rank = 2 * 148 // world
+    with DeviceSession.loopback(world, heap_bytes=1 << 20, staging_bytes=64 << 20) as s:
+        for n in (512 * per_rank * 16 - 33, 512 * per_rank * 16, 1600 * per_rank * 16 + 17, 5_000_003):
+            for shift in (0, 3, 16):
+                ins = [torch.randint(0, 255, (n + 32,), dtype=torch.uint8, device="cuda")[shift:n + shift]
+                       for _ in range(world)]
+                total = n if root is not None else n * world
+                out = [torch.full((total + 64,), 7, dtype=torch.uint8, device="cuda") for _ in range(world)]
+                views = [o[shift:total + shift] for o in out]
+                if root is None:
+                    s.all_gather(ins, views)
+                else:
+                    s.broadcast(ins, out=views, root=root)
+                torch.cuda.synchronize()
+                s.check()
+                want = torch.cat(ins) if root is None else ins[root]
+                for o, v in zip(out, views):
+                    assert torch.equal(v, want), (n, shift)
+                    assert bool((o[:shift] == 7).all()) and bool((o[total + shift:] == 7).all())
+
+
 @pytest.mark.parametrize("push", [False, True])
 @pytest.mark.parametrize("n", [17, 70_001, 3_000_001])
 def test_ranks_without_a_destination_take_part(sess, n, push):
