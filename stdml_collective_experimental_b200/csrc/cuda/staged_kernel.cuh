@@ -175,6 +175,22 @@ __device__ __forceinline__ SlowVec slow_vec(const StagedArgs &a, int vr, const u
     return s;
 }
 
+// The elements of a vector that is not whole, eight at a time: one after the other they cost a memory latency
+// each (187 ragged bf16 tensors, 3 ranks 22.7 us, so 19.6; four at a time 20.6).
+template <int N, typename Load, typename Store>
+__device__ __forceinline__ void copy_elements(Load load, Store store)
+{
+    constexpr int B = N < 8 ? N : 8;
+#pragma unroll 1
+    for (int i = 0; i < N; i += B) {
+        decltype(load(0)) x[B];
+#pragma unroll
+        for (int j = 0; j < B; ++j) { x[j] = load(i + j); }
+#pragma unroll
+        for (int j = 0; j < B; ++j) { store(i + j, x[j]); }
+    }
+}
+
 // The vector in the wire type, to `to` (elements past the tensor's end: zero).
 template <int DT>
 __device__ __forceinline__ void slow_load(const SlowVec &s, bool user_f32, void *to)
@@ -195,8 +211,8 @@ __device__ __forceinline__ void slow_load(const SlowVec &s, bool user_f32, void 
                 }
                 return;
             }
-#pragma unroll 1
-            for (int i = 0; i < N; ++i) { out[i] = s.first + i < s.count ? Tr<DT>::narrow(f[i]) : S(0); }
+            copy_elements<N>([&](int i) { return s.first + i < s.count ? Tr<DT>::narrow(f[i]) : S(0); },
+                             [&](int i, S x) { out[i] = x; });
             return;
         }
     }
@@ -205,8 +221,7 @@ __device__ __forceinline__ void slow_load(const SlowVec &s, bool user_f32, void 
         *reinterpret_cast<uint4 *>(out) = *reinterpret_cast<const uint4 *>(p);
         return;
     }
-#pragma unroll 1
-    for (int i = 0; i < N; ++i) { out[i] = s.first + i < s.count ? p[i] : S(0); }
+    copy_elements<N>([&](int i) { return s.first + i < s.count ? p[i] : S(0); }, [&](int i, S x) { out[i] = x; });
 }
 
 // A vector of the wire type in shared memory to the tensor.
@@ -230,8 +245,10 @@ __device__ __forceinline__ void slow_store(const SlowVec &s, bool user_f32, cons
                 }
                 return;
             }
-#pragma unroll 1
-            for (int i = 0; i < n; ++i) { f[i] = Tr<DT>::widen(in[i]); }
+            copy_elements<N>([&](int i) { return in[i]; },
+                             [&](int i, S x) {
+                                 if (i < n) { f[i] = Tr<DT>::widen(x); }
+                             });
             return;
         }
     }
@@ -240,8 +257,10 @@ __device__ __forceinline__ void slow_store(const SlowVec &s, bool user_f32, cons
         *reinterpret_cast<uint4 *>(p) = *reinterpret_cast<const uint4 *>(in);
         return;
     }
-#pragma unroll 1
-    for (int i = 0; i < n; ++i) { p[i] = in[i]; }
+    copy_elements<N>([&](int i) { return in[i]; },
+                     [&](int i, S x) {
+                         if (i < n) { p[i] = x; }
+                     });
 }
 
 constexpr int kStagedUnroll = 4;  // vectors of a worker in flight, shared memory to global
