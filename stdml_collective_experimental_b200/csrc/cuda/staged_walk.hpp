@@ -50,7 +50,9 @@ struct StagedWalk {
 struct StagedGeometry {
     int blocks = 0;  // 0: the slot cannot hold the ring of even one block
     int tile_shift = kStagedMinShift, rounds = 1;
-    bool full = false;  // the slot holds the rings of as many blocks as there may be
+    // A message longer than the slot goes round in it in one launch: the slot holds the rings of as many blocks
+    // as there may be.
+    bool full = false;
 };
 
 // Grid and tile for `nvec` vectors on `num_sms` SMs that `vranks` ranks share.  A tile is kStagedRoundVec
@@ -74,22 +76,33 @@ inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_byt
         const int resident = std::min(kMaxBlocks, staged_per_sm(world, shift, user_f32) * num_sms / vranks);
         return static_cast<size_t>(std::max(1, want_blocks > 0 ? std::min(want_blocks, resident) : resident));
     };
+    const auto tiles_of = [&](int shift) { return (longest + (size_t{1} << shift) - 1) >> shift; };
+    // The slot holds the rings of all blocks that have a tile of this size.
+    const auto fits = [&](int shift) { return ring_bytes(shift) * std::min(tiles_of(shift), most(shift)) <= staging_bytes; };
+    // No block goes without a ring for the sake of larger tiles.  161 f32 tensors of 102 MB, us, with tiles of up
+    // to 256 vectors in as many blocks as the slot holds / so: 4 ranks, slots of 8 MB 413 / 304, of 4 MB 664 / 451; 8 ranks,
+    // 4 MB 856 / 616.  Where the smallest tiles do not fit either, fewer blocks with larger ones: 8 ranks, 1 MB
+    // 2471 / 2689 in the smallest.
+    const bool cramped = !fits(kStagedMinShift);
     const size_t want = std::max<size_t>(kStagedRoundVec / static_cast<size_t>(world), size_t{1} << kStagedMinShift);
     const auto good = [&](int shift) {
         const size_t tile = size_t{1} << shift;
         if (tile > want || staged_smem(world, shift, user_f32) > kStagedSmem) { return false; }
+        if (cramped ? tile > 256 || ring_bytes(shift) > staging_bytes : !fits(shift)) { return false; }
         // A short message has fewer blocks, not smaller tiles than about a vector per worker, and larger ones
         // rather than a second round (a set of ragged tensors pays several memory latencies per vector: 224 of
         // them, 4 ranks, 20.6 us with 256 vectors at least, 14.5 so).
-        if (tile <= kStagedThreads && tile * (world - 1) <= 256) { return ring_bytes(shift) <= staging_bytes; }
-        if (tile <= 256) { return tile / 2 * most(shift - 1) < longest && ring_bytes(shift) <= staging_bytes; }
-        return tile * most(shift) <= longest && ring_bytes(shift) * most(shift) <= staging_bytes;
+        if (tile <= kStagedThreads && tile * (world - 1) <= 256) { return true; }
+        if (tile <= 256) { return tile / 2 * most(shift - 1) < longest; }
+        return tile * most(shift) <= longest;
     };
     while (good(g.tile_shift + 1)) { ++g.tile_shift; }
-    const size_t tiles = (longest + (size_t{1} << g.tile_shift) - 1) >> g.tile_shift;
+    const size_t tiles = tiles_of(g.tile_shift);
     const size_t fit = staging_bytes / ring_bytes(g.tile_shift);
     g.blocks = static_cast<int>(std::min<size_t>({tiles, most(g.tile_shift), fit}));
-    g.full = fit >= most(g.tile_shift);
+    // Rounds of 64 vectors cost more than a launch per slot (2 ranks, slots of 2 MB: 798 us, 622 so; 128 vectors, 4 MB:
+    // 406, 411 so).
+    g.full = fit >= most(g.tile_shift) && static_cast<size_t>(world) << g.tile_shift > 64;
     if (g.blocks > 0) { g.rounds = static_cast<int>((tiles + g.blocks - 1) / g.blocks); }
     return g;
 }

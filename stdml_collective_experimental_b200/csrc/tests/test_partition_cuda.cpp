@@ -80,6 +80,14 @@ int main()
         std::vector<unsigned long long> bound(world + 1);
         for (int s = 0; s <= world; ++s) { bound[s] = StagedWalk::shard_begin(nvec, world, s); }
         EXPECT(bound[0] == 0 && bound[world] == nvec);
+        // no block goes without a ring for the sake of larger tiles, if the smallest would do
+        unsigned long long longest = 0;
+        for (int s = 0; s < world; ++s) { longest = std::max(longest, bound[s + 1] - bound[s]); }
+        const unsigned long long tiles = (longest + (1ull << g.tile_shift) - 1) >> g.tile_shift;
+        const int most = std::max(1, std::min(per_sm * sms / rows, kMaxBlocks));
+        const unsigned long long ring32 = (static_cast<unsigned long long>(kStagedRing) * world << kStagedMinShift) * 16;
+        EXPECT(g.blocks == std::min<unsigned long long>(tiles, want > 0 ? std::min(want, most) : most) ||
+               ring32 * std::min<unsigned long long>((longest + 31) / 32, kStagedMinPerSm * sms / rows) > slot);
         for (int s = 0; s < world; ++s) {
             unsigned long long expect = bound[s];
             for (int k = 0; k < g.rounds; ++k) {
@@ -93,6 +101,13 @@ int main()
                 }
             }
             EXPECT(expect == bound[s + 1]);
+        }
+    }
+    // 102 MB go round in slots far smaller than that in one launch, in as many blocks as are resident
+    for (const int world : {2, 3, 4, 8}) {
+        for (const size_t mb : {4, 8, 16, 32, 64}) {
+            const StagedGeometry g = staged_geometry(world, 102'000'000 / 16, mb << 20, 148, world, 0, false);
+            EXPECT(g.full && g.blocks == kStagedMinPerSm * 148 / world);
         }
     }
     // pull: over blocks and rounds the tiles cover the vectors of every rank's block exactly
