@@ -163,6 +163,7 @@ constexpr int kPullLongBlock = kPullLongThreads + 128;  // and a warp each that 
 constexpr int kPullLongPerSm = 2;
 constexpr int kPullLongSources = 7;
 constexpr size_t kPullLongMin = 512;  // vectors per block, at least
+constexpr unsigned int kPullLongMinTile = 256;
 constexpr int kPullLag = 6;
 constexpr int kPullDepth = 2;  // rounds of ring pieces in shared memory
 constexpr int kPullLongRing = 2 * kPullLag + 1;

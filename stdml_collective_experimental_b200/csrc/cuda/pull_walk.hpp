@@ -91,12 +91,14 @@ inline PullGeometry pull_geometry(int sources, size_t bytes, size_t staging_byte
     g.lng = true;
     g.ring = kPullLongRing;
     most = resident(kPullLongPerSm);
-    g.tile = pull_long_tile(sources);
+    // The largest tile of which the slot holds the rings of all blocks.  Broadcast of 94 MB, us, pull_kernel / so: 4 ranks,
+    // tiles of 256 vectors (slots of 4 MB) 462 / 315, of 128 (2 MB) 508 / 621; 2 ranks, 512 (16 MB) 136 / 88, 256 (8 MB)
+    // 220 / 160, 128 (4 MB) 246 / 311; 3 ranks, 192 (4 MB) 331 / 348; all_gather of 8 x 2.47 MB, 256 (2 MB) 57 / 46,
+    // 128 (1 MB) 62 both.
+    g.tile = static_cast<unsigned int>(
+        std::min<size_t>(pull_long_tile(sources), staging_bytes / (kPullLongRing * 16 * most) / 32 * 32));
+    if (sources > kPullLongSources || nvec < kPullLongMin * most || g.tile < kPullLongMinTile) { return s; }
     lay_out();
-    if (sources > kPullLongSources || nvec < kPullLongMin * most ||
-        staging_bytes < static_cast<size_t>(g.ring) * g.tile * 16 * most) {
-        return s;
-    }
     g.blocks = static_cast<int>(most);
     // tiles of equal size that just fill their rounds
     const size_t per_round = static_cast<size_t>(g.rounds) * g.blocks;

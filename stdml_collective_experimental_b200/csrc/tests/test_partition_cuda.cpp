@@ -132,6 +132,11 @@ int main()
         } else {
             EXPECT(g.ring == kPullRing && (g.tile & (g.tile - 1)) == 0 && g.tile >= 1u << kPullStepShift);
         }
+        // a smaller slot gives the long kernel smaller tiles, before it takes it away
+        const size_t resident = std::max(1, std::min(want > 0 ? want : kMaxBlocks, kPullLongPerSm * sms / rows));
+        if (pull_geometry(sources, bytes, size_t{1} << 40, sms, rows, want).lng) {
+            EXPECT(g.lng == (slot >= resident * kPullLongRing * kPullLongMinTile * 16));
+        }
         const unsigned long long piece = g.tile * 16ull, ring = piece * g.ring;
         EXPECT(ring * g.blocks == g.ring_bytes() && g.ring_bytes() <= slot);
         unsigned long long expect = 0;
