@@ -9,6 +9,7 @@
 #include <mutex>
 #include <new>
 #include <stdexcept>
+#include <utility>
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -199,6 +200,8 @@ class World final : public DeviceWorld
     int debug_inject_ = 0;  // tests: hand the next all_reduce kernel arguments that its
                             // own checks must refuse (1: misaligned offset, 2: offset
                             // inside the signal pad); implies debug_checks for that launch
+    int debug_absent_ = 0;  // tests (loopback): the last ranks, so many, take no part in the next call through
+                            // a ring; the waits of the others run out
     unsigned long long wait_timeout_ns_;
 
   public:
@@ -440,6 +443,11 @@ class World final : public DeviceWorld
             debug_checks_ = value != 0;
         } else if (name == "debug_inject") {
             debug_inject_ = static_cast<int>(value);
+        } else if (name == "debug_absent") {
+            if (!opt_.loopback || value < 0 || value >= vranks_) {
+                throw std::invalid_argument("debug_absent: loopback world and fewer ranks than it has");
+            }
+            debug_absent_ = static_cast<int>(value);
         } else {
             throw std::invalid_argument("device world: unknown knob '" + name + "'");
         }
@@ -893,6 +901,9 @@ class World final : public DeviceWorld
                staged_geometry(opt_.world, nvec, opt_.staging_bytes, num_sms_, vranks_, 0, user_f32).full;
     }
 
+    // Grid rows of the next kernel that goes through a ring.
+    int ring_rows() { return vranks_ - std::exchange(debug_absent_, 0); }
+
     // Peer-load two-shot of memory outside the arena: rounds over a small ring.
     int all_reduce_staged(const AllReduceCall &c, size_t nvec, int user_dt, void *stream)
     {
@@ -920,7 +931,7 @@ class World final : public DeviceWorld
         if (g.blocks == 0) { return -1; }
         a.tile_shift = g.tile_shift;
         a.rounds = g.rounds;
-        const int rc = launch_staged(make_ctx(), a, c.dt, c.op, g.blocks, vranks_, stream);
+        const int rc = launch_staged(make_ctx(), a, c.dt, c.op, g.blocks, ring_rows(), stream);
         if (rc < 0) { throw std::invalid_argument("all_reduce: (dtype, op) not built"); }
         return rc;
     }
@@ -1009,7 +1020,7 @@ class World final : public DeviceWorld
         a.tile_shift = std::bit_width(geo.tile) - 1;
         a.rounds = geo.rounds;
         a.lng = geo.lng ? 1 : 0;
-        return launch_pull(make_ctx(), a, geo.blocks, vranks_, stream);
+        return launch_pull(make_ctx(), a, geo.blocks, ring_rows(), stream);
     }
 
     int gather(const GatherCall &c, void *stream) override

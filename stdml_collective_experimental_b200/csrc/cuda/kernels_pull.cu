@@ -291,8 +291,6 @@ struct PullLong {
             const unsigned long long last = first + 16ull * n + (at != first ? 16ull : 0ull);
             const unsigned long long hi = last < end ? last : end;
             if (k >= 2 && !ring_wait(ctx, sh.dead, sh.packed, k - 2)) {
-                // its copies in flight end before the block does
-                drain(ctx, sh.tensor, k - 2);
                 drain(ctx, sh.tensor, k - 1);
                 return;
             }
@@ -317,7 +315,7 @@ struct PullLong {
             if (ok && i < ctx.world) { ok = poll_acquire(ctx, rank, i, sh.epoch + static_cast<uint32_t>(t) + 1u, 0); }
             if (!warp_agrees(ok)) {
                 *static_cast<volatile int *>(&sh.dead) = 1;
-                for (int j = 1; j <= kPullDepth; ++j) { drain(ctx, sh.pieces, t - j < a.rounds ? t - j : -1); }
+                drain(ctx, sh.pieces, (t < a.rounds ? t : a.rounds) - 1);
                 return;
             }
             if (!more) { continue; }

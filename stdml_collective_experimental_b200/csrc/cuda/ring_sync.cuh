@@ -66,11 +66,14 @@ __device__ __forceinline__ bool ring_wait(const CommCtx &ctx, int &dead, const P
     return true;
 }
 
-// A warp that gives up: its copies of round k in flight end before the block does.
+// A warp that gives up: its copies in flight end before the block does.  `last`: the last round that it has
+// asked for (-1: none), which up to N - 1 before it may still be under way with.
 template <int N>
-__device__ __forceinline__ void drain(const CommCtx &ctx, const Phases<N> &phases, int k)
+__device__ __forceinline__ void drain(const CommCtx &ctx, const Phases<N> &phases, int last)
 {
-    if (k >= 0) { (void)mbar_wait(ctx, phases.at(k), static_cast<uint32_t>(k / N & 1), ctx.timeout_ns / 4); }
+    for (int k = last; k >= 0 && k > last - N; --k) {
+        (void)mbar_wait(ctx, phases.at(k), static_cast<uint32_t>(k / N & 1), ctx.timeout_ns / 4);
+    }
 }
 
 __device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok ? 1 : 0) != 0; }

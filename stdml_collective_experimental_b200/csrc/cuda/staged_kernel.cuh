@@ -338,6 +338,7 @@ __device__ __forceinline__ void staged_load(const CommCtx &ctx, const StagedArgs
         }
         return lo;
     };
+    int asked = -1, asked_own = -1;  // last rounds asked for
     for (int k = 0; k < a.rounds + kStagedLag - 1 || k < 2; ++k) {
         TileDesc d;
         d.src = nullptr;
@@ -379,6 +380,7 @@ __device__ __forceinline__ void staged_load(const CommCtx &ctx, const StagedArgs
             const bool whole = warp_agrees(s >= world || d.fast == 1u << a.tile_shift);
             if (s == 0) { sh.whole[k % kStagedDescs] = whole ? 1 : 0; }
             ask_stream(sh.tensor.at(k), bufs.tensor(s), d.src, s != rank ? d.fast * unit : 0u, policy);
+            asked = k;
         }
         // The own tiles, the first two of them at once: pass k - 1 reduced the one that was in the buffer.
         const int t = k < 2 ? k : k - kStagedLag + 1;
@@ -388,11 +390,11 @@ __device__ __forceinline__ void staged_load(const CommCtx &ctx, const StagedArgs
                 const TileDesc &o = sh.descs[t % kStagedDescs][rank];
                 ask_stream(sh.own.at(t), bufs.own(t), o.src, o.fast * unit, policy);
             }
+            if (ok) { asked_own = t; }
         }
         if (!ok) {
-            // its copies in flight end before the block does (for a round not asked for the wait just runs out)
-            drain(ctx, sh.tensor, k - 1 < a.rounds ? k - 1 : a.rounds - 1);
-            for (int i = 1; i <= 2; ++i) { drain(ctx, sh.own, t - i < a.rounds ? t - i : -1); }
+            drain(ctx, sh.tensor, asked);
+            drain(ctx, sh.own, asked_own);
             return;
         }
     }
@@ -435,8 +437,8 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
         }
         if (!ok) {
             *static_cast<volatile int *>(&sh.dead) = 1;
-            // its copies in flight end before the block does (of a round not asked for the wait just runs out)
-            for (int i = 0; i <= 2; ++i) { drain(ctx, sh.operands, t - i < a.rounds ? t - i : -1); }
+            // (of a round not asked for the wait just runs out)
+            drain(ctx, sh.operands, t < a.rounds ? t : a.rounds - 1);
             if (stores) { drain(ctx, sh.results, u - 1); }
             return;
         }

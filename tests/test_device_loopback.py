@@ -879,6 +879,49 @@ def test_bounded_wait_reports_and_recovers():
         s.close()
 
 
+@pytest.mark.parametrize("call", ["all_reduce", "all_gather", "broadcast"])
+def test_ring_kernels_give_up(call):
+    """The last rank takes no part in a call of many rounds: the waits for its flag run out, every warp
+    leaves, the host reads which rank was missing, and after recover() the same call gets through."""
+    w, n = 3, 3_000_001
+    with DeviceSession.loopback(w, heap_bytes=1 << 20, staging_bytes=32 << 20, wait_timeout_ms=200) as s:
+        host = make_inputs(w, n, torch.float32, seed=9)
+        ins = [h.cuda() for h in host]
+        out = [torch.zeros(n * w if call == "all_gather" else n, device="cuda") for _ in range(w)]
+
+        def run():
+            if call == "all_reduce":
+                s.all_reduce(ins, out=out)
+            elif call == "all_gather":
+                s.all_gather(ins, out)
+            else:
+                s.broadcast(ins, out=out, root=0)
+
+        run()
+        torch.cuda.synchronize()
+        s.check()
+        s.set_knob("debug_absent", 1)
+        ends = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        ends[0].record()
+        run()
+        ends[1].record()
+        torch.cuda.synchronize()
+        code, rank, block, peer, phase, want, have = s.status()
+        assert code == 1 and rank in (0, 1) and peer == 2 and phase == 0 and want == have + 1
+        assert 200 < ends[0].elapsed_time(ends[1]) < 300
+        with pytest.raises(DeviceTimeoutError):
+            run()
+        s.recover()
+        for o in out:
+            o.zero_()
+        run()
+        torch.cuda.synchronize()
+        s.check()
+        want = {"all_reduce": reduce_many(host, "sum"), "all_gather": torch.cat(host), "broadcast": host[0]}[call]
+        for r in range(w):
+            assert same(out[r].cpu(), want) and same(ins[r].cpu(), host[r]), r
+
+
 def test_profile_summary_counts_device_time(sess):
     sess.enable_profile()
     x = [torch.ones(100_000, device="cuda") for _ in range(sess.world)]
