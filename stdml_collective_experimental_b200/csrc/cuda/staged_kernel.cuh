@@ -415,6 +415,7 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
         const StagedTile tile = walk.tile_of(s, t);
         return static_cast<unsigned int>(tile.hi - tile.lo) * 16u;
     };
+    int asked_op = -1, asked_res = -1;  // last rounds asked for
     for (int t = 0; t < passes; ++t) {
         const int u = t - kStagedLag;
         const bool reduces = t < a.rounds, unpacks = u >= 0 && stores;
@@ -429,17 +430,18 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
         if (ok && reduces) {
             if (p == 0) { mbar_expect_tx(sh.operands.at(t), n_op * bufs.others); }
             if (peer && n_op != 0u) { bulk_load(to_op, from_op, n_op, sh.operands.at(t)); }
+            asked_op = t;
         }
         if (ok && unpacks) {
             ok = u < 1 || warp_agrees(ring_wait(ctx, sh.dead, sh.unpacked, u - 1));
             if (ok && p == 0) { mbar_expect_tx(sh.results.at(u), all_res); }
             if (ok && n_res != 0u) { bulk_load(to_res, from_res, n_res, sh.results.at(u)); }
+            if (ok) { asked_res = u; }
         }
         if (!ok) {
             *static_cast<volatile int *>(&sh.dead) = 1;
-            // (of a round not asked for the wait just runs out)
-            drain(ctx, sh.operands, t < a.rounds ? t : a.rounds - 1);
-            if (stores) { drain(ctx, sh.results, u - 1); }
+            drain(ctx, sh.operands, asked_op);
+            drain(ctx, sh.results, asked_res);
             return;
         }
     }

@@ -908,7 +908,8 @@ def test_ring_kernels_give_up(call):
         torch.cuda.synchronize()
         code, rank, block, peer, phase, want, have = s.status()
         assert code == 1 and rank in (0, 1) and peer == 2 and phase == 0 and want == have + 1
-        assert 200 < ends[0].elapsed_time(ends[1]) < 300
+        # (a warp that waited for copies that it never asked for would add a quarter of the timeout)
+        assert 200 < ends[0].elapsed_time(ends[1]) < 235
         with pytest.raises(DeviceTimeoutError):
             run()
         s.recover()
