@@ -57,14 +57,16 @@ enum : int {
     kStatusBadArgs = 2,    // launch arguments failed the kernel's own checks
 };
 
+constexpr int kPhaseRing = 128;  // a wait between the warps of a block (ring_sync.cuh); `want` is the round
+
 struct StatusBlock {
     int code;      // first failure wins (atomicCAS from 0)
     int rank;      // rank that observed it
     int block;     // blockIdx.x
-    int peer;      // peer whose flag was missing (timeout)
+    int peer;      // peer whose flag was missing (timeout); -1: a wait inside the block
     unsigned int want;  // flag value waited for
     unsigned int have;  // flag value last seen
-    int phase;     // barrier ordinal inside the kernel
+    int phase;     // barrier ordinal inside the kernel, or kPhaseRing
     int pad;
 };
 

@@ -194,8 +194,8 @@ void DeviceSession::check()
     }
     if (s.code != 0) {
         throw DeviceTimeout("device collective gave up: rank " + std::to_string(s.rank) +
-                                " block " + std::to_string(s.block) + " waited for rank " +
-                                std::to_string(s.peer) + " (barrier " + std::to_string(s.phase) +
+                                " block " + std::to_string(s.block) + " waited for " +
+                                (s.peer < 0 ? "its own copies or warps" : "rank " + std::to_string(s.peer)) + " (barrier " + std::to_string(s.phase) +
                                 ", want " + std::to_string(s.want) + ", have " +
                                 std::to_string(s.have) + "); call recover() on every rank",
                             s);

@@ -207,6 +207,7 @@ struct PullShared {
     Phases<2> packed;
     Phases<kPullDepth> stored;
     Phases<8> done;  // passes: tile k packed, tile k - lag here
+    Phases<1> left;  // workers and storer have come through
     uint32_t epoch;
     int dead;  // the block gives up
 };
@@ -314,7 +315,7 @@ struct PullLong {
                                                            : ring_wait(ctx, sh.dead, sh.done, before + kPullLag));
             if (ok && i < ctx.world) { ok = poll_acquire(ctx, rank, i, sh.epoch + static_cast<uint32_t>(t) + 1u, 0); }
             if (!warp_agrees(ok)) {
-                *static_cast<volatile int *>(&sh.dead) = 1;
+                ring_give_up(sh.dead);
                 drain(ctx, sh.pieces, (t < a.rounds ? t : a.rounds) - 1);
                 return;
             }
@@ -383,11 +384,17 @@ struct PullLong {
     // The storer: a lane per source takes its tiles on to the destination.
     __device__ __forceinline__ void store() const
     {
-        if (!stores || sources == 0) { return; }
+        if (!stores || sources == 0) {
+            warp_arrive(sh.left.at(0));
+            return;
+        }
         const int i = static_cast<int>(threadIdx.x & 31u);
         const unsigned long long policy = evict_first_policy();
         for (int t = 0; t < a.rounds; ++t) {
-            if (!warp_agrees(ring_wait(ctx, sh.dead, sh.pieces, t))) { break; }
+            if (!warp_agrees(ring_wait(ctx, sh.dead, sh.pieces, t))) {
+                asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+                return;
+            }
             if (i < sources) {
                 const Run run = run_of(source_at(i), t, piece(i, t));
                 if (run.n != 0u && run.alike()) {
@@ -409,6 +416,7 @@ struct PullLong {
             warp_arrive(sh.stored.at(t));
         }
         asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+        warp_arrive(sh.left.at(0));
     }
 
     __device__ __forceinline__ void work() const
@@ -433,6 +441,7 @@ struct PullLong {
                 warp_arrive(sh.stored.at(t));
             }
         }
+        warp_arrive(sh.left.at(0));
     }
 };
 
@@ -452,6 +461,7 @@ __global__ void __launch_bounds__(kPullLongBlock, kPullLongPerSm)
         sh.packed.init(kPullLongThreads / 32);
         sh.stored.init(kPullLongThreads / 32 + 1);
         sh.done.init(kPullLongThreads / 32);
+        sh.left.init(kPullLongThreads / 32 + 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_proxy();
     }
@@ -464,7 +474,7 @@ __global__ void __launch_bounds__(kPullLongBlock, kPullLongPerSm)
     } else if (tid < kPullLongThreads + 32) {
         pull.load();
     } else if (tid < kPullLongThreads + 64) {
-        ring_tell(ctx, sh.dead, sh.epoch, sh.done, pull.rank, told);
+        ring_tell(ctx, sh.dead, sh.epoch, sh.done, pull.rank, told, sh.left);
     } else if (tid < kPullLongThreads + 96) {
         pull.fetch(told);
     } else {

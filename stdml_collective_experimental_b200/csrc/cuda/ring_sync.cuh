@@ -47,7 +47,10 @@ struct Phases {
     }
 };
 
-// Waits for round k of something.  False: the block gives up (`dead`, in shared memory).
+// Waits for round k of something.  False: the block gives up.  `dead`, in shared memory, says why: 1, a peer's
+// flag did not come, which the poll has reported; kRanOut + k, this wait ran out (the teller reports it).
+constexpr int kRanOut = 2;
+
 template <int N>
 __device__ __forceinline__ bool ring_wait(const CommCtx &ctx, int &dead, const Phases<N> &phases, int k)
 {
@@ -59,11 +62,17 @@ __device__ __forceinline__ bool ring_wait(const CommCtx &ctx, int &dead, const P
         if (t0 == 0) { t0 = now; }
         // (twice the limit of a wait for a peer's flag, of whose end `dead` tells)
         if (now - t0 > 2 * ctx.timeout_ns || spins >= ctx.max_spins) {
-            *static_cast<volatile int *>(&dead) = 1;
+            *static_cast<volatile int *>(&dead) = kRanOut + k;
             return false;
         }
     }
     return true;
+}
+
+// A warp that gives up with another's wait or its own poll, which has reported.
+__device__ __forceinline__ void ring_give_up(int &dead)
+{
+    if (*static_cast<volatile int *>(&dead) == 0) { *static_cast<volatile int *>(&dead) = 1; }
 }
 
 // A warp that gives up: its copies in flight end before the block does.  `last`: the last round that it has
@@ -104,14 +113,16 @@ __device__ __forceinline__ void ask_stream(uint32_t bar, uint32_t dst, const voi
 // The teller: lets the peers know what the passes have stored.  A warp of its own: its fences wait for
 // all of the block's stores.  Over links and within a GPU alike they and the flags' way take
 // longer than a pass, hence the lag.
-// `done`: a phase per pass.
+// `done`: a phase per pass.  `left`: over when all warps that wait for something later than these have come
+// through.  The teller stays until then, to report a wait of the block that ran out.  (Calls in the workers' code, at
+// the waits or at its end, cost the bf16 wire 5 to 7 %.)
 template <int N>
 __device__ __forceinline__ void ring_tell(const CommCtx &ctx, int &dead, uint32_t epoch, const Phases<N> &done,
-                                          int rank, int passes)
+                                          int rank, int passes, const Phases<1> &left)
 {
     const int p = static_cast<int>(threadIdx.x & 31u);
     for (int k = 0; k < passes; ++k) {
-        if (!warp_agrees(ring_wait(ctx, dead, done, k))) { return; }
+        if (!warp_agrees(ring_wait(ctx, dead, done, k))) { break; }
         // (one fence for all that are over by now)
         while (k + 1 < passes && warp_agrees(done.over(k + 1))) { ++k; }
         fence_ranks(ctx);
@@ -120,6 +131,14 @@ __device__ __forceinline__ void ring_tell(const CommCtx &ctx, int &dead, uint32_
             st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank], epoch + static_cast<uint32_t>(k) + 1u);
         }
     }
+    if (p != 0) { return; }
+    // (in slices of a 64th of the limit, between which it looks at `dead`; the waits of the others end before it)
+    int why = 0;
+    for (int i = 0; i < 2048 && !mbar_wait(ctx, left.at(0), 0u, ctx.timeout_ns / 64); ++i) {
+        why = *static_cast<volatile int *>(&dead);
+        if (why != 0) { break; }
+    }
+    if (why >= kRanOut) { report_timeout(ctx, rank, -1, static_cast<uint32_t>(why - kRanOut), 0u, kPhaseRing); }
 }
 
 }  // namespace stdml::collective::cuda

@@ -306,6 +306,7 @@ struct StagedShared {
     // pass k packs and reduces is stored.
     Phases<1> packed, unpacked;
     Phases<4> reduced;
+    Phases<1> left;  // the workers have come through
     uint32_t epoch;
     int dead;  // the block gives up
     // first vectors of the table's entries, for the searches of every round
@@ -439,7 +440,7 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
             if (ok) { asked_res = u; }
         }
         if (!ok) {
-            *static_cast<volatile int *>(&sh.dead) = 1;
+            ring_give_up(sh.dead);
             drain(ctx, sh.operands, asked_op);
             drain(ctx, sh.results, asked_res);
             return;
@@ -649,6 +650,7 @@ __global__ void __launch_bounds__(kStagedBlock, kStagedMinPerSm)
         sh.packed.init(kStagedThreads / 32);
         sh.reduced.init(kStagedThreads / 32);
         sh.unpacked.init(kStagedThreads / 32);
+        sh.left.init(kStagedThreads / 32);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_proxy();
     }
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(kStagedBlock, kStagedMinPerSm)
     if (tid >= kStagedThreads) {
         const int role = (tid - kStagedThreads) / 32;
         if (role == 0) { staged_load<DT>(ctx, a, sh, walk, bufs, vr); }
-        if (role == 1) { ring_tell(ctx, sh.dead, sh.epoch, sh.reduced, rank, a.rounds + kStagedLag); }
+        if (role == 1) { ring_tell(ctx, sh.dead, sh.epoch, sh.reduced, rank, a.rounds + kStagedLag, sh.left); }
         if (role == 2) { staged_fetch(ctx, a, sh, walk, bufs, stores); }
         return;
     }
@@ -687,6 +689,7 @@ __global__ void __launch_bounds__(kStagedBlock, kStagedMinPerSm)
             return;
         }
     }
+    warp_arrive(sh.left.at(0));
 }
 
 template <int DT, int OP>

@@ -1,12 +1,15 @@
 """Device kernels on ONE GPU: all ranks are emulated as rows of one cooperative
 launch (a loopback world), results are compared bit for bit with the native
 host reducer (rank-ascending order, one rounding for 16-bit floats)."""
+import os
+import subprocess
+
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-from stdml_collective_experimental_b200 import DeviceSession, DeviceTimeoutError  # noqa: E402
+from stdml_collective_experimental_b200 import DeviceSession, DeviceTimeoutError, _native  # noqa: E402
 from stdml_collective_experimental_b200.ops.device import (ALGO_ONESHOT,  # noqa: E402
                                                            ALGO_TWOSHOT, ALGO_TWOSHOT_TMA)
 from stdml_collective_experimental_b200.utils.oracle import reduce_many  # noqa: E402
@@ -921,6 +924,14 @@ def test_ring_kernels_give_up(call):
         want = {"all_reduce": reduce_many(host, "sum"), "all_gather": torch.cat(host), "broadcast": host[0]}[call]
         for r in range(w):
             assert same(out[r].cpu(), want) and same(ins[r].cpu(), host[r]), r
+
+
+def test_waits_between_the_warps_of_a_block():
+    prog = os.path.join(_native.CSRC, "build", "bin", "test_ring_sync_cuda")
+    if not os.path.exists(prog):
+        pytest.skip("needs the C++ programs (make -C csrc)")
+    res = subprocess.run([prog], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True, timeout=120)
+    assert res.returncode == 0 and "test-ring-sync: OK" in res.stdout, res.stdout
 
 
 def test_profile_summary_counts_device_time(sess):
