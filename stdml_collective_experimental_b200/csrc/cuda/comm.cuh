@@ -127,6 +127,11 @@ inline void tma_geometry(int world, unsigned int want_tile_vec, int *stages,
     *smem_bytes = st * static_cast<unsigned int>(world) * tv * 16u;
 }
 
+// Shared memory of an SM, of which a block takes its dynamic part, its static part (the dynamic one starts on
+// 128 bytes) and 1 KB for the system.  Cooperative grids count on what fits.
+constexpr size_t kSmSmem = 228u << 10;
+STDML_HD constexpr size_t other_smem(size_t static_bytes) { return (static_bytes + 127) / 128 * 128 + (1u << 10); }
+
 // The staged all-reduce (staged_kernel.cuh): workers and threads of a block, blocks per SM.
 constexpr int kStagedThreads = 192;
 constexpr int kStagedBlock = kStagedThreads + 96;  // and a warp each that loads, tells, fetches
@@ -137,7 +142,7 @@ constexpr int kStagedMinShift = 5;  // smallest tile: one vector per lane of a w
 constexpr int kStagedStarts = 1024;  // table entries searched in shared memory
 constexpr unsigned int kStagedRoundVec = 1024;
 constexpr size_t kStagedSmem = 100u << 10;  // of dynamic shared memory, at most
-constexpr size_t kStagedOtherSmem = 11u << 10;  // of a block beside it, at most
+constexpr size_t kStagedOtherSmem = 11u << 10;  // of a block beside it, at most (checked in staged_kernel.cuh)
 
 // Bytes of the tile buffers of a block (StagedBuffers in staged_kernel.cuh).
 STDML_HD constexpr size_t staged_smem(int world, int tile_shift, bool user_f32)
@@ -148,7 +153,7 @@ STDML_HD constexpr size_t staged_smem(int world, int tile_shift, bool user_f32)
 // Blocks of which an SM holds so many at once.
 STDML_HD constexpr int staged_per_sm(int world, int tile_shift, bool user_f32)
 {
-    const size_t fit = (size_t{228} << 10) / (staged_smem(world, tile_shift, user_f32) + kStagedOtherSmem);
+    const size_t fit = kSmSmem / (staged_smem(world, tile_shift, user_f32) + kStagedOtherSmem);
     return fit < kStagedMinPerSm ? static_cast<int>(fit) : kStagedMinPerSm;
 }
 

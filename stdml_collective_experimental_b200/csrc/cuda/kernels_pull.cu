@@ -211,6 +211,7 @@ struct PullShared {
     uint32_t epoch;
     int dead;  // the block gives up
 };
+static_assert(kPullLongPerSm * (kPullLongSmem + other_smem(sizeof(PullShared))) <= kSmSmem, "so many blocks fit an SM");
 static_assert(kPullLag <= 7, "passes that the workers may be ahead of the warp that tells the peers");
 
 // n bytes of shared memory to a destination of any alignment: the lanes of `threads` threads that share a run

@@ -312,6 +312,7 @@ struct StagedShared {
     // first vectors of the table's entries, for the searches of every round
     unsigned int starts[kStagedStarts];
 };
+static_assert(other_smem(sizeof(StagedShared)) <= kStagedOtherSmem, "the blocks that staged_per_sm() promises fit an SM");
 static_assert(kStagedLag <= 3, "passes that the workers may be ahead of the warp that tells the peers");
 
 // The loader warp: a lane per shard finds the tensor of each of its tiles, a chain of dependent

@@ -67,7 +67,7 @@ int main()
         const int want = trial % 7 == 0 ? 1 + static_cast<int>(rng() % 300) : 0;
         const StagedGeometry g = staged_geometry(world, nvec, slot, sms, rows, want, user_f32);
         const int per_sm = staged_per_sm(world, g.tile_shift, user_f32);
-        EXPECT(per_sm >= 1 && (staged_smem(world, g.tile_shift, user_f32) + kStagedOtherSmem) * per_sm <= 228u << 10);
+        EXPECT(per_sm >= 1 && (staged_smem(world, g.tile_shift, user_f32) + kStagedOtherSmem) * per_sm <= kSmSmem);
         EXPECT((g.blocks - 1) * rows < per_sm * sms && (want == 0 || g.blocks <= want) && g.tile_shift >= kStagedMinShift);
         const unsigned long long ring =
             ((static_cast<unsigned long long>(kStagedRing) * world) << g.tile_shift) * 16;
