@@ -31,13 +31,6 @@ __device__ __forceinline__ void st_stream_v4(void *p, const uint4 &v, unsigned l
                  : "memory");
 }
 
-// Asks for [p, p + bytes) of this GPU's own memory in the L2, ahead of the loads that
-// want it: one instruction of one thread.  16-byte aligned, a multiple of 16 bytes.
-__device__ __forceinline__ void prefetch_l2(const void *p, unsigned int bytes)
-{
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
-}
-
 // Bytes [a, a + 16) of the 32 bytes lo, hi (0 <= a < 16).
 __device__ __forceinline__ uint4 shift_bytes(const uint4 &lo, const uint4 &hi, unsigned int a)
 {
@@ -76,18 +69,6 @@ struct ShiftedSource {
         : begin(static_cast<const char *>(p)), end(begin + bytes), phase(ph),
           odd(static_cast<unsigned int>((reinterpret_cast<unsigned long long>(p) - ph) & 15ull))
     {
-    }
-
-    // Vectors [v, v + n) into the L2, as far as they are the tensor's (whole aligned 16 bytes).
-    __device__ __forceinline__ void prefetch(unsigned long long v, unsigned long long n) const
-    {
-        const char *lo = begin + 16ull * v - phase;
-        const char *hi = lo + 16ull * n;
-        lo = lo > begin ? lo : begin;
-        hi = hi < end ? hi : end;
-        const unsigned long long a = (reinterpret_cast<unsigned long long>(lo) + 15ull) & ~15ull;
-        const unsigned long long b = reinterpret_cast<unsigned long long>(hi) & ~15ull;
-        if (a < b) { prefetch_l2(reinterpret_cast<const void *>(a), static_cast<unsigned int>(b - a)); }
     }
 
     // A vector all of whose bytes are the tensor's: no look at the ends.
