@@ -125,8 +125,11 @@ __device__ __forceinline__ void ring_tell(const CommCtx &ctx, int &dead, uint32_
         if (!warp_agrees(ring_wait(ctx, dead, done, k))) { break; }
         // (one fence for all that are over by now)
         while (k + 1 < passes && warp_agrees(done.over(k + 1))) { ++k; }
+        // The peers read the ring by bulk copies, which only this proxy fence orders behind the generic stores: the
+        // fetchers have none between the flag's acquire and their loads, it is enough that one lies on the way.  It
+        // stands before the release, so that it is part of what the flag publishes.
+        fence_async_proxy_global();
         fence_ranks(ctx);
-        fence_async_proxy_global();  // the peers read it by bulk copies
         if (p < ctx.world) {
             st_relaxed_sys_u32(&pad_of(ctx, p)->flag[blockIdx.x][rank], epoch + static_cast<uint32_t>(k) + 1u);
         }
