@@ -564,20 +564,23 @@ template <int DT, int OP>
 __device__ __forceinline__ bool staged_reduce(const CommCtx &ctx, const StagedArgs &a, StagedShared &sh, uint32_t smem,
                                               int t)
 {
-    if (!ring_wait(ctx, sh.dead, sh.operands, t) || !ring_wait(ctx, sh.dead, sh.own, t)) { return false; }
+    if (!ring_wait(ctx, sh.dead, sh.own, t)) { return false; }
     const StagedWorker<DT> w(ctx, a, sh, smem);
     const unsigned long long policy = evict_first_policy();
     const TileDesc &d = sh.descs[t % kStagedDescs][w.rank];
     const unsigned long long at = a.off + w.walk().piece(t, w.rank);
     const uint32_t own = w.bufs.own(t);
-    const unsigned int fast = d.fast, n = d.n;
+    const unsigned int fast = d.fast, n = d.n, unit = w.user_f32 ? 32u : 16u;
+    // Slow vectors: the own operand, then the result, by way of the own tile's buffer, in the wire type.  Their
+    // chains of loads run while the peers' operands are on their way.
+#pragma unroll 1
+    for (unsigned int i = w.tid; fast < n && i < n; i += kStagedThreads) {
+        if (i >= fast) { slow_load<DT>(slow_vec<DT>(a, w.vr, sh.starts, d, i), w.user_f32, generic_of(own + i * unit)); }
+    }
+    if (!ring_wait(ctx, sh.dead, sh.operands, t)) { return false; }
 #pragma unroll 1
     for (unsigned int i = w.tid; i < n; i += kStagedThreads) {
-        // a slow vector: the own operand, then the result, by way of the own tile's buffer, in the wire type
-        const uint32_t here = own + i * (w.user_f32 ? 32u : 16u);
-        if (i >= fast) {
-            slow_load<DT>(slow_vec<DT>(a, w.vr, sh.starts, d, i), w.user_f32, generic_of(here));
-        }
+        const uint32_t here = own + i * unit;
         const uint4 res = staged_sum<DT, OP>(w, t, i, i < fast ? load_fast<DT>(own, i, w.user_f32) : ld_shared_v4(here));
 #pragma unroll 4
         for (int r = 0; r < ctx.world; ++r) {
