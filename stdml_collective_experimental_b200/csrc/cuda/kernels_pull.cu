@@ -321,6 +321,7 @@ struct PullLong {
                 return;
             }
             if (!more) { continue; }
+            fence_async_proxy_global();
             if (i == 0) { mbar_expect_tx(sh.pieces.at(t), all); }
             if (bytes != 0u) { bulk_load(to, from, bytes, sh.pieces.at(t)); }
         }

@@ -85,7 +85,13 @@ __device__ __forceinline__ void drain(const CommCtx &ctx, const Phases<N> &phase
     }
 }
 
-__device__ __forceinline__ bool warp_agrees(bool ok) { return __all_sync(0xffffffffu, ok ? 1 : 0) != 0; }
+// What each lane has acquired (a peer's flag, a phase) is then seen by all of them: a vote orders nothing between lanes.
+__device__ __forceinline__ bool warp_agrees(bool ok)
+{
+    const bool all = __all_sync(0xffffffffu, ok ? 1 : 0) != 0;
+    __syncwarp();
+    return all;
+}
 
 // One lane of a worker warp for all of it.
 __device__ __forceinline__ void warp_arrive(uint32_t bar)
@@ -125,9 +131,8 @@ __device__ __forceinline__ void ring_tell(const CommCtx &ctx, int &dead, uint32_
         if (!warp_agrees(ring_wait(ctx, dead, done, k))) { break; }
         // (one fence for all that are over by now)
         while (k + 1 < passes && warp_agrees(done.over(k + 1))) { ++k; }
-        // The peers read the ring by bulk copies, which only this proxy fence orders behind the generic stores: the
-        // fetchers have none between the flag's acquire and their loads, it is enough that one lies on the way.  It
-        // stands before the release, so that it is part of what the flag publishes.
+        // The peers read the ring by bulk copies, which proxy fences order behind the generic stores: this one, before the
+        // release, so that it is part of what the flag publishes, and the fetchers' between the flag's acquire and their loads.
         fence_async_proxy_global();
         fence_ranks(ctx);
         if (p < ctx.world) {

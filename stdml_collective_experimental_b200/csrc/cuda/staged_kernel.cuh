@@ -429,6 +429,7 @@ __device__ __forceinline__ void staged_fetch(const CommCtx &ctx, const StagedArg
         bool ok = !reduces || t < 2 || ring_wait(ctx, sh.dead, sh.reduced, t - 2 + kStagedLag);
         if (ok && p < ctx.world) { ok = poll_acquire(ctx, rank, p, sh.epoch + static_cast<uint32_t>(t) + 1u, 0); }
         ok = warp_agrees(ok);
+        fence_async_proxy_global();
         if (ok && reduces) {
             if (p == 0) { mbar_expect_tx(sh.operands.at(t), n_op * bufs.others); }
             if (peer && n_op != 0u) { bulk_load(to_op, from_op, n_op, sh.operands.at(t)); }
