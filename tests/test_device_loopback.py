@@ -788,8 +788,7 @@ def test_tiles_drawn_by_ticket(job, algo):
 
 @pytest.mark.parametrize("shift", [0, 5])
 def test_pull_at_the_slots_of_a_job(job, shift):
-    """all_gather and broadcast of three rounds, tiles of several steps (by the kernel of long
-    messages: broadcast from three ranks up, all_gather among three), from and to addresses
+    """all_gather and broadcast of several rounds, by the kernel of long messages, from and to addresses
     `shift` bytes off a vector boundary."""
     w = job.world
     for op, n in (("all_gather", {2: 20_000_003, 3: 14_000_001, 4: 7_000_001, 8: 2_000_003}[w]),
@@ -1038,6 +1037,57 @@ def test_staged_collectives_of_several_ranks_in_a_graph(n):
                 assert all(bool((t == total).all()) for t in group[r]), (it, r)
             s.all_reduce(ins, out=out)
             s.broadcast(ins, out=bc)
+        torch.cuda.synchronize()
+        s.check()
+
+
+@pytest.mark.parametrize("world,n", [(2, 3_000_001), (3, 3_000_001), (8, 2_500_003)])
+def test_ring_kernels_of_many_rounds_in_a_graph(world, n):
+    """Messages of more than a slot, each in one launch, out of place, with a rank without a destination:
+    replayed back to back from a graph, between ordinary calls that use the same slots.  At these sizes
+    and slots all_gather and broadcast go by the kernel of long messages."""
+    with DeviceSession.loopback(world, heap_bytes=1 << 20, staging_bytes=8 << 20) as s:
+        base = (torch.arange(n, device="cuda") % 1009).float()
+        ins = [torch.empty(n, device="cuda") for _ in range(world)]
+        blank = [None if r == world - 1 else r for r in range(world)]
+        out, bc, ag = ([None if r is None else torch.empty(m, device="cuda") for r in blank] for m in (n, n, n * world))
+        cuts = [n // 3 + 1, 5, n - n // 3 - 6]
+        group_out = [torch.empty(n, device="cuda") for _ in range(world)]
+        lists = [[list(torch.split(t, cuts)) for t in side] for side in (ins, group_out)]
+
+        def calls(stream=None):
+            s.all_reduce(ins, out=out, stream=stream)
+            s.all_gather(ins, ag, stream=stream)
+            s.broadcast(ins, out=bc, root=0, stream=stream)
+            s.group_all_reduce(lists[0], outs=lists[1], stream=stream)
+
+        for t in ins:
+            t.zero_()
+        calls()  # the group's table is made outside the capture
+        torch.cuda.synchronize()
+        g, cap = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        before = s.launches
+        with torch.cuda.graph(g, stream=cap):
+            calls(cap)
+        assert s.launches == before + 4
+        for it in range(3):
+            for r in range(world):
+                ins[r].copy_(base * (r + 1) + it)  # (sums of whole numbers below 2^24)
+            for t in out + bc + ag + group_out:
+                if t is not None:
+                    t.fill_(-1)
+            g.replay()
+            g.replay()
+            torch.cuda.synchronize()
+            s.check()
+            total = sum(t.double() for t in ins).float()
+            for r in range(world):
+                assert torch.equal(group_out[r], total), (it, r)
+                if r < world - 1:
+                    assert torch.equal(out[r], total) and torch.equal(bc[r], ins[0]), (it, r)
+                    assert torch.equal(ag[r], torch.cat(ins)), (it, r)
+            calls()
+            s.broadcast(ins, out=bc, root=0)
         torch.cuda.synchronize()
         s.check()
 
