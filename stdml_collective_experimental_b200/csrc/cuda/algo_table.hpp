@@ -5,6 +5,7 @@
 // other and against NCCL).
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <cstddef>
 
 #include "comm.cuh"
@@ -35,6 +36,22 @@ inline size_t oneshot_limit(const AlgoTuning &t)
     if (t.oneshot_max != 0) { return t.oneshot_max; }
     const size_t w = static_cast<size_t>(t.world);
     return w <= 2 ? (8u << 20) : (16u << 20) / (w * w);
+}
+
+// The same for one message of ordinary tensors among ranks of one GPU: against the staged kernel, whose rounds of
+// flags a short message does not repay.  us per call (one-shot / staged kernel), f32:
+//   3 ranks: 2.3 MB 10.4 / 14.4, 8.9 MB 24.7 / 26.5; 4: 1.3 MB 10.3 / 12.9, 5 MB 18.6 / 21.7, 7.8 MB 29.3 / 28.8;
+//   5: 2.6 MB 16.5 / 18.4, 4 MB 22.6 / 23.4, 5 MB 28.8 / 26.7; 6: 2.8 MB 20.6 / 22.7; 7: 2.6 MB 21.4 / 23.2;
+//   8: 1 MB 14.4 / 16.6, 2 MB 20.6 / 22.0, 3 MB 28.8 / 27.5; 12: 1.1 MB 20.6 / 22.8; 16: 0.6 MB 20.6 / 22.4.
+// Of two bytes, where every rank widens every element, bf16: 3: 5.7 MB 18.5 / 21.9; 4: 4 MB 18.5 / 20.5; 5: 2 MB 16.5 / 17.7,
+//   3.2 MB 22.6 / 20.6; 8: 1 MB 16.4 / 16.9, 1.6 MB 20.6 / 18.8; 16: 0.4 MB 18.5 / 18.4.
+// Of one byte (4: 1 MB 16.5 / 12.4) and groups keep the limit above: a one-shot walks the tensors of a block one after
+// the other (8 ranks, 30 tensors of 0.57 MB in all: 18.6 / 16.6).
+inline size_t staged_oneshot_limit(const AlgoTuning &t, size_t elem_size)
+{
+    if (t.oneshot_max != 0 || t.vranks <= 1 || t.world <= 2 || elem_size == 1) { return oneshot_limit(t); }
+    const double mb = (elem_size >= 4 ? 44 : 26) << 20, w = t.world;
+    return std::max(oneshot_limit(t), static_cast<size_t>(mb / (w * std::sqrt(w))));
 }
 
 inline size_t nvls_oneshot_limit(const AlgoTuning &t)

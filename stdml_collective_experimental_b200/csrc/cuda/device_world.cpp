@@ -770,6 +770,10 @@ class World final : public DeviceWorld
             // tensors, 1.1 MB, 4 ranks: 57 us one-shot, 22 us so).
             algo = kAlgoTwoShot;
         }
+        if (c.algo < 0 && c.staged && c.table == nullptr && algo == kAlgoTwoShot && !any_dst_null && c.root < 0 &&
+            c.phases == kPhaseAll && bytes <= staged_oneshot_limit(tuning(), esize)) {
+            algo = kAlgoOneShot;
+        }
         if (algo >= kAlgoCount) { throw std::invalid_argument("all_reduce: unknown algorithm"); }
         const bool owner = is_owner_algo(algo);
         const bool nvls =

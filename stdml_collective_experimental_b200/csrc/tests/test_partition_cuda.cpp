@@ -379,6 +379,22 @@ int main()
         loop.vranks = 8;
         loop.has_nvls = false;
         EXPECT(select_blocks(loop, (1ull << 30) / 16, kAlgoTwoShot) == 18);  // 148 SMs / 8 rows
+        {   // one-shots of ordinary tensors: further among ranks of one GPU, never where the knob says how far
+            AlgoTuning t;
+            for (t.world = 2; t.world <= kMaxRanks; ++t.world) {
+                t.vranks = 1;
+                EXPECT(staged_oneshot_limit(t, 4) == oneshot_limit(t));
+                t.vranks = t.world;
+                const size_t wide = staged_oneshot_limit(t, 4), narrow = staged_oneshot_limit(t, 2);
+                EXPECT(narrow >= oneshot_limit(t) && (t.world == 2 ? wide == oneshot_limit(t) : wide > narrow));
+                t.oneshot_max = 1024;
+                EXPECT(staged_oneshot_limit(t, 4) == 1024);
+                t.oneshot_max = 0;
+            }
+            t.world = t.vranks = 4;
+            EXPECT(staged_oneshot_limit(t, 8) == 44u << 17 && staged_oneshot_limit(t, 2) == 26u << 17 &&
+                   staged_oneshot_limit(t, 1) == oneshot_limit(t));
+        }
         for (int w = 1; w <= 16; ++w) {  // never zero, never above the pad size
             AlgoTuning t;
             t.world = w;

@@ -697,6 +697,34 @@ def test_staged_group_at_the_slots_of_a_job(job, dtype, wire):
         assert same(torch.cat(dev[r]).cpu(), want), r
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.int64])
+@pytest.mark.parametrize("world", [3, 4, 8, 16])
+def test_longest_one_shot_of_ordinary_tensors(world, dtype):
+    """Around the size from which single messages go by rounds instead: the same bits on both sides,
+    in and out of place, also off a vector boundary, and from the staged kernel when it is asked for."""
+    most = int(((44 if dtype.itemsize >= 4 else 26) << 20) / world ** 1.5) // dtype.itemsize
+    with DeviceSession.loopback(world, heap_bytes=1 << 20, staging_bytes=64 << 20) as s:
+        for n in (most - 1, most, most + 1):
+            host = make_inputs(world, n, dtype, seed=n % 1000)
+            want = reduce_many(host, "sum")
+            for shift in (0, 1):
+                ins = [torch.empty(n + 1, dtype=dtype, device="cuda")[shift:n + shift] for _ in host]
+                for t, h in zip(ins, host):
+                    t.copy_(h)
+                outs = [[torch.zeros(n + 2, dtype=dtype, device="cuda") for _ in host] for _ in range(2)]
+                views = [[t[shift:n + shift] for t in side] for side in outs]
+                s.all_reduce(ins, out=views[0])
+                s.all_reduce(ins, out=views[1], algo="twoshot")
+                s.all_reduce(ins)
+                torch.cuda.synchronize()
+                s.check()
+                for r in range(world):
+                    for got in (views[0][r], views[1][r], ins[r]):
+                        assert same(got.cpu(), want), (n, shift, r)
+                    for side in outs:
+                        assert not side[r][:shift].any() and not side[r][n + shift:].any(), (n, shift, r)
+
+
 @pytest.mark.parametrize("world,dtype,wire,slot,n", [
     (3, torch.float32, None, 32, 9_500_003), (8, torch.bfloat16, None, 16, 9_000_001),
     (2, torch.float32, torch.bfloat16, 32, 17_000_005), (16, torch.int32, None, 16, 4_400_001)])
