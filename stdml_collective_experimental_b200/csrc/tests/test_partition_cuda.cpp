@@ -135,7 +135,8 @@ int main()
         // a smaller slot gives the long kernel smaller tiles, before it takes it away
         const size_t resident = std::max(1, std::min(want > 0 ? want : kMaxBlocks, kPullLongPerSm * sms / rows));
         if (pull_geometry(sources, bytes, size_t{1} << 40, sms, rows, want).lng) {
-            EXPECT(g.lng == (slot >= resident * kPullLongRing * kPullLongMinTile * 16));
+            EXPECT(g.lng == (slot >= resident * kPullLongRing * kPullLongMinTile * 16) ||
+                   ((bytes + 30) / 16 < 2 * kPullLongMin * resident && slot < resident * kPullLongRing * 512 * 16));
         }
         const unsigned long long piece = g.tile * 16ull, ring = piece * g.ring;
         EXPECT(ring * g.blocks == g.ring_bytes() && g.ring_bytes() <= slot);
