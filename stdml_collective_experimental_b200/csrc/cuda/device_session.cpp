@@ -393,7 +393,7 @@ void DeviceSession::all_reduce(const void *const *in, void *const *out, size_t c
     }
     // the staged kernel goes round in a slot: one launch, whatever the length
     const bool ring = total_bytes > slot_elems * es &&
-                      world_->staged_any_length(count, dt, op, algo, false);
+                      world_->staged_any_length(count, dt, op, algo, false, false);
     if (ring) { slot_elems = count; }
     std::vector<const void *> src(vr);
     std::vector<void *> dst(vr);
@@ -866,7 +866,7 @@ void DeviceSession::group_all_reduce(size_t n, const void *const *ins, void *con
                            !in_capture && (algo < 0 || is_owner_algo(algo));
     // Or one chunk in all: the staged kernel goes round in a slot.
     const bool ring = !pipelined && nvec > slot &&
-                      world_->staged_any_length(nvec * (16 / es), dt, op, algo, user_dt >= 0);
+                      world_->staged_any_length(nvec * (16 / es), dt, op, algo, user_dt >= 0, true);
     const GroupPlan &plan = plan_group(n, ins, outs, counts, dt, user_dt, ring ? nvec : slot, in_capture);
     if (pipelined) {
         std::vector<std::vector<const GroupEntry *>> all_tabs;

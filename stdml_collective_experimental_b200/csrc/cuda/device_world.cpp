@@ -895,11 +895,16 @@ class World final : public DeviceWorld
         return rc;
     }
 
-    bool staged_any_length(size_t count, int dt, int op, int algo, bool user_f32) const override
+    bool staged_any_length(size_t count, int dt, int op, int algo, bool user_f32, bool table) const override
     {
         static const size_t sizes[12] = {1, 2, 4, 8, 1, 2, 4, 8, 2, 2, 4, 8};
         if (dt < 0 || dt > DT_F64_) { return false; }
         const size_t bytes = count * sizes[dt], nvec = (bytes + 15) / 16;
+        // Two ranks on one GPU: a one-shot per slot (16 MB in slots of 8 MB 28.8 us, of 2 MB 65.7; in rounds 33.0, 71.9; 24 MB
+        // 47.5, 98.6 and 45.9, 104.9, as bf16 53.4, 109 and 56.8, 127).
+        if (algo < 0 && !table && vranks_ == 2 && bytes <= (24u << 20) && opt_.staging_bytes <= oneshot_limit(tuning())) {
+            return false;
+        }
         if (algo < 0) { algo = pick_algo(bytes, dt, op, false); }
         return opt_.world > 1 && (algo == kAlgoTwoShot || algo == kAlgoTwoShotTma) &&
                staged_geometry(opt_.world, nvec, opt_.staging_bytes, num_sms_, vranks_, 0, user_f32).full;

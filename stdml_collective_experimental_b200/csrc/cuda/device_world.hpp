@@ -186,7 +186,8 @@ class DeviceWorld
     virtual bool pulls_staged(size_t bytes, int root) const = 0;
     // Whether a staged all_reduce of `count` elements in all goes by rounds over a ring in a
     // staging slot, which takes messages of any length in one launch.  Alike on every rank.
-    virtual bool staged_any_length(size_t count, int dt, int op, int algo, bool user_f32) const = 0;
+    virtual bool staged_any_length(size_t count, int dt, int op, int algo, bool user_f32,
+                                   bool table) const = 0;
     // Two-shot all-reduce over a table of registered tensors (see PeerEntry).
     virtual int group_peer(const PeerEntry *table, int ntable, size_t nvec, int dt, int op,
                            double scale, void *stream) = 0;

@@ -50,14 +50,13 @@ struct StagedWalk {
 struct StagedGeometry {
     int blocks = 0;  // 0: the slot cannot hold the ring of even one block
     int tile_shift = kStagedMinShift, rounds = 1;
-    // A message longer than the slot goes round in it in one launch: the slot holds the rings of as many blocks
-    // as there may be.
+    // A message longer than the slot goes round in it in one launch: the slot holds the rings of enough blocks.
     bool full = false;
 };
 
 // Grid and tile for `nvec` vectors on `num_sms` SMs that `vranks` ranks share.  A tile is kStagedRoundVec
 // vectors over all shards of a round at most, smaller where its buffers would outgrow the shared
-// memory of a block or the rings of all blocks the staging slot, and where the message would
+// memory of a block or the rings of enough blocks the staging slot, and where the message would
 // otherwise leave blocks without a tile.
 inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_bytes, int num_sms, int vranks,
                                       int want_blocks, bool user_f32)
@@ -77,18 +76,22 @@ inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_byt
         return static_cast<size_t>(std::max(1, want_blocks > 0 ? std::min(want_blocks, resident) : resident));
     };
     const auto tiles_of = [&](int shift) { return (longest + (size_t{1} << shift) - 1) >> shift; };
-    // The slot holds the rings of all blocks that have a tile of this size.
-    const auto fits = [&](int shift) { return ring_bytes(shift) * std::min(tiles_of(shift), most(shift)) <= staging_bytes; };
-    // No block goes without a ring for the sake of larger tiles.  161 f32 tensors of 102 MB, us, with tiles of up
-    // to 256 vectors in as many blocks as the slot holds / so: 4 ranks, slots of 8 MB 413 / 304, of 4 MB 664 / 451; 8 ranks,
-    // 4 MB 856 / 616.  Where the smallest tiles do not fit either, fewer blocks with larger ones: 8 ranks, 1 MB
-    // 2471 / 2689 in the smallest.
-    const bool cramped = !fits(kStagedMinShift);
+    // Rings of enough blocks: of most SMs, or of two on each for tiles from 256 vectors on among two or three ranks.  In
+    // between a slot gives as many blocks as it holds.  Tensors of 96 MB, f32, us, one launch in tiles of 64 / 128 / 256 /
+    // 512 vectors: 2 ranks, slots of 2 MB 447 / 410 / 532 / 663, 4 MB 331 / 252 / 267 / 336 (bf16 24 MB 65 / 92 with 128 / 256),
+    // 8 MB 334 / 191 / 157 / 172, 16 MB 361 / 205 / 132 / 109; 3 ranks, 4 MB 382 / 274 / 286, 8 MB 407 / 243 / 180; 4 ranks,
+    // 2 MB 579 / 483 / 598, 4 MB 424 / 329 / 308, 8 MB 480 / 300 / 239; 8 ranks, 2 MB 766 / 679, 4 MB 630 / 505.
+    const auto enough = [&](int shift) {
+        const int some = std::max(1, (shift < 8 || world > 3 ? 1 : 2) * num_sms * 3 / 4 / vranks);
+        return ring_bytes(shift) * std::min<size_t>({tiles_of(shift), most(shift), static_cast<size_t>(some)}) <= staging_bytes;
+    };
+    // (where the smallest tiles do not fit so either, fewer blocks with larger ones)
+    const bool cramped = !enough(kStagedMinShift);
     const size_t want = std::max<size_t>(kStagedRoundVec / static_cast<size_t>(world), size_t{1} << kStagedMinShift);
     const auto good = [&](int shift) {
         const size_t tile = size_t{1} << shift;
         if (tile > want || staged_smem(world, shift, user_f32) > kStagedSmem) { return false; }
-        if (cramped ? tile > 256 || ring_bytes(shift) > staging_bytes : !fits(shift)) { return false; }
+        if (cramped ? tile > 256 || ring_bytes(shift) > staging_bytes : !enough(shift)) { return false; }
         // A short message has fewer blocks, not smaller tiles than about a vector per worker, and larger ones
         // rather than a second round (a set of ragged tensors pays several memory latencies per vector: 224 of
         // them, 4 ranks, 20.6 us with 256 vectors at least, 14.5 so).
@@ -100,9 +103,9 @@ inline StagedGeometry staged_geometry(int world, size_t nvec, size_t staging_byt
     const size_t tiles = tiles_of(g.tile_shift);
     const size_t fit = staging_bytes / ring_bytes(g.tile_shift);
     g.blocks = static_cast<int>(std::min<size_t>({tiles, most(g.tile_shift), fit}));
-    // Rounds of 64 vectors cost more than a launch per slot (2 ranks, slots of 2 MB: 798 us, 622 so; 128 vectors, 4 MB:
-    // 406, 411 so).
-    g.full = fit >= most(g.tile_shift) && static_cast<size_t>(world) << g.tile_shift > 64;
+    // A launch per slot instead: 8 ranks, slots of 2 MB, 96 MB 1280 us (679 so); 2 ranks, 8 MB 286 (157).
+    // Slots below 2 MB have a launch each, as callers may count on.
+    g.full = !cramped && staging_bytes >= 2u << 20;
     if (g.blocks > 0) { g.rounds = static_cast<int>((tiles + g.blocks - 1) / g.blocks); }
     return g;
 }

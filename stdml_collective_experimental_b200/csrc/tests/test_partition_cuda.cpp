@@ -80,14 +80,15 @@ int main()
         std::vector<unsigned long long> bound(world + 1);
         for (int s = 0; s <= world; ++s) { bound[s] = StagedWalk::shard_begin(nvec, world, s); }
         EXPECT(bound[0] == 0 && bound[world] == nvec);
-        // no block goes without a ring for the sake of larger tiles, if the smallest would do
+        // larger tiles leave three SMs of four a block, if the smallest ones do
         unsigned long long longest = 0;
         for (int s = 0; s < world; ++s) { longest = std::max(longest, bound[s + 1] - bound[s]); }
-        const unsigned long long tiles = (longest + (1ull << g.tile_shift) - 1) >> g.tile_shift;
-        const int most = std::max(1, std::min(per_sm * sms / rows, kMaxBlocks));
+        const int all = want > 0 ? std::min(want, per_sm * sms / rows) : per_sm * sms / rows;
+        const unsigned long long some = std::max(1, std::min({all, kMaxBlocks, (g.tile_shift < 8 || world > 3 ? 1 : 2) * sms * 3 / 4 / rows}));
         const unsigned long long ring32 = (static_cast<unsigned long long>(kStagedRing) * world << kStagedMinShift) * 16;
-        EXPECT(g.blocks == std::min<unsigned long long>(tiles, want > 0 ? std::min(want, most) : most) ||
-               ring32 * std::min<unsigned long long>((longest + 31) / 32, kStagedMinPerSm * sms / rows) > slot);
+        const unsigned long long tiles = (longest + (1ull << g.tile_shift) - 1) >> g.tile_shift;
+        if (g.full) { EXPECT(static_cast<unsigned long long>(g.blocks) >= std::min(tiles, some)); }
+        if (g.tile_shift < 8) { EXPECT(g.full == (ring32 * some <= slot && slot >= 2u << 20) || tiles < some); }
         for (int s = 0; s < world; ++s) {
             unsigned long long expect = bound[s];
             for (int k = 0; k < g.rounds; ++k) {
@@ -103,11 +104,12 @@ int main()
             EXPECT(expect == bound[s + 1]);
         }
     }
-    // 102 MB go round in slots far smaller than that in one launch, in as many blocks as are resident
+    // 102 MB go round in slots far smaller than that in one launch, with a block on most SMs; in 64 MB in all that are resident
     for (const int world : {2, 3, 4, 8}) {
-        for (const size_t mb : {4, 8, 16, 32, 64}) {
+        for (const size_t mb : {2, 4, 8, 16, 32, 64}) {
             const StagedGeometry g = staged_geometry(world, 102'000'000 / 16, mb << 20, 148, world, 0, false);
-            EXPECT(g.full && g.blocks == kStagedMinPerSm * 148 / world);
+            EXPECT(g.full && g.blocks * world >= 144 && g.tile_shift >= 7);
+            if (mb == 64) { EXPECT(g.blocks == kStagedMinPerSm * 148 / world); }
         }
     }
     // pull: over blocks and rounds the tiles cover the vectors of every rank's block exactly

@@ -1069,7 +1069,7 @@ def test_staged_collectives_of_several_ranks_in_a_graph(n):
         s.check()
 
 
-@pytest.mark.parametrize("world,n", [(2, 3_000_001), (3, 3_000_001), (8, 2_500_003)])
+@pytest.mark.parametrize("world,n", [(2, 7_000_001), (3, 3_000_001), (8, 2_500_003)])
 def test_ring_kernels_of_many_rounds_in_a_graph(world, n):
     """Messages of more than a slot, each in one launch, out of place, with a rank without a destination:
     replayed back to back from a graph, between ordinary calls that use the same slots.  At these sizes
