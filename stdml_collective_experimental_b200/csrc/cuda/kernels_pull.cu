@@ -192,9 +192,9 @@ __global__ void __launch_bounds__(kPullThreads, kPullPerSm)
 // from two of the piece's.  Ring of 2 lag + 1: tile k goes over tile k - 2 lag - 1, which its readers had
 // in their shared memory before the flags that the fetcher saw for pass k - 1.
 // Measured among ranks of one GPU, us, against a kernel that copied by bulk copies in lockstep with the pack, or
-// pull_kernel: broadcast of 94 MB to 3 others 108 / 90, 100 MB to 7 220 / 186, 9 MB to 5 27 / 20; all_gather of
-// 8 x 2.47 MB (an odd size) 54 / 42, 8 x 8 MB 142 / 118, 3 x 34 MB 104 / 96, 8 x 0.7 MB 25.5 / 18; to destinations off a
-// vector boundary 8 x 2.47 MB 435 / 51, broadcast of 34 MB to 3 321 / 42.
+// pull_kernel: broadcast in place of 94 MB to 3 others 108 / 93, into other tensors 144 / 116, of 100 MB to 7 284 / 234, 9 MB
+// to 5 33 / 23; all_gather of 8 x 2.47 MB (an odd size) 54 / 42, 8 x 8 MB 142 / 125, 3 x 34 MB 104 / 98, 8 x 0.7 MB 25 / 18; to
+// destinations off a vector boundary 8 x 2.47 MB 429 / 52, broadcast of 34 MB to 3 364 / 50.
 // By lag, broadcast of 94 MB: 2: 143, 3: 121, 5: 100, 7: 95 (before there was a storer); no more from there on.
 // Two blocks per SM and 100 KB each, or three and 64: 8 x 2.47 MB 42 / 44, 94 MB 91 / 89; buffers for three or four rounds
 // of pieces, with smaller tiles: 49, 57 and 93, 102.

@@ -28,7 +28,8 @@
 //
 // Measured among ranks of one GPU, us, against the kernel whose blocks packed, exchanged flags, reduced and
 // unpacked by turns, a load per thread in flight, a launch per slot: 161 f32 tensors, 2 / 4 / 8 ranks
-// 148 / 286 / 622, now 105 / 243 / 558; BERT-base as bf16 wire, 2 ranks 434, now 331.  By lag, 4 ranks: 1: 398, 2: 249,
+// 150 / 285 / 607, now 103 / 239 / 507 (4 ranks, inputs that change: 287, 245); BERT-base as bf16 wire, 2 ranks 437, now
+// 335 (438, 344).  Messages of a few rounds, which gain nothing: staged_oneshot_limit.  By lag, 4 ranks: 1: 398, 2: 249,
 // 3: 242 (a lag of 1 with the polls and fences in the workers' own warps 380).
 // By workers 128 / 192 / 256 of 3 blocks per SM: 253 / 243 / 242 (f32), 373 / 328 / 345 (bf16 wire).
 //

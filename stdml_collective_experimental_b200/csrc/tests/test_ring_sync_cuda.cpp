@@ -57,6 +57,8 @@ int main()
     }
     cudaEvent_t ends[2];
     for (auto &e : ends) { cudaEventCreate(&e); }
+    cudaFuncAttributes loaded;  // (not within the time that is measured)
+    EXPECT(cudaFuncGetAttributes(&loaded, waits) == cudaSuccess);
     for (const int gave_up_before : {0, 1}) {
         *status = StatusBlock{};
         got[0] = got[1] = got[2] = -1;

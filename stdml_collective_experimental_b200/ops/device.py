@@ -282,7 +282,8 @@ class DeviceSession:
 
     def group_all_reduce(self, tensors, outs=None, op="sum", scale=None, wire_dtype=None,
                          algo=None, stream=None):
-        """Fused all-reduce of a whole list of tensors in one launch per staging slot.
+        """Fused all-reduce of a whole list of tensors in one launch; in one per staging slot where
+        the slot is smaller than 2 MB, where the switch reduces, and where a job pipelines (from 256 MB).
 
         `wire_dtype` (bf16/f16) sends f32 tensors as 16-bit floats (cast fused into
         the pack/unpack phases).  Loopback: `tensors[rank][i]`."""
